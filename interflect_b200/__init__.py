@@ -623,8 +623,8 @@ class Context:
                     "set_wait_limit")
 
     def set_leaf_grid(self, on: bool) -> None:
-        """Whether the next upload builds the per-cell leaf lists of large
-        BVHs for cone-shadow marches (results are identical either way)."""
+        """Whether the next upload builds the per-cell object lists that
+        distance queries use (results are identical either way)."""
         self._check(lib().ifx_set_leaf_grid(self._h, 1 if on else 0), "set_leaf_grid")
 
     def set_stage_limit(self, max_bytes: int) -> None:

@@ -61,9 +61,8 @@ struct ifx_ctx {
     DBuf blob;
     BlobRef blobref{};
     uint32_t stage_limit = kDefaultStageLimit;
-    bool leafgrid_on = true;  // build per-cell leaf lists for large BVHs (ifx_set_leaf_grid)
-    DBuf lg_U, lg_count, lg_start, lg_leaves, lg_leaf, lg_key;
-    uint32_t lg_cells = 0, lg_entries = 0;
+    bool objgrid_on = true;  // build the object grid at the next upload (ifx_set_leaf_grid)
+    DBuf og_cells;           // its per-cell masks or lists
     SceneConsts sc{};
     DBuf status;  // uint32 device status word
     DBuf srgb_t;  // 256 f32 thresholds
@@ -477,8 +476,7 @@ extern "C" void ifx_ctx_destroy(ifx_ctx* ctx) {
                     &ctx->sell_rows, &ctx->sell_sizes, &ctx->sell_off, &ctx->sell_idx, &ctx->sell_w,
                     &ctx->path_sincos, &ctx->shsc, &ctx->lff, &ctx->lvis, &ctx->lq, &ctx->lsc,
                     &ctx->vkey, &ctx->vkey_alt, &ctx->vval, &ctx->vval_alt, &ctx->ckey, &ctx->ckey_alt,
-                    &ctx->cval, &ctx->cval_alt, &ctx->msum, &ctx->gen_head_acc, &ctx->gen_next_acc, &ctx->lg_U, &ctx->lg_count,
-                    &ctx->lg_start, &ctx->lg_leaves, &ctx->lg_leaf, &ctx->lg_key};
+                    &ctx->cval, &ctx->cval_alt, &ctx->msum, &ctx->gen_head_acc, &ctx->gen_next_acc, &ctx->og_cells};
     for (DBuf* b : bufs) free_buf(*b);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     for (cudaEvent_t ev : {ctx->ev0, ctx->ev1, ctx->kv0, ctx->kv1, ctx->kc0, ctx->kc1, ctx->tm0, ctx->tm1})
@@ -568,83 +566,95 @@ extern "C" int ifx_set_stage_limit(ifx_ctx* ctx, uint32_t max_bytes) {
     return IFX_OK;
 }
 
-// The leaf grid of a scene with a BVH of more than three nodes whose objects
-// all have exact distance functions (every kind but the cone): 64 cells along
-// the longest side of the scene bounds.
-static int leafgrid_build(ifx_ctx* ctx, const std::vector<uint8_t>& blob) {
-    ctx->blobref.lg = LeafGrid{};
+// Whether a primitive meets the object grid's conditions (objgrid.h): finite,
+// 1-Lipschitz, and inside its box; `scale` is raised to its largest
+// coordinate, length or radius. Cones are left out, as are the degenerate
+// forms that the parser lets through (negative sizes, a rounding radius above
+// the half-size, cylinders whose squared length f32 cannot carry well).
+static bool og_admits(const DPrim& p, double& scale) {
+    const float* v = p.v;
+    for (int i = 0; i < 12; ++i)
+        if (!std::isfinite(v[i])) return false;
+    auto up = [&](std::initializer_list<float> xs) {
+        for (float x : xs) scale = std::max(scale, std::fabs((double)x));
+    };
+    switch (p.kind) {
+        case K_SPHERE:
+            up({v[0], v[1], v[2], v[3]});
+            return v[3] >= 0.0f;
+        case K_BOX:
+        case K_BOX_ROT:
+            up({v[0], v[1], v[2], v[3], v[4], v[5], v[6]});
+            return v[3] >= 0.0f && v[4] >= 0.0f && v[5] >= 0.0f && v[6] >= 0.0f;
+        case K_PLANE: {
+            up({v[3]});
+            const double l2 = (double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2];
+            return std::fabs(l2 - 1.0) < 1e-5;
+        }
+        case K_CAPSULE:
+            up({v[0], v[1], v[2], v[3], v[4], v[5], v[7]});
+            return v[6] > 1e-8f && v[7] >= 0.0f;
+        case K_TORUS:
+            up({v[0], v[1], v[2], v[3], v[4]});
+            return v[3] >= 0.0f && v[4] >= 0.0f;
+        case K_CYLINDER:
+            up({v[0], v[1], v[2], v[3], v[4], v[5], v[7]});
+            return v[6] > 1e-8f && v[6] < 1e8f && v[7] >= 0.0f;
+    }
+    return false;
+}
+
+// The object grid of a scene with a BVH whose primitives og_admits all.
+static int objgrid_build(ifx_ctx* ctx, const std::vector<uint8_t>& blob) {
+    ctx->blobref.og = ObjGrid{};
     const BlobHeader* bh = reinterpret_cast<const BlobHeader*>(blob.data());
-    if (!ctx->leafgrid_on || !bh->use_bvh || bh->n_nodes <= 3) return IFX_OK;
-    const DPrim* prims = reinterpret_cast<const DPrim*>(blob.data() + bh->off_prims);
-    for (int i = 0; i < bh->n_prims; ++i)
-        if (prims[i].kind == K_CONE) return IFX_OK;
-    const DNode* nodes = reinterpret_cast<const DNode*>(blob.data() + bh->off_nodes);
-    std::vector<uint32_t> leaves;
-    for (int i = 0; i < bh->n_nodes; ++i)
-        if (nodes[i].count > 0) leaves.push_back((uint32_t)i);
+    const uint32_t nobj = (uint32_t)(bh->n_planes + bh->n_objects);
+    if (!ctx->objgrid_on || !bh->use_bvh || bh->n_nodes == 0 || nobj > kOgMaxObjects) return IFX_OK;
     const float* lo = ctx->sc.lo;
     const float* hi = ctx->sc.hi;
-    double ext = 0.0, mag = 0.0;
+    double ext = 0.0, scale = 0.0;
     for (int a = 0; a < 3; ++a) {
         ext = std::max(ext, (double)hi[a] - (double)lo[a]);
-        mag = std::max(mag, std::max(std::fabs((double)lo[a]), std::fabs((double)hi[a])));
+        scale = std::max(scale, std::max(std::fabs((double)lo[a]), std::fabs((double)hi[a])));
     }
-    if (!(ext > 0.0)) return IFX_OK;
-    const int kCells = 64;
+    const DPrim* prims = reinterpret_cast<const DPrim*>(blob.data() + bh->off_prims);
+    for (int i = 0; i < bh->n_prims; ++i)
+        if (!og_admits(prims[i], scale)) return IFX_OK;
+    const DObject* objs = reinterpret_cast<const DObject*>(blob.data() + bh->off_objects);
+    for (uint32_t i = 0; i < nobj; ++i) {
+        if (!std::isfinite(objs[i].smooth)) return IFX_OK;
+        scale = std::max(scale, std::fabs((double)objs[i].smooth));
+    }
+    scale += (double)ctx->sc.diag;
+    if (!(ext > 0.0) || !std::isfinite(scale)) return IFX_OK;
+    const bool masks = nobj <= kOgMaskObjects;
+    const int kCells = masks ? 64 : 96;
     const double cs = ext / kCells;
-    LeafGrid g{};
-    uint32_t ncells = 1;
+    ObjGrid g{};
+    g.delta = (float)(scale / 65536.0);
+    // A scene whose coordinates dwarf its extent: the margins would list everything.
+    if ((double)g.delta > 0.25 * cs) return IFX_OK;
+    g.inv = (float)(1.0 / cs);
+    size_t ncells = 1;
     for (int a = 0; a < 3; ++a) {
-        g.lo[a] = lo[a];
-        g.dim[a] = std::min(kCells, std::max(1, (int)std::ceil(((double)hi[a] - (double)lo[a]) / cs)));
-        ncells *= (uint32_t)g.dim[a];
+        g.bias[a] = (float)(-(double)lo[a] / cs - 0.5);
+        g.dim[a] = (uint32_t)std::min(kCells, std::max(1, (int)std::ceil(((double)hi[a] - (double)lo[a]) / cs)));
+        ncells *= g.dim[a];
     }
-    g.inv_cell = (float)(1.0 / cs);
-    // 2^-12 of the coordinates' scale: thousands of times any f32 rounding
-    // of a distance at that scale, small against the distances marched.
-    g.tol = (float)((mag + (double)ctx->sc.diag) / 4096.0);
-    const double pad = g.tol;
-    const float half_diag = (float)((cs * 0.5 + pad) * std::sqrt(3.0) * (1.0 + 1e-6) + pad);
-    const uint32_t nleaf = (uint32_t)leaves.size();
-    ENSURE(ctx->lg_U, (size_t)ncells * 4);
-    ENSURE(ctx->lg_count, ((size_t)ncells + 1) * 4);
-    ENSURE(ctx->lg_start, ((size_t)ncells + 1) * 4);
-    ENSURE(ctx->lg_leaves, (size_t)nleaf * 4);
-    CK(cudaMemcpyAsync(ctx->lg_leaves.p, leaves.data(), (size_t)nleaf * 4, cudaMemcpyHostToDevice, ctx->st));
-    float* U = (float*)ctx->lg_U.p;
-    uint32_t* count = (uint32_t*)ctx->lg_count.p;
-    uint32_t* start = (uint32_t*)ctx->lg_start.p;
-    launch_lg_bound(ctx->st, ctx->blobref, g, (float)cs, half_diag, ncells, U, (uint32_t*)ctx->status.p);
-    launch_lg_lists(ctx->st, (const uint8_t*)ctx->blob.p, g, cs, pad, ncells, U, (const uint32_t*)ctx->lg_leaves.p,
-                    nleaf, count, nullptr, nullptr, nullptr);
-    CK(cudaMemsetAsync(count + ncells, 0, 4, ctx->st));
-    ctx->launches += 2;
-    CKL();
-    CUB([&](void* t, size_t& b) {
-        return cub::DeviceScan::ExclusiveSum(t, b, count, start, (int)ncells + 1, ctx->st);
-    });
-    uint32_t total = 0;
-    CK(cudaMemcpyAsync(&total, start + ncells, 4, cudaMemcpyDeviceToHost, ctx->st));
-    int r = check_status(ctx);  // synchronises
-    if (r) return r;
-    ENSURE(ctx->lg_leaf, (size_t)total * 4);
-    ENSURE(ctx->lg_key, (size_t)total * 4);
-    launch_lg_lists(ctx->st, (const uint8_t*)ctx->blob.p, g, cs, pad, ncells, U, (const uint32_t*)ctx->lg_leaves.p,
-                    nleaf, nullptr, start, (uint32_t*)ctx->lg_leaf.p, (float*)ctx->lg_key.p);
+    ENSURE(ctx->og_cells, ncells * (masks ? 4 : 16));
+    g.mode = masks ? kOgMask : kOgList;
+    launch_og_build(ctx->st, ctx->blobref, g, lo, (float)cs, masks ? (uint32_t*)ctx->og_cells.p : nullptr,
+                    masks ? nullptr : (uint4*)ctx->og_cells.p, (uint32_t*)ctx->status.p);
     ctx->launches++;
     CKL();
-    g.start = start;
-    g.leaf = (const uint32_t*)ctx->lg_leaf.p;
-    g.enabled = 1;
-    ctx->blobref.lg = g;
-    ctx->lg_entries = total;
-    ctx->lg_cells = ncells;
+    g.mask = g.list = (const uint32_t*)ctx->og_cells.p;
+    ctx->blobref.og = g;
     return IFX_OK;
 }
 
 extern "C" int ifx_set_leaf_grid(ifx_ctx* ctx, int on) {
     if (!ctx) return IFX_ERR_INVALID;
-    ctx->leafgrid_on = on != 0;
+    ctx->objgrid_on = on != 0;
     return IFX_OK;
 }
 
@@ -674,7 +684,6 @@ extern "C" int ifx_scene_upload(ifx_ctx* ctx, const ifx_scene* scene) {
     std::vector<float4> le = light_emissions(s);
     ENSURE(ctx->lemit, le.size() * 16);
     if (!le.empty()) CK(cudaMemcpyAsync(ctx->lemit.p, le.data(), le.size() * 16, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
     ctx->nl = (uint32_t)le.size();
     frame_changed(ctx);
     ctx->scene = s;
@@ -684,15 +693,15 @@ extern "C" int ifx_scene_upload(ifx_ctx* ctx, const ifx_scene* scene) {
     choose_staging(ctx);
     ctx->blobref.stack_depth = maxd + 2;
     ctx->blobref.wait_polls = ctx->wait_polls;
-    {
-        const BlobHeader* bh = reinterpret_cast<const BlobHeader*>(blob.data());
-        ctx->blobref.tree3 = bh->use_bvh && bh->n_nodes == 3 ? 1 : 0;
-    }
     ctx->sc = scene_consts(s);
     {
-        int r = leafgrid_build(ctx, blob);
+        int r = objgrid_build(ctx, blob);
         if (r) return r;
+        // The three-node kernels read the grid as masks.
+        const BlobHeader* bh = reinterpret_cast<const BlobHeader*>(blob.data());
+        ctx->blobref.tree3 = bh->use_bvh && bh->n_nodes == 3 && ctx->blobref.og.mode != kOgList ? 1 : 0;
     }
+    CK(cudaStreamSynchronize(ctx->st));
     ctx->has_scene = true;
     ctx->has_transfer = false;
     ctx->has_grid = false;

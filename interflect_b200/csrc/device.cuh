@@ -11,6 +11,7 @@
 
 #include "layout.h"
 #include "libm_f32.h"
+#include "objgrid.h"
 #include "sqcmp.h"
 
 namespace ifx {
@@ -82,6 +83,7 @@ struct SceneView {
     const DObject* objs;
     const DPrim* prims;
     const DNode* nodes;
+    const DFast* fast;
     const DQuadLight* lights;
     const DSphereLight* slights;
     const DMaterial* mats;
@@ -89,7 +91,7 @@ struct SceneView {
     int n_planes, n_objects, n_nodes, n_lights, n_slights, use_bvh;
     int n_prims, n_mats;
     uint32_t* status;  // the kernel's status word (bounds checks of IFX_CHECKED builds)
-    LeafGrid lg;       // per-cell candidate leaves (shadow marches in large BVHs)
+    ObjGrid og;        // candidate objects per cell
     // This thread's BVH traversal stack in shared memory: entry i lives at
     // stk[i * stk_stride] (node index) and stkd[i * stk_stride] (the node's
     // box distance, computed when it was pushed); stk_depth entries (the tree
@@ -103,6 +105,7 @@ struct SceneView {
     __device__ __forceinline__ const DObject& obj(int i) const { return objs[IFX_CK(i, n_planes + n_objects, status)]; }
     __device__ __forceinline__ const DPrim& prim(int i) const { return prims[IFX_CK(i, n_prims, status)]; }
     __device__ __forceinline__ const DNode& node(int i) const { return nodes[IFX_CK(i, n_nodes, status)]; }
+    __device__ __forceinline__ const DFast& fobj(int i) const { return fast[IFX_CK(i, n_planes + n_objects, status)]; }
     __device__ __forceinline__ const DQuadLight& light(int i) const { return lights[IFX_CK(i, n_lights, status)]; }
     __device__ __forceinline__ const DSphereLight& slight(int i) const {
         return slights[IFX_CK(i, n_slights, status)];
@@ -121,6 +124,7 @@ __device__ __forceinline__ SceneView make_view(const uint8_t* base) {
     v.objs = reinterpret_cast<const DObject*>(base + h->off_objects);
     v.prims = reinterpret_cast<const DPrim*>(base + h->off_prims);
     v.nodes = reinterpret_cast<const DNode*>(base + h->off_nodes);
+    v.fast = reinterpret_cast<const DFast*>(base + h->off_fast);
     v.lights = reinterpret_cast<const DQuadLight*>(base + h->off_lights);
     v.slights = reinterpret_cast<const DSphereLight*>(base + h->off_sphere_lights);
     v.mats = reinterpret_cast<const DMaterial*>(base + h->off_materials);
@@ -134,7 +138,7 @@ __device__ __forceinline__ SceneView make_view(const uint8_t* base) {
     v.n_prims = h->n_prims;
     v.n_mats = h->n_materials;
     v.status = nullptr;
-    v.lg = LeafGrid{};
+    v.og = ObjGrid{};
     return v;
 }
 
@@ -369,10 +373,10 @@ struct DistHit {
     uint32_t mat;
 };
 
-// scene.rs:191-208 with bvh.rs:100-150 (query) or bvh.rs:155-163 (linear).
+// scene.rs:191-208 with bvh.rs:100-150 (query) or bvh.rs:155-163 (linear):
+// the reference's own traversal.
 template <class C>
-__device__ __forceinline__ DistHit dist_mat(const SceneView& sv, V p, C& cnt) {
-    cnt.add(CN_SDF);
+__device__ __forceinline__ DistHit dist_mat_ref(const SceneView& sv, V p, C& cnt) {
     DistHit best{kMaxF, 0u};
     for (int i = 0; i < sv.n_planes; ++i) {
         const DObject o = sv.obj(i);
@@ -469,6 +473,97 @@ __device__ __forceinline__ DistHit dist_mat(const SceneView& sv, V p, C& cnt) {
     return best;
 }
 
+// obj_dist of stored object o from its packed form: the operations of
+// prim_dist in its order. A sphere is a box of no extent (|x| - 0 and
+// max(|x|, 0) keep its squares, the inside term is 0), and a torus is one
+// after its first radius (its third square is +0), so those three share the
+// code after the torus's own step, to the bit.
+__device__ __forceinline__ float fast_dist(const SceneView& sv, int o, V p, float best) {
+    const float4* q = reinterpret_cast<const float4*>(&sv.fobj(o));
+    const float4 a = q[0], b = q[1];
+    const int tag = __float_as_int(b.w);
+    V d = p - mk4(a);
+    float bx = b.x;
+    if (tag != F_BOX) {
+        if (tag == F_TORUS) {
+            d.x = sqrtf(d.x * d.x + d.z * d.z) - bx;
+            d.z = 0.0f;
+            bx = 0.0f;
+        } else if (tag == F_BOX_ROT) {
+            const float4 c = q[2];
+            d = V{c.x * d.x - c.y * d.z, d.y, c.y * d.x + c.x * d.z};
+        } else if (tag == F_PLANE) {
+            return dot(p, mk4(a)) - a.w;
+        } else if (tag == F_CAPSULE) {
+            const V ba = mk4(b);
+            const float h = clampr(dot(d, ba) / q[2].x, 0.0f, 1.0f);
+            return len(d - ba * h) - a.w;
+        } else {
+            NoCount nc;
+            return obj_dist(sv, sv.obj(o), p, nc, best);
+        }
+    }
+    const V qq = vabs(d) - V{bx, b.y, b.z};
+    return len(vmax(qq, V{0.0f, 0.0f, 0.0f})) + fminf(fmaxf(qq.x, fmaxf(qq.y, qq.z)), 0.0f) - a.w;
+}
+
+// The nearest and second-nearest of the objects a query has evaluated.
+struct OgBest {
+    float d1, d2;
+    int o1;
+    __device__ __forceinline__ OgBest() : d1(kMaxF), d2(kMaxF), o1(0) {}
+    // An object that cannot come within delta of the nearest needs no exact
+    // value (obj_dist's `best`), so its subtractions are skipped.
+    __device__ __forceinline__ void eval(const SceneView& sv, int o, V p) {
+        const float d = fast_dist(sv, o, p, fmaxf(d1, 0.0f) + 2.0f * sv.og.delta);
+        o1 = d < d1 ? o : o1;
+        d2 = fminf(d2, fmaxf(d, d1));
+        d1 = fminf(d1, d);
+    }
+    // Whether the reference's query returns d1 (and, unless dist_only, o1).
+    __device__ __forceinline__ bool exact(const SceneView& sv, V p, bool dist_only) const {
+        if (og_exact(d1, d2, sv.og.delta, dist_only)) return true;
+        const int leaf = sv.fobj(o1).leaf;
+        if (leaf < 0) return dist_only || d2 > d1;
+        NoCount nc;
+        return og_exact_box(d1, d2, sqrtf(aabb_dist2(p, sv.node(leaf), nc)), dist_only);
+    }
+};
+
+// The 16-bit entries of a cell's list, taken one by one.
+struct OgList {
+    uint4 e;
+    __device__ __forceinline__ uint32_t head() const { return e.x & 0xffffu; }
+    __device__ __forceinline__ void pop() {
+        e.x = __funnelshift_r(e.x, e.y, 16);
+        e.y = __funnelshift_r(e.y, e.z, 16);
+        e.z = __funnelshift_r(e.z, e.w, 16);
+        e.w = (e.w >> 16) | 0xffff0000u;
+    }
+};
+
+// scene.rs:191-208 for one lane: the object grid's answer where it is the
+// reference's (objgrid.h), the reference's traversal elsewhere. The counting
+// kernels always traverse.
+template <class C>
+__device__ __forceinline__ DistHit dist_mat(const SceneView& sv, V p, C& cnt) {
+    cnt.add(CN_SDF);
+    if constexpr (sizeof(C) == 1) {
+        uint32_t cell;
+        if (sv.og.mode != kOgOff && og_cell(sv.og, p.x, p.y, p.z, cell)) {
+            OgBest b;
+            if (C::kTree3 || sv.og.mode == kOgMask) {
+                for (uint32_t m = __ldg(&sv.og.mask[cell]); m; m &= m - 1u) b.eval(sv, __ffs((int)m) - 1, p);
+            } else {
+                OgList l{__ldg(reinterpret_cast<const uint4*>(sv.og.list) + cell)};
+                for (uint32_t o = l.head(); o < kOgOverflow; l.pop(), o = l.head()) b.eval(sv, (int)o, p);
+            }
+            if (b.d1 < kMaxF && b.exact(sv, p, false)) return DistHit{b.d1, sv.obj(b.o1).mat};
+        }
+    }
+    return dist_mat_ref(sv, p, cnt);
+}
+
 template <class C>
 __device__ __forceinline__ float scene_dist(const SceneView& sv, V p, C& cnt) {
     return dist_mat(sv, p, cnt).d;
@@ -528,7 +623,7 @@ __device__ __forceinline__ DistHit dist_mat_warp3(const SceneView& sv, V p, bool
     return best;
 }
 
-// dist_mat for a whole warp (all 32 lanes call it; lanes with !active only
+// dist_mat_ref for a whole warp (all 32 lanes call it; lanes with !active only
 // take part in the votes). Each active lane runs its own near-first BVH
 // traversal with the reference's pruning, but leaves are evaluated in
 // warp-synchronous rounds: a lane advances through interior nodes until it
@@ -542,10 +637,9 @@ __device__ __forceinline__ DistHit dist_mat_warp3(const SceneView& sv, V p, bool
 // tests, object evaluations and best-distance updates is exactly the one
 // dist_mat() makes.
 template <class C>
-__device__ __forceinline__ DistHit dist_mat_warp(const SceneView& sv, V p, bool active, C& cnt) {
+__device__ __forceinline__ DistHit dist_mat_ref_warp(const SceneView& sv, V p, bool active, C& cnt) {
     DistHit best{kMaxF, 0u};
     if (active) {
-        cnt.add(CN_SDF);
         for (int i = 0; i < sv.n_planes; ++i) {
             const DObject o = sv.obj(i);
             float d = obj_dist(sv, o, p, cnt, best.d);
@@ -627,6 +721,51 @@ __device__ __forceinline__ DistHit dist_mat_warp(const SceneView& sv, V p, bool 
         }
     }
     return best;
+}
+
+// dist_mat for a whole warp (all 32 lanes call it; lanes with !active get
+// nothing). Scenes of few objects hold a mask per cell: the warp walks the
+// union of its lanes' masks, so that every lane evaluates the same object at
+// a time and the loads and the primitive code are uniform (an object that a
+// lane does not list can only be farther). Larger scenes hold a short list
+// per cell, which each lane walks by itself. The lanes that the grid cannot
+// answer exactly, outside it or at a near tie, take the reference's
+// traversal together. kDistOnly: only the distance is used, by a march that
+// stops at any value <= 0 alike; the material is then not set.
+//
+// The marches are bound by issued instructions, and the traversal spent most
+// of them on box tests, objects far from the point and lanes at different
+// leaves (a 512-object scene's visibility ran 10 of 32 lanes). Whole frames,
+// traversal -> grid with open_steps: Cornell box 5.61 -> 3.76 ms, 1920 x 1080
+// product scene 7.06 -> 5.66 ms, 512 objects at 961 x 541 97.8 -> 30.1 ms.
+template <bool kDistOnly, class C>
+__device__ __forceinline__ DistHit dist_warp(const SceneView& sv, V p, bool active, C& cnt) {
+    if (active) cnt.add(CN_SDF);
+    if constexpr (sizeof(C) == 1) {
+        if (sv.og.mode != kOgOff) {
+            uint32_t cell = 0;
+            bool ok = active && og_cell(sv.og, p.x, p.y, p.z, cell);
+            OgBest b;
+            if (C::kTree3 || sv.og.mode == kOgMask) {
+                uint32_t m = __reduce_or_sync(0xffffffffu, ok ? __ldg(&sv.og.mask[cell]) : 0u);
+                for (; m; m &= m - 1u) b.eval(sv, __ffs((int)m) - 1, p);
+            } else if (ok) {
+                OgList l{__ldg(reinterpret_cast<const uint4*>(sv.og.list) + cell)};
+                for (uint32_t o = l.head(); o < kOgOverflow; l.pop(), o = l.head()) b.eval(sv, (int)o, p);
+            }
+            DistHit h{b.d1, 0u};
+            ok = ok && b.d1 < kMaxF && b.exact(sv, p, kDistOnly);
+            if constexpr (!kDistOnly)
+                if (ok) h.mat = sv.obj(b.o1).mat;
+            const bool need = active && !ok;
+            if (__any_sync(0xffffffffu, need)) {
+                const DistHit r = dist_mat_ref_warp(sv, p, need, cnt);
+                if (need) h = r;
+            }
+            return h;
+        }
+    }
+    return dist_mat_ref_warp(sv, p, active, cnt);
 }
 
 // scene.rs:218-236: tetrahedron taps K = (1,-1,-1), (-1,-1,1), (-1,1,-1), (1,1,1).
@@ -722,54 +861,26 @@ __device__ __forceinline__ float soft_shadow(const SceneView& sv, V ro, V rd, fl
 }
 
 // ------------------------------------------------- resumable ray marches ----
-// The loops of trace() and soft_shadow() split into single steps, so that a
-// persistent kernel can advance many rays one SDF query at a time and refill
-// lanes whose ray ended. The arithmetic per step is exactly the loop body's.
+// The loops of trace.rs split into single steps, so that a persistent kernel
+// can advance many rays one SDF query at a time and refill lanes whose ray
+// ended.
 
-// trace.rs:84-124 as a state machine.
+// trace.rs:84-124 as a state machine. ph is the previous step's distance; a
+// march that skipped queries (open_steps) does not know it, and takes it at
+// the point before the step that turns out to need it (kPhNone, kPhBack).
 struct ShadowRay {
     V ro, rd;
     float t, tmax, k, res, ph;
     uint32_t steps;
+    float tp;  // kPhNone, kPhBack: the previous step's t
+    int mode;
 };
+enum : int { kPhKnown = 0, kPhNone = 1, kPhBack = 2 };
 __device__ __forceinline__ ShadowRay shadow_begin(V ro, V rd, float tmin, float tmax, float k) {
-    return ShadowRay{ro, rd, tmin, tmax, k, 1.0f, 1e20f, 0u};
+    return ShadowRay{ro, rd, tmin, tmax, k, 1.0f, 1e20f, 0u, 0.0f, kPhKnown};
 }
 // True when the march cannot take a first step (the loop body never runs).
 __device__ __forceinline__ bool shadow_done_before_start(const ShadowRay& s) { return !(s.t < s.tmax); }
-// One loop iteration. Returns true when the march has ended, with `vis` set.
-template <class C>
-__device__ __forceinline__ bool shadow_step(const SceneView& sv, ShadowRay& s, float& vis, C& cnt) {
-    float h = scene_dist(sv, s.ro + s.rd * s.t, cnt);
-    cnt.add(CN_SSTEP);
-    s.steps += 1;
-    if (h < 1e-4f) {
-        vis = 0.0f;
-        return true;
-    }
-    if (!cone_cannot_lower(h, s.t, s.k, s.res)) {
-        float y, d;
-        if (h < s.ph) {
-            y = h * h / (2.0f * s.ph);
-            d = sqrtf(fmaxf(h * h - y * y, 0.0f));
-        } else {
-            y = 0.0f;
-            d = h;
-        }
-        s.res = fminf(s.res, s.k * d / fmaxf(s.t - y, 1e-4f));
-    }
-    if (s.res < 1e-3f) {
-        vis = 0.0f;
-        return true;
-    }
-    s.ph = h;
-    s.t += clampr(h, 0.006f, 0.12f);
-    if (!(s.steps < kShadowSteps && s.t < s.tmax)) {
-        vis = clampr(s.res, 0.0f, 1.0f);
-        return true;
-    }
-    return false;
-}
 
 // trace.rs:27-58 as a state machine.
 struct TraceRay {
@@ -778,155 +889,97 @@ struct TraceRay {
     uint32_t steps;
 };
 enum : int { kMarching = 0, kHit = 1, kMiss = 2 };
-// One loop iteration. On kHit, `p`/`mat` are the hit and r.t its distance;
-// r.steps then includes the four normal taps (trace.rs:48).
-template <class C>
-__device__ __forceinline__ int trace_step(const SceneView& sv, TraceRay& r, V& p, uint32_t& mat, C& cnt) {
-    p = r.ro + r.rd * r.t;
-    DistHit h = dist_mat(sv, p, cnt);
-    cnt.add(CN_TSTEP);
-    r.steps += 1;
-    float eps = 1e-4f * fmaxf(r.t, 1.0f);
-    if (h.d < eps) {
-        mat = h.mat;
-        r.steps += 4;
-        return kHit;
-    }
-    r.t += h.d;
-    if (r.t > r.tmax || r.steps >= kMaxSteps) return kMiss;
-    return kMarching;
+// cone_cannot_lower with the previous distance known: this step's X from
+// approximate reciprocals, each of its parts with more slack than their error
+// (1e-3 of X, 1e-5 of the terms of t - y), compared by squares. NaN fails.
+__device__ __forceinline__ bool cone_above(float h, float ph, float t, float k, float res) {
+    const float y = h < ph ? __fdividef(h * h, 2.0f * ph) : 0.0f;
+    const float m = res * (fmaxf(t - y, 1e-4f) + 1e-5f * (t + h));
+    return k * k * (h * h - y * y) >= m * m * 1.001f;
 }
 
-// Scene::dist (scene.rs:211-213) for a cone-shadow step, through the cell's
-// candidate leaves instead of the BVH: the planes, then each listed leaf whose
-// box is nearer than best + tol, its objects' minimum taken with the same
-// strict `<`. Returns that minimum G; `ok` says whether G is exactly the value
-// the reference's pruned near-first query (bvh.rs:100-150) returns:
-//  * a leaf not listed, or listed but skipped, lies at least best + tol away,
-//    and every object's distance is at least its leaf box's distance less a
-//    rounding error far below tol (exact SDFs; measured below 3e-7 on the
-//    stress scene), so no object outside the evaluated leaves is below G;
-//  * the reference evaluates every plane, and reaches the leaf L1 holding G
-//    unless it prunes L1 or an ancestor, which needs a best <= box(L1) first;
-//    so G is its answer when G is a plane's, when box(L1) <= G, or when no
-//    other leaf or plane reaches box(L1) (then nothing can have pruned L1).
-// At or inside a surface (G <= 0) the value may differ from the reference's
-// but both are below every stopping threshold of the marches that use it
-// (shadow 1e-4, trace 1e-4 * max(t, 1)), so the march ends at the same step.
-// Otherwise (and outside the grid) ok is false and the caller asks the
-// reference query.
-__device__ __forceinline__ float dist_fast(const SceneView& sv, V p, bool& ok) {
-    NoCount nc;
-    const LeafGrid& g = sv.lg;
-    float P = kMaxF;
-    for (int i = 0; i < sv.n_planes; ++i) {
-        const float d = obj_dist(sv, sv.obj(i), p, nc);
-        if (d < P) P = d;
+// The steps after one at distance h that are certain to be open: the distance
+// is at least 0.12 (so the march advances exactly that, and neither stops nor
+// hits), and the cone term cannot lower res. They are taken without a query;
+// the distance after them is not known. Returns true when the march has
+// ended.
+__device__ __forceinline__ bool open_steps(ShadowRay& s, float h, float delta) {
+    for (float lower = og_open_first(h, delta); lower >= kOpenStep && cone_cannot_lower(lower, s.t, s.k, s.res);
+         lower = og_open_next(lower)) {
+        s.steps += 1;
+        s.tp = s.t;
+        s.mode = kPhNone;
+        s.t += kOpenStep;
+        if (!(s.steps < kShadowSteps && s.t < s.tmax)) return true;
     }
-    ok = false;
-    const float fx = (p.x - g.lo[0]) * g.inv_cell, fy = (p.y - g.lo[1]) * g.inv_cell,
-                fz = (p.z - g.lo[2]) * g.inv_cell;
-    if (!(fx >= 0.0f && fy >= 0.0f && fz >= 0.0f && fx < (float)g.dim[0] && fy < (float)g.dim[1] &&
-          fz < (float)g.dim[2]))
-        return P;
-    const uint32_t cell = (uint32_t)fx + (uint32_t)g.dim[0] * ((uint32_t)fy + (uint32_t)g.dim[1] * (uint32_t)fz);
-    const uint32_t e = __ldg(&g.start[cell + 1]);
-    float best = P, m1 = kMaxF, m2 = kMaxF, d2_1 = 0.0f;
-    for (uint32_t k = __ldg(&g.start[cell]); k < e; ++k) {
-        const DNode& nd = sv.node((int)__ldg(&g.leaf[k]));
-        const float d2 = aabb_dist2(p, nd, nc);
-        const float lim = best + g.tol;
-        if (!(lim > 0.0f) || d2 >= lim * lim) continue;
-        float m = kMaxF;
-        for (int j = nd.link; j < nd.link + nd.count; ++j) {
-            const float d = obj_dist(sv, sv.obj(j), p, nc);
-            if (d < m) m = d;
-        }
-        if (m < m1) {
-            m2 = m1;
-            m1 = m;
-            d2_1 = d2;
-        } else if (m < m2) {
-            m2 = m;
-        }
-        if (m < best) best = m;
-    }
-    const float G = P <= m1 ? P : m1;
-    // At or inside a surface: the reference's value is <= 0 too, or within
-    // rounding of it (a leaf can only be pruned against a best <= its box
-    // distance, which is ~0 here), so both stop the march at this step.
-    if (G <= 0.0f || P <= m1) {
-        ok = true;
-        return G;
-    }
-    const float v1 = sqrtf(d2_1);
-    ok = v1 <= m1 || (m2 > v1 && P > v1);
-    return m1;
+    return false;
 }
 
-// The distance a cone-shadow step needs, for a whole warp: dist_fast where
-// the scene has a leaf grid (uncounted kernels), the reference query for the
-// lanes it cannot answer exactly, dist_mat_warp everywhere else.
-template <class C>
-__device__ __forceinline__ float shadow_dist_w(const SceneView& sv, V p, bool active, C& cnt) {
-    if constexpr (sizeof(C) == 1 && !C::kTree3) {
-        if (sv.lg.enabled) {
-            bool ok = true;
-            float h = 0.0f;
-            if (active) h = dist_fast(sv, p, ok);
-            const bool need = active && !ok;
-            if (__any_sync(0xffffffffu, need)) {
-                const float r = dist_mat_warp(sv, p, need, cnt).d;
-                if (need) h = r;
-            }
-            return h;
-        }
-    }
-    return dist_mat_warp(sv, p, active, cnt).d;
-}
+// One step of a ray march for a whole warp: all 32 lanes call them, the SDF
+// query is dist_warp, and lanes with !active change nothing. The arithmetic
+// per step is exactly the loop body's.
 
-// Warp-collective forms of the two steps above: all 32 lanes call them, the
-// SDF query is dist_mat_warp (shadow_dist_w for the cone march), and lanes
-// with !active change nothing.
+// trace.rs:84-124. Returns true when the march has ended, with `vis` set.
 template <class C>
 __device__ __forceinline__ bool shadow_step_w(const SceneView& sv, ShadowRay& s, bool active, float& vis, C& cnt) {
-    const float h = shadow_dist_w(sv, s.ro + s.rd * s.t, active, cnt);
+    constexpr bool kSkips = sizeof(C) == 1;
+    const bool back = kSkips && s.mode == kPhBack;
+    float h = dist_warp<true>(sv, s.ro + s.rd * (back ? s.tp : s.t), active, cnt).d;
     if (!active) return false;
-    cnt.add(CN_SSTEP);
-    s.steps += 1;
-    if (h < 1e-4f) {
-        vis = 0.0f;
-        return true;
+    if (back) {
+        // The previous distance, now known, for the step whose own is in ph.
+        const float hs = s.ph;
+        s.ph = h;
+        h = hs;
+        s.mode = kPhKnown;
+    } else {
+        cnt.add(CN_SSTEP);
+        s.steps += 1;
+        if (h < 1e-4f) {
+            vis = 0.0f;
+            return true;
+        }
     }
     if (!cone_cannot_lower(h, s.t, s.k, s.res)) {
-        float y, d;
-        if (h < s.ph) {
-            y = h * h / (2.0f * s.ph);
-            d = sqrtf(fmaxf(h * h - y * y, 0.0f));
-        } else {
-            y = 0.0f;
-            d = h;
+        if (kSkips && s.mode == kPhNone) {
+            s.ph = h;
+            s.mode = kPhBack;
+            return false;
         }
-        s.res = fminf(s.res, s.k * d / fmaxf(s.t - y, 1e-4f));
+        if (!kSkips || !cone_above(h, s.ph, s.t, s.k, s.res)) {
+            float y, d;
+            if (h < s.ph) {
+                y = h * h / (2.0f * s.ph);
+                d = sqrtf(fmaxf(h * h - y * y, 0.0f));
+            } else {
+                y = 0.0f;
+                d = h;
+            }
+            s.res = fminf(s.res, s.k * d / fmaxf(s.t - y, 1e-4f));
+            if (s.res < 1e-3f) {
+                vis = 0.0f;
+                return true;
+            }
+        }
     }
-    if (s.res < 1e-3f) {
-        vis = 0.0f;
-        return true;
-    }
+    s.mode = kPhKnown;
     s.ph = h;
     s.t += clampr(h, 0.006f, 0.12f);
-    if (!(s.steps < kShadowSteps && s.t < s.tmax)) {
+    if (!(s.steps < kShadowSteps && s.t < s.tmax) ||
+        (kSkips && sv.og.mode != kOgOff && open_steps(s, h, sv.og.delta))) {
         vis = clampr(s.res, 0.0f, 1.0f);
         return true;
     }
     return false;
 }
 
+// trace.rs:27-58. On kHit, `p`/`mat` are the hit and r.t its distance;
+// r.steps then includes the four normal taps (trace.rs:48).
 template <class C>
 __device__ __forceinline__ int trace_step_w(const SceneView& sv, TraceRay& r, bool active, V& p, uint32_t& mat,
                                             C& cnt) {
     p = r.ro + r.rd * r.t;
-    const DistHit h = dist_mat_warp(sv, p, active, cnt);
+    const DistHit h = dist_warp<false>(sv, p, active, cnt);
     if (!active) return kMarching;
     cnt.add(CN_TSTEP);
     r.steps += 1;
@@ -942,11 +995,10 @@ __device__ __forceinline__ int trace_step_w(const SceneView& sv, TraceRay& r, bo
 }
 
 // trace_step_w for marches that need only hit or miss and the step count
-// (the hemisphere closure, trace.rs:165-186): the query is shadow_dist_w's,
-// whose value is the reference's exactly, so the march is the same.
+// (the hemisphere closure, trace.rs:165-186): the query needs no material.
 template <class C>
 __device__ __forceinline__ int trace_step_dist_w(const SceneView& sv, TraceRay& r, bool active, C& cnt) {
-    const float hd = shadow_dist_w(sv, r.ro + r.rd * r.t, active, cnt);
+    const float hd = dist_warp<true>(sv, r.ro + r.rd * r.t, active, cnt).d;
     if (!active) return kMarching;
     cnt.add(CN_TSTEP);
     r.steps += 1;

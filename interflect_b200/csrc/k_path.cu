@@ -37,7 +37,7 @@ __device__ __forceinline__ V cosine_hemisphere(V n, Pcg32& rng, const float2* si
 }
 
 // reference.rs:61-137 as a per-lane state machine, so that every loop
-// iteration is one warp-synchronous SDF query (dist_mat_warp) for whatever
+// iteration is one warp-synchronous SDF query (dist_warp) for whatever
 // each lane marches at that moment: its camera or bounce ray, one of the four
 // normal taps at a hit, or the hard shadow ray toward a light. A lane that
 // finishes a march moves on at once (next light, next bounce, next sample,
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(128) k_path(ShadeParams P, uint32_t spp, const
         const float kx = (tap == 0 || tap == 3) ? 1.0f : -1.0f, ky = tap >= 2 ? 1.0f : -1.0f,
                     kz = (tap == 1 || tap == 3) ? 1.0f : -1.0f;
         const V qp = phase == kPhTap ? hp + V{kx, ky, kz} * 5e-4f : ray.ro + ray.rd * ray.t;
-        const DistHit h = dist_mat_warp(sv, qp, active, cnt);
+        const DistHit h = dist_warp<false>(sv, qp, active, cnt);
         if (!active) continue;
 
         // Where the lane goes after this query.

@@ -25,7 +25,7 @@ __device__ __forceinline__ bool scene_prologue(const BlobRef& blob, uint8_t* dsm
                                                uint32_t* status, SceneView& sv) {
     sv = make_view(blob.ptr);
     sv.status = status;
-    sv.lg = blob.lg;
+    sv.og = blob.og;
     uint32_t used = 0;
     if (blob.staged) {
         if (!stage_scene(blob.ptr, blob.stage_bytes, dsmem, mbar, status, blob.wait_polls)) return false;
@@ -33,6 +33,7 @@ __device__ __forceinline__ bool scene_prologue(const BlobRef& blob, uint8_t* dsm
         sv.objs = s.objs;
         sv.prims = s.prims;
         sv.nodes = s.nodes;
+        sv.fast = s.fast;
         used = align16(blob.stage_bytes);
     }
     uint32_t* stk = reinterpret_cast<uint32_t*>(dsmem + used);

@@ -5,14 +5,15 @@
 #include <cuda_runtime.h>
 
 #include "layout.h"
+#include "objgrid.h"
 
 namespace ifx {
 
 struct GatherView;
 
 // Program blob as handed to every tracing kernel. When `staged` is set the
-// kernel copies its geometry prefix (header, objects, primitives, BVH nodes:
-// the first stage_bytes bytes, all the ray marches read) into dynamic shared
+// kernel copies its geometry prefix (header, objects, primitives, BVH nodes,
+// packed objects: the first stage_bytes bytes, all the ray marches read) into dynamic shared
 // memory; lights, materials and the linear order are always read from global
 // memory. Unstaged (large) scenes are read from global memory through L1.
 struct BlobRef {
@@ -23,7 +24,7 @@ struct BlobRef {
     int stack_depth;  // BVH traversal stack entries per thread (tree depth + 2)
     uint32_t wait_polls;  // poll budget of the staging wait (kDefaultWaitPolls unless the host lowers it)
     int tree3;            // BVH in use and made of a root and two leaves: the NoCount3 kernels apply
-    LeafGrid lg;          // enabled only for the scenes dist_fast serves (large BVHs)
+    ObjGrid og;           // candidate objects per cell (objgrid.h); mode kOgOff where it does not apply
 };
 
 // Default poll budget of every bounded device-side wait (the scene-staging
@@ -363,14 +364,10 @@ void configure_solve_kernels(int max_dyn_smem);
 void configure_shade_kernels(int max_dyn_smem);
 void configure_diff_kernels(int max_dyn_smem);
 void configure_path_kernels(int max_dyn_smem);
-void configure_leafgrid_kernels(int max_dyn_smem);
-// The leaf grid (k_leafgrid.cu): per-cell bounds U, then the lists (count
-// pass with start == nullptr, fill pass with the scanned starts).
-void launch_lg_bound(cudaStream_t st, const BlobRef& blob, const LeafGrid& g, float cell, float half_diag,
-                     uint32_t ncells, float* U, uint32_t* status);
-void launch_lg_lists(cudaStream_t st, const uint8_t* blob, const LeafGrid& g, double cell, double pad, uint32_t ncells,
-                     const float* U, const uint32_t* leaves, uint32_t nleaf, uint32_t* count, const uint32_t* start,
-                     uint32_t* out, float* key);
+// The object grid (objgrid.h) of the staged scene: lo is the grid's corner,
+// cell its cells' side; g.mode picks which of mask and list is written.
+void launch_og_build(cudaStream_t st, const BlobRef& blob, const ObjGrid& g, const float lo[3], float cell,
+                     uint32_t* mask, uint4* list, uint32_t* status);
 // The path-traced reference mode (k_path.cu): p.film / p.out8 receive the
 // frame; sincos holds (sinf, cosf) of the 2^24 sampler angles.
 int launch_path(cudaStream_t st, const ShadeParams& p, uint32_t spp, const float2* sincos,
@@ -382,7 +379,6 @@ inline void configure_kernels(int max_dyn_smem) {
     configure_shade_kernels(max_dyn_smem);
     configure_diff_kernels(max_dyn_smem);
     configure_path_kernels(max_dyn_smem);
-    configure_leafgrid_kernels(max_dyn_smem);
 }
 
 }  // namespace ifx

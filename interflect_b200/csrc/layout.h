@@ -3,12 +3,14 @@
 // A scene becomes one contiguous, 16-byte aligned "program" blob that every
 // tracing kernel copies into shared memory once per CTA (one bulk copy):
 //
-//   BlobHeader                      64 B
+//   BlobHeader                      80 B
 //   DObject[n_planes + n_objects]   16 B each: planes first, then the
 //                                   bounded objects in BVH leaf order
 //   DPrim[n_prims]                  64 B each: an object's base primitive
 //                                   followed by its subtracted primitives
 //   DNode[n_nodes]                  32 B each: flattened BVH, left child = i+1
+//   DFast[n_planes + n_objects]     48 B each: the same objects, packed for
+//                                   the object grid's queries
 //   DQuadLight[n_lights]           160 B each
 //   DSphereLight[n_sphere_lights]   32 B each
 //   DMaterial[n_materials]          64 B each (index 0 = default material)
@@ -54,6 +56,27 @@ struct alignas(16) DObject {
     float smooth;    // smooth-subtraction radius (extension); 0 = max(d, -s)
 };
 
+// One stored object as the object grid's queries read it: two or three 16-byte
+// loads by object index, with no primitive index or kind to look up first.
+// Spheres and tori take the box's form (device.cuh fast_dist), so that lanes
+// at different objects run the same instructions; objects with subtractions
+// are evaluated from their DObject.
+enum FastTag : int32_t {
+    F_BOX = 0,      // box, or a sphere as a box of no extent
+    F_TORUS = 1,    // b.x = major radius
+    F_BOX_ROT = 2,  // c = (cos, sin)
+    F_PLANE = 3,    // a = (normal, height)
+    F_CAPSULE = 4,  // a = (a, radius), b = b - a, c.x = dot(b, b)
+    F_GENERAL = 5,  // as the DObject says
+};
+struct alignas(16) DFast {
+    float a[4];      // centre, radius
+    float b[3];      // half-extent less the rounding radius
+    int32_t tag;
+    float c[3];
+    int32_t leaf;    // BVH leaf holding the object; -1 for a plane
+};
+
 struct alignas(16) DNode {
     float lo[3];
     int32_t count;   // > 0: leaf with `count` objects starting at `link`
@@ -88,22 +111,7 @@ struct alignas(16) BlobHeader {
     int32_t n_lights, n_sphere_lights, n_materials, use_bvh;
     uint32_t off_objects, off_prims, off_nodes, off_lights;
     uint32_t off_sphere_lights, off_materials, off_linear, total_bytes;
-};
-
-// Candidate leaves per cell of a uniform grid over the scene, used by the
-// distance-only queries of cone-shadow marches in large BVHs (device.cuh,
-// dist_fast). A cell lists every BVH leaf whose box comes within
-// U(cell) + 2 tol of the cell, U(cell) being the reference's distance at the
-// cell centre plus the cell's half-diagonal (an upper bound of the nearest
-// distance anywhere in the cell); leaves appear nearest-first.
-struct LeafGrid {
-    const uint32_t* start;  // per cell: first entry of its list; start[ncells] = total
-    const uint32_t* leaf;   // BVH node index of each listed leaf
-    float lo[3];
-    float inv_cell;
-    int dim[3];
-    float tol;              // pruning margin, far above any f32 rounding of the distances
-    int enabled;
+    uint32_t off_fast, pad[3];
 };
 
 // Per-scene scalars passed to kernels by value.

@@ -1,0 +1,123 @@
+// The object grid: for each cell of a uniform grid over the scene, the stored
+// objects that can be nearest to a point of the cell. A distance query then
+// evaluates one or two objects (1.2 listed per cell in the product and Cornell
+// scenes, 1.9 in the 512-object stress scene) instead of traversing the BVH,
+// and answers the reference's traversal exactly or says that it cannot.
+//
+// The rules, shared by the kernels and by the CPU check against the
+// reference's traversal (tests/cpp/objgrid_check.cpp):
+//
+//  * Every admitted object's distance function is 1-Lipschitz and is nowhere
+//    below the distance to its BVH leaf's box (leaf box distance 0 inside),
+//    but for f32 rounding, which delta exceeds: delta is 2^-16 of the largest
+//    coordinate, length or radius in the scene plus its diagonal, about 32
+//    times what eight roundings at that scale amount to.
+//  * A cell lists every object whose distance at the cell's centre is at most
+//    max(the nearest distance there, 0) + og_margin. An object that is not
+//    listed is then, everywhere in the cell, farther than max(G, 0) + 3 delta,
+//    G being the nearest distance at that point.
+//  * The query returns the smallest listed distance d1, its object o1, and d2,
+//    the second smallest. If d2 > max(d1, 0) + delta, the reference's query
+//    (bvh.rs:100-150: prune a node when its box distance >= the best so far,
+//    objects by strict <) returns exactly (d1, o1): every other object is
+//    farther than any box distance on o1's path in the tree, which is at most
+//    max(d1, 0) plus rounding, so o1 cannot have been pruned, and no other
+//    object is as near.
+//  * A march that only stops at a surface needs no more than that the point is
+//    inside: at d1 <= -delta the point is inside o1's box, so the reference
+//    either evaluates o1 or pruned it against a best <= 0.
+//  * At a near tie, the distance v1 to o1's leaf's box decides (the boxes on
+//    o1's path are no farther): if d2 > v1 nothing can have pruned o1; if
+//    v1 <= d1, only an object as near as o1 can. Planes are never pruned.
+// Anything else (points outside the grid, ties within rounding of a box that
+// both objects touch) asks the reference query.
+//
+// The same conditions let a cone-shadow march (trace.rs:84-124) skip queries:
+// it advances 0.12 wherever the distance is at least that, and the distance
+// changes by at most the step, so that a distance h guarantees the next
+// (h - 0.12) / 0.12 steps.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#define IFX_OG_FN __host__ __device__ __forceinline__
+#else
+#define IFX_OG_FN inline
+#endif
+
+namespace ifx {
+
+struct ObjGrid {
+    const uint32_t* mask;  // kOgMask: per cell, bit i = stored object i is listed
+    const uint32_t* list;  // kOgList: per cell, eight 16-bit stored-object indices, nearest first, kOgNone-padded
+    float inv;             // cells per unit length
+    float bias[3];         // -lo * inv - 0.5: the cell index is the nearest integer to p * inv + bias
+    uint32_t dim[3];
+    float delta;
+    int mode;              // kOgOff, kOgMask, kOgList
+};
+enum : int { kOgOff = 0, kOgMask = 1, kOgList = 2 };
+// Scenes of at most this many stored objects (planes and bounded) use masks.
+static constexpr uint32_t kOgMaskObjects = 32;
+static constexpr uint32_t kOgMaxObjects = 32768;
+static constexpr uint32_t kOgListLen = 8;
+static constexpr uint32_t kOgNone = 0xffffu;      // end of a list
+static constexpr uint32_t kOgOverflow = 0xfffeu;  // first entry of a cell with more than kOgListLen objects
+
+IFX_OG_FN uint32_t og_bits(float x) {
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(x);
+#else
+    uint32_t u;
+    std::memcpy(&u, &x, 4);
+    return u;
+#endif
+}
+
+// One coordinate's cell: adding 2^23 rounds to the nearest integer, whose
+// bits then follow from 2^23's. Negative, huge and NaN coordinates give an
+// index no grid has.
+IFX_OG_FN uint32_t og_axis(float p, float inv, float bias) {
+    return og_bits(fmaf(p, inv, bias) + 8388608.0f) - 0x4B000000u;
+}
+
+IFX_OG_FN bool og_cell(const ObjGrid& g, float x, float y, float z, uint32_t& cell) {
+    const uint32_t i = og_axis(x, g.inv, g.bias[0]), j = og_axis(y, g.inv, g.bias[1]),
+                   k = og_axis(z, g.inv, g.bias[2]);
+    cell = i + g.dim[0] * (j + g.dim[1] * k);
+    return i < g.dim[0] && j < g.dim[1] && k < g.dim[2];
+}
+
+// Half-diagonal of a cube of side `side`, with room for the rounding of the
+// cell index and of the centre.
+IFX_OG_FN float og_half(float side, float delta) { return side * 0.8660255f + delta; }
+
+// The listing margin over a cell of half-diagonal `half`: the nearest distance
+// and an object's distance can each change by `half` between the centre and a
+// point of the cell.
+IFX_OG_FN float og_margin(float half, float delta) { return 2.0f * half + 4.0f * delta; }
+
+IFX_OG_FN bool og_listed(float d, float nearest, float margin) { return !(d > fmaxf(nearest, 0.0f) + margin); }
+
+// dist_only: the caller uses the distance to march and stops at any value
+// <= 0 alike.
+IFX_OG_FN bool og_exact(float d1, float d2, float delta, bool dist_only) {
+    return d2 > fmaxf(d1, 0.0f) + delta || (dist_only && d1 <= -delta);
+}
+
+// og_exact at a near tie: v1 is the distance to o1's leaf's box.
+IFX_OG_FN bool og_exact_box(float d1, float d2, float v1, bool dist_only) {
+    return (d2 > v1 && d2 > d1) || (v1 <= d1 && (dist_only || d2 > d1));
+}
+
+// What a distance h at one point of a cone-shadow march says of the distance
+// one 0.12 step on (rounding of the step, the position and h included), and
+// what that says of the step after.
+static constexpr float kOpenStep = 0.12f;
+IFX_OG_FN float og_open_first(float h, float delta) { return h - 0.12002f - 4.0f * delta; }
+IFX_OG_FN float og_open_next(float lower) { return lower - 0.12002f; }
+
+}  // namespace ifx

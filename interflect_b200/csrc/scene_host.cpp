@@ -754,6 +754,42 @@ std::vector<uint8_t> flatten_scene(const HScene& s) {
     for (DNode& n : nodes)
         if (n.count > 0) n.link += (int32_t)s.planes.size();
 
+    // The objects as the object grid's queries read them.
+    std::vector<DFast> fast(objs.size());
+    for (size_t i = 0; i < objs.size(); ++i) {
+        DFast& f = fast[i];
+        memset(&f, 0, sizeof f);
+        f.leaf = -1;
+        const DPrim& p = prims[(size_t)objs[i].prim];
+        const float* v = p.v;
+        f.tag = F_GENERAL;
+        if (objs[i].nsub > 0) continue;
+        if (p.kind == K_SPHERE || p.kind == K_PLANE) {
+            f.tag = p.kind == K_SPHERE ? F_BOX : F_PLANE;
+            memcpy(f.a, v, 16);
+        } else if (p.kind == K_BOX || p.kind == K_BOX_ROT) {
+            f.tag = p.kind == K_BOX ? F_BOX : F_BOX_ROT;
+            memcpy(f.a, v, 12);
+            memcpy(f.b, v + 3, 12);
+            f.a[3] = v[6];
+            f.c[0] = v[7];
+            f.c[1] = v[8];
+        } else if (p.kind == K_TORUS) {
+            f.tag = F_TORUS;
+            memcpy(f.a, v, 12);
+            f.a[3] = v[4];
+            f.b[0] = v[3];
+        } else if (p.kind == K_CAPSULE) {
+            f.tag = F_CAPSULE;
+            memcpy(f.a, v, 12);
+            f.a[3] = v[7];
+            memcpy(f.b, v + 3, 12);
+            f.c[0] = v[6];
+        }
+    }
+    for (size_t n = 0; n < nodes.size(); ++n)
+        for (int32_t k = 0; k < nodes[n].count; ++k) fast[(size_t)(nodes[n].link + k)].leaf = (int32_t)n;
+
     std::vector<DQuadLight> ql;
     for (const HQuadLight& l : s.lights) {
         DQuadLight d;
@@ -821,6 +857,8 @@ std::vector<uint8_t> flatten_scene(const HScene& s) {
     off += align16((uint32_t)(prims.size() * sizeof(DPrim)));
     h.off_nodes = off;
     off += align16((uint32_t)(nodes.size() * sizeof(DNode)));
+    h.off_fast = off;
+    off += align16((uint32_t)(fast.size() * sizeof(DFast)));
     h.off_lights = off;
     off += align16((uint32_t)(ql.size() * sizeof(DQuadLight)));
     h.off_sphere_lights = off;
@@ -838,6 +876,7 @@ std::vector<uint8_t> flatten_scene(const HScene& s) {
     put(h.off_objects, objs.data(), objs.size() * sizeof(DObject));
     put(h.off_prims, prims.data(), prims.size() * sizeof(DPrim));
     put(h.off_nodes, nodes.data(), nodes.size() * sizeof(DNode));
+    put(h.off_fast, fast.data(), fast.size() * sizeof(DFast));
     put(h.off_lights, ql.data(), ql.size() * sizeof(DQuadLight));
     put(h.off_sphere_lights, sl.data(), sl.size() * sizeof(DSphereLight));
     put(h.off_materials, mats.data(), mats.size() * sizeof(DMaterial));
