@@ -164,7 +164,7 @@ struct ifx_ctx {
     // scratch
     DBuf cub_tmp, small;  // small: 8 x u64 counters / results
     DBuf gen_cand, gen_keep, gen_off, gen_head, gen_pts, gen_next, gen_state, gen_out;  // surfel generation
-    DBuf gen_head_acc, gen_next_acc;
+    DBuf gen_head_acc, gen_next_acc, gen_rank, gen_st;
 
     // measurement: per-kernel events, work counters (IFX_NUM_KERNELS x 21 u64), timer
     cudaEvent_t kv0 = nullptr, kv1 = nullptr, kc0 = nullptr, kc1 = nullptr, tm0 = nullptr, tm1 = nullptr;
@@ -476,7 +476,8 @@ extern "C" void ifx_ctx_destroy(ifx_ctx* ctx) {
                     &ctx->sell_rows, &ctx->sell_sizes, &ctx->sell_off, &ctx->sell_idx, &ctx->sell_w,
                     &ctx->path_sincos, &ctx->shsc, &ctx->lff, &ctx->lvis, &ctx->lq, &ctx->lsc,
                     &ctx->vkey, &ctx->vkey_alt, &ctx->vval, &ctx->vval_alt, &ctx->ckey, &ctx->ckey_alt,
-                    &ctx->cval, &ctx->cval_alt, &ctx->msum, &ctx->gen_head_acc, &ctx->gen_next_acc, &ctx->og_cells};
+                    &ctx->cval, &ctx->cval_alt, &ctx->msum, &ctx->gen_head_acc, &ctx->gen_next_acc, &ctx->gen_rank, &ctx->gen_st,
+                    &ctx->og_cells};
     for (DBuf* b : bufs) free_buf(*b);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     for (cudaEvent_t ev : {ctx->ev0, ctx->ev1, ctx->kv0, ctx->kv1, ctx->kc0, ctx->kc1, ctx->tm0, ctx->tm1})
@@ -794,11 +795,8 @@ extern "C" int ifx_surfels_download(ifx_ctx* ctx, float* p, float* nrm, float* a
     return IFX_OK;
 }
 
-// surfel.rs:147-255. The projection of every Halton seed runs on the GPU in
-// chunks; the Poisson-disc test is inherently sequential in seed order (a
-// seed is rejected by any earlier accepted surfel within d_min) and runs on
-// the host over the projected points, chunk by chunk, until `target`
-// surfels are placed.
+// surfel.rs:147-255. The Halton seeds are projected in chunks and thinned in
+// batches, in seed order, until `target` surfels are placed.
 extern "C" int ifx_surfels_generate(ifx_ctx* ctx, uint64_t target, uint64_t* placed) {
     if (!ctx || !ctx->has_scene) return fail(ctx, IFX_ERR_INVALID, "no scene uploaded");
     if (target == 0 || target > 2000000ull) return fail(ctx, IFX_ERR_LIMIT, "surfel target out of range");
@@ -822,11 +820,13 @@ extern "C" int ifx_surfels_generate(ifx_ctx* ctx, uint64_t target, uint64_t* pla
 
     // Seeds are projected and thinned on the GPU in batches of consecutive
     // indices (k_surfels.cu); the host only reads each batch's counts.
-    const uint32_t kChunk = 1u << 18;
+    const uint32_t kChunk = 1u << 18;       // seeds projected at a time
+    const uint32_t kFirstBatch = 1u << 12;  // seeds thinned in the first batch
     const size_t ncells = (size_t)dim[0] * (size_t)dim[1] * (size_t)dim[2];
     ENSURE(ctx->gen_cand, (size_t)kChunk * sizeof(float4));
     ENSURE(ctx->gen_keep, ((size_t)kChunk + 1) * 4);
     ENSURE(ctx->gen_off, ((size_t)kChunk + 1) * 4);
+    ENSURE(ctx->gen_rank, ((size_t)kChunk + 1) * 4);
     ENSURE(ctx->gen_head, ncells * 4);
     ENSURE(ctx->gen_head_acc, ncells * 4);
     ENSURE(ctx->gen_next_acc, (size_t)seeds * 4);
@@ -851,54 +851,62 @@ extern "C" int ifx_surfels_generate(ifx_ctx* ctx, uint64_t target, uint64_t* pla
     g.state = (uint32_t*)ctx->gen_state.p;
     g.cap = seeds;
     g.err = (uint32_t*)ctx->status.p;
+    ENSURE(ctx->gen_st, sizeof(GenState));
+    CK(cudaMemsetAsync(ctx->gen_st.p, 0, sizeof(GenState), ctx->st));
+    g.st = (GenState*)ctx->gen_st.p;
     uint32_t* keep = (uint32_t*)ctx->gen_keep.p;
     uint32_t* off = (uint32_t*)ctx->gen_off.p;
-    unsigned long long* small = (unsigned long long*)ctx->small.p;
-    uint32_t* undecided = (uint32_t*)&small[5];
-    uint32_t base = 0;    // points kept so far (all batches)
-    uint64_t placed_n = 0;
+    uint32_t* rank = (uint32_t*)ctx->gen_rank.p;
+    uint32_t placed_n = 0;
     for (uint32_t s0 = 0; s0 < seeds && placed_n < target; s0 += kChunk) {
-        const uint32_t cnt = seeds - s0 < kChunk ? seeds - s0 : kChunk;
-        launch_gen_project(ctx->st, ctx->blobref, ctx->sc, s0, cnt, eps, (float4*)ctx->gen_cand.p,
+        const uint32_t chunk = seeds - s0 < kChunk ? seeds - s0 : kChunk;
+        launch_gen_project(ctx->st, ctx->blobref, ctx->sc, s0, chunk, eps, (float4*)ctx->gen_cand.p,
                            (uint32_t*)ctx->status.p);
         ctx->launches++;
-        ctx->launches += (uint64_t)launch_gen_filter(ctx->st, g, (const float4*)ctx->gen_cand.p, cnt, keep);
-        CK(cudaMemsetAsync(keep + cnt, 0, 4, ctx->st));
         CKL();
-        CUB([&](void* t, size_t& bb) { return cub::DeviceScan::ExclusiveSum(t, bb, keep, off, (int)cnt + 1, ctx->st); });
-        ctx->launches += (uint64_t)launch_gen_append(ctx->st, g, (const float4*)ctx->gen_cand.p, keep, off, cnt, base);
-        uint32_t kept = 0;
-        CK(cudaMemcpyAsync(&kept, off + cnt, 4, cudaMemcpyDeviceToHost, ctx->st));
-        int r = check_status(ctx);  // synchronises
-        if (r) return r;
-        if (kept == 0) continue;
-        // Rounds until every point of the batch is decided; each round
-        // decides at least the earliest open point, so kept rounds suffice.
-        for (uint32_t round = 0;; ++round) {
-            if (round > kept) return fail(ctx, IFX_ERR_TIMEOUT, "Poisson thinning did not settle");
-            CK(cudaMemsetAsync(undecided, 0, 4, ctx->st));
-            ctx->launches += (uint64_t)launch_gen_resolve(ctx->st, g, base, kept, undecided);
+        // Thinning batches of the chunk: as long as all seeds before them.
+        for (uint32_t b0 = 0; b0 < chunk && placed_n < target;) {
+            const uint32_t want = s0 + b0 > kFirstBatch ? s0 + b0 : kFirstBatch;
+            const uint32_t cnt = chunk - b0 < want ? chunk - b0 : want;
+            const float4* cand = (const float4*)ctx->gen_cand.p + b0;
+            ctx->launches += (uint64_t)launch_gen_filter(ctx->st, g, cand, cnt, keep);
+            CK(cudaMemsetAsync(keep + cnt, 0, 4, ctx->st));
             CKL();
-            uint32_t open = 0;
-            CK(cudaMemcpyAsync(&open, undecided, 4, cudaMemcpyDeviceToHost, ctx->st));
-            CK(cudaStreamSynchronize(ctx->st));
-            if (open == 0) break;
+            CUB([&](void* t, size_t& bb) {
+                return cub::DeviceScan::ExclusiveSum(t, bb, keep, off, (int)cnt + 1, ctx->st);
+            });
+            ctx->launches += (uint64_t)launch_gen_append(ctx->st, g, cand, keep, off, cnt);
+            // Rounds until every point of the batch is decided, kGenRounds at
+            // a time; each round decides at least the earliest open point, so
+            // as many rounds as points suffice.
+            GenState h{};
+            for (uint32_t round = 0;; round += kGenRounds) {
+                if (round > cnt) return fail(ctx, IFX_ERR_TIMEOUT, "Poisson thinning did not settle");
+                if (round) CK(cudaMemsetAsync(g.st->open, 0, sizeof h.open, ctx->st));
+                for (int k = 0; k < kGenRounds; ++k)
+                    ctx->launches += (uint64_t)launch_gen_resolve(ctx->st, g, off, cnt, k);
+                // Accepted points in seed order, up to the target (surfel.rs:184-186).
+                ctx->launches += (uint64_t)launch_gen_accept_flags(ctx->st, g, off, cnt, keep);
+                CKL();
+                CUB([&](void* t, size_t& bb) {
+                    return cub::DeviceScan::ExclusiveSum(t, bb, keep, rank, (int)cnt + 1, ctx->st);
+                });
+                ctx->launches += (uint64_t)launch_gen_emit(ctx->st, g, off, cnt, rank, (uint32_t)target,
+                                                           (float4*)ctx->gen_out.p);
+                ctx->launches += (uint64_t)launch_gen_advance(ctx->st, g, off, cnt, rank, (uint32_t)target);
+                CKL();
+                CK(cudaMemcpyAsync(&h, g.st, sizeof h, cudaMemcpyDeviceToHost, ctx->st));
+                int r = check_status(ctx);  // synchronises
+                if (r) return r;
+                bool decided = false;
+                for (uint32_t o : h.open) decided |= o == 0;
+                if (decided) break;
+            }
+            placed_n = h.placed;
+            b0 += cnt;
         }
-        // Accepted points in seed order, up to the target (surfel.rs:184-186).
-        ctx->launches += (uint64_t)launch_gen_accept_flags(ctx->st, g, base, kept, keep);
-        CUB([&](void* t, size_t& bb) { return cub::DeviceScan::ExclusiveSum(t, bb, keep, off, (int)kept + 1, ctx->st); });
-        uint32_t acc_n = 0;
-        CK(cudaMemcpyAsync(&acc_n, off + kept, 4, cudaMemcpyDeviceToHost, ctx->st));
-        const uint32_t quota = (uint32_t)(target - placed_n);
-        ctx->launches += (uint64_t)launch_gen_emit(ctx->st, g, base, kept, off, quota,
-                                                   (float4*)ctx->gen_out.p + placed_n);
-        ctx->launches += (uint64_t)launch_gen_retire(ctx->st, g, base, kept);
-        CKL();
-        if ((r = check_status(ctx))) return r;
-        placed_n += acc_n < quota ? acc_n : quota;
-        base += kept;
     }
-    const uint32_t n = (uint32_t)placed_n;
+    const uint32_t n = placed_n;
     size_t b = (size_t)n * sizeof(float4);
     ENSURE(ctx->sp, b);
     ENSURE(ctx->sn, b);

@@ -8,13 +8,22 @@ namespace ifx {
 // on-surface and in-bounds tests. Writes the projected point with w = 1 if
 // the seed survives, w = 0 otherwise. The Poisson-disc thinning that follows
 // (below) keeps the reference's seed-order semantics.
+//
+// Consecutive Halton points lie far apart, points whose indices differ by a
+// multiple of 32 * 9 * 25 in the same 1/32 x 1/9 x 1/25 box of the bounds:
+// lanes take the chunk's seeds in that stride, so that a warp's points meet
+// the same objects and take similar numbers of steps.
+static constexpr uint32_t kGenStride = 32u * 9u * 25u;
 __global__ void __launch_bounds__(128) k_gen_project(BlobRef blob, SceneConsts sc, uint32_t seed0,
                                                       uint32_t count, float eps, float4* out, uint32_t* status) {
     IFX_SCENE_PROLOGUE(blob, status, sv);
     NoCount nc;
     const V lo{sc.lo[0], sc.lo[1], sc.lo[2]}, hi{sc.hi[0], sc.hi[1], sc.hi[2]};
     const float diag = sc.diag;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x) {
+    const uint32_t per = (count + kGenStride - 1u) / kGenStride, total = per * kGenStride;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
+        const uint32_t j = (k % per) * kGenStride + k / per;
+        if (j >= count) continue;
         uint32_t i = seed0 + j;
         V s{radical_inverse(i + 1, 2), radical_inverse(i + 1, 3), radical_inverse(i + 1, 5)};
         V p = lo + (hi - lo) * s;
@@ -68,9 +77,13 @@ __global__ void __launch_bounds__(128) k_gen_finalize(BlobRef blob, const float4
 //            information, so the fixed point is the sequential result and
 //            does not depend on scheduling; each round decides at least the
 //            earliest open point;
-//   retire   the batch's accepted points join the accepted-point lists that
-//            later filters walk, and the batch lists are emptied, so that no
-//            walk ever passes a rejected point.
+//   emit     the batch's accepted points go out and join the accepted-point
+//            lists that later filters walk, and the batch lists are emptied,
+//            so that no walk ever passes a rejected point.
+// A batch is as long as all seeds before it (within limits the host sets), so
+// that its lists stay short: seeds project in thousands onto the same edges
+// and corners, and a first batch of 2^18 walked lists of thousands for each of
+// thousands (0.73 ms a round, 33 of the 50 ms that 4.8M seeds took).
 // Lists are walked with a bound (the point capacity); an over-long walk sets
 // kStatusGenWalk.
 __device__ __forceinline__ int gen_cell(const GenGrid& g, float v, int a) {
@@ -127,8 +140,9 @@ __global__ void k_gen_filter(GenGrid g, const float4* cand, uint32_t cnt, uint32
     }
 }
 
-__global__ void k_gen_append(GenGrid g, const float4* cand, const uint32_t* keep, const uint32_t* off, uint32_t cnt,
-                             uint32_t base) {
+__global__ void k_gen_append(GenGrid g, const float4* cand, const uint32_t* keep, const uint32_t* off, uint32_t cnt) {
+    const uint32_t base = g.st->base;
+    if (blockIdx.x == 0 && threadIdx.x < kGenRounds) g.st->open[threadIdx.x] = 0u;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += gridDim.x * blockDim.x) {
         if (!keep[j]) continue;
         const uint32_t pid = base + off[j];
@@ -143,7 +157,9 @@ __global__ void k_gen_append(GenGrid g, const float4* cand, const uint32_t* keep
     }
 }
 
-__global__ void k_gen_resolve(GenGrid g, uint32_t base, uint32_t count, uint32_t* undecided) {
+__global__ void k_gen_resolve(GenGrid g, const uint32_t* off, uint32_t cnt, int round) {
+    if (round > 0 && g.st->open[round - 1] == 0u) return;
+    const uint32_t base = g.st->base, count = off[cnt];
     volatile uint32_t* state = g.state;
     uint32_t open = 0;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
@@ -164,32 +180,43 @@ __global__ void k_gen_resolve(GenGrid g, uint32_t base, uint32_t count, uint32_t
         else ++open;
     }
     for (int o = 16; o >= 1; o >>= 1) open += __shfl_xor_sync(0xffffffffu, open, o);
-    if ((threadIdx.x & 31) == 0 && open) atomicAdd(undecided, open);
+    if ((threadIdx.x & 31) == 0 && open) atomicAdd(&g.st->open[round], open);
 }
 
-__global__ void k_gen_accept_flags(GenGrid g, uint32_t base, uint32_t count, uint32_t* flags) {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k <= count; k += gridDim.x * blockDim.x)
+// Whether the batch's points are all decided: a round left none open.
+__device__ __forceinline__ bool gen_decided(const GenGrid& g) {
+    for (int r = 0; r < kGenRounds; ++r)
+        if (g.st->open[r] == 0u) return true;
+    return false;
+}
+
+__global__ void k_gen_accept_flags(GenGrid g, const uint32_t* off, uint32_t cnt, uint32_t* flags) {
+    if (!gen_decided(g)) return;
+    const uint32_t base = g.st->base, count = off[cnt];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k <= cnt; k += gridDim.x * blockDim.x)
         flags[k] = k < count && g.state[base + k] == 1u ? 1u : 0u;
 }
 
-__global__ void k_gen_emit(GenGrid g, uint32_t base, uint32_t count, const uint32_t* rank, uint32_t quota,
+__global__ void k_gen_emit(GenGrid g, const uint32_t* off, uint32_t cnt, const uint32_t* rank, uint32_t target,
                            float4* out) {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x)
-        if (g.state[base + k] == 1u && rank[k] < quota) out[rank[k]] = g.pts[base + k];
-}
-
-__global__ void k_gen_retire(GenGrid g, uint32_t base, uint32_t count) {
+    if (!gen_decided(g)) return;
+    const uint32_t base = g.st->base, count = off[cnt], placed = g.st->placed;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
         const uint32_t pid = base + k;
-        const size_t cell = gen_cell_index(g, g.pts[pid]);
+        const float4 p = g.pts[pid];
+        const size_t cell = gen_cell_index(g, p);
         g.head[cell] = 0u;
-        if (g.state[pid] == 1u) g.next_acc[pid] = atomicExch(&g.head_acc[cell], pid + 1u);
+        if (g.state[pid] != 1u) continue;
+        if (rank[k] < target - placed) out[placed + rank[k]] = p;
+        g.next_acc[pid] = atomicExch(&g.head_acc[cell], pid + 1u);
     }
 }
 
-int launch_gen_retire(cudaStream_t st, const GenGrid& g, uint32_t base, uint32_t count) {
-    k_gen_retire<<<grid_for(count, 256), 256, 0, st>>>(g, base, count);
-    return 1;
+__global__ void k_gen_advance(GenGrid g, const uint32_t* off, uint32_t cnt, const uint32_t* rank, uint32_t target) {
+    if (!gen_decided(g)) return;
+    const uint32_t left = target - g.st->placed, n = rank[cnt];
+    g.st->placed += n < left ? n : left;
+    g.st->base += off[cnt];
 }
 
 int launch_gen_filter(cudaStream_t st, const GenGrid& g, const float4* cand, uint32_t cnt, uint32_t* keep) {
@@ -197,21 +224,26 @@ int launch_gen_filter(cudaStream_t st, const GenGrid& g, const float4* cand, uin
     return 1;
 }
 int launch_gen_append(cudaStream_t st, const GenGrid& g, const float4* cand, const uint32_t* keep,
-                      const uint32_t* off, uint32_t cnt, uint32_t base) {
-    k_gen_append<<<grid_for(cnt, 256), 256, 0, st>>>(g, cand, keep, off, cnt, base);
+                      const uint32_t* off, uint32_t cnt) {
+    k_gen_append<<<grid_for(cnt, 256), 256, 0, st>>>(g, cand, keep, off, cnt);
     return 1;
 }
-int launch_gen_resolve(cudaStream_t st, const GenGrid& g, uint32_t base, uint32_t count, uint32_t* undecided) {
-    k_gen_resolve<<<grid_for(count, 256), 256, 0, st>>>(g, base, count, undecided);
+int launch_gen_resolve(cudaStream_t st, const GenGrid& g, const uint32_t* off, uint32_t cnt, int round) {
+    k_gen_resolve<<<grid_for(cnt, 256), 256, 0, st>>>(g, off, cnt, round);
     return 1;
 }
-int launch_gen_accept_flags(cudaStream_t st, const GenGrid& g, uint32_t base, uint32_t count, uint32_t* flags) {
-    k_gen_accept_flags<<<grid_for((unsigned long long)count + 1, 256), 256, 0, st>>>(g, base, count, flags);
+int launch_gen_accept_flags(cudaStream_t st, const GenGrid& g, const uint32_t* off, uint32_t cnt, uint32_t* flags) {
+    k_gen_accept_flags<<<grid_for((unsigned long long)cnt + 1, 256), 256, 0, st>>>(g, off, cnt, flags);
     return 1;
 }
-int launch_gen_emit(cudaStream_t st, const GenGrid& g, uint32_t base, uint32_t count, const uint32_t* rank,
-                    uint32_t quota, float4* out) {
-    k_gen_emit<<<grid_for(count, 256), 256, 0, st>>>(g, base, count, rank, quota, out);
+int launch_gen_emit(cudaStream_t st, const GenGrid& g, const uint32_t* off, uint32_t cnt, const uint32_t* rank,
+                    uint32_t target, float4* out) {
+    k_gen_emit<<<grid_for(cnt, 256), 256, 0, st>>>(g, off, cnt, rank, target, out);
+    return 1;
+}
+int launch_gen_advance(cudaStream_t st, const GenGrid& g, const uint32_t* off, uint32_t cnt, const uint32_t* rank,
+                       uint32_t target) {
+    k_gen_advance<<<1, 1, 0, st>>>(g, off, cnt, rank, target);
     return 1;
 }
 

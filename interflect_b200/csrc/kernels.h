@@ -66,6 +66,7 @@ void launch_gen_finalize(cudaStream_t st, BlobRef blob, const float4* pts, uint3
 
 // Poisson-disc thinning of the projected seeds (surfel.rs:206-227) on the
 // GPU, in batches of consecutive seeds; see k_surfels.cu.
+struct GenState;
 struct GenGrid {
     float lo[3];
     float inv_cell;
@@ -79,25 +80,35 @@ struct GenGrid {
     uint32_t* state;      // per point: 0 undecided, 1 accepted, 2 rejected
     uint32_t cap;         // capacity of pts / next / state
     uint32_t* err;        // device status word (bounded list walks)
+    GenState* st;
+};
+// Progress of the thinning, on the device: points kept and surfels placed by
+// the batches so far, and the points still open after each round of this one.
+static constexpr int kGenRounds = 4;
+struct GenState {
+    uint32_t base, placed;
+    uint32_t open[kGenRounds];
 };
 static constexpr uint32_t kStatusGenWalk = 1u << 5;
 // keep[j] = seed j of the batch projected onto the surface and no accepted
 // point of an earlier batch lies within d_min of it.
 int launch_gen_filter(cudaStream_t st, const GenGrid& g, const float4* cand, uint32_t cnt, uint32_t* keep);
-// Appends the kept seeds at base + off[j] (undecided) and links them into
-// their cells.
+// Appends the kept seeds at st->base + off[j] (undecided) and links them into
+// their cells; clears the batch's round counters.
 int launch_gen_append(cudaStream_t st, const GenGrid& g, const float4* cand, const uint32_t* keep,
-                      const uint32_t* off, uint32_t cnt, uint32_t base);
-// One round of deciding the batch's points [base, base + count) in seed
-// order; *undecided counts those still open.
-int launch_gen_resolve(cudaStream_t st, const GenGrid& g, uint32_t base, uint32_t count, uint32_t* undecided);
-int launch_gen_accept_flags(cudaStream_t st, const GenGrid& g, uint32_t base, uint32_t count, uint32_t* flags);
-// out[before + rank] = accepted point, for ranks below quota.
-// After a batch: its accepted points join the accepted lists, and its cells
-// of the batch lists are emptied for the next batch.
-int launch_gen_retire(cudaStream_t st, const GenGrid& g, uint32_t base, uint32_t count);
-int launch_gen_emit(cudaStream_t st, const GenGrid& g, uint32_t base, uint32_t count, const uint32_t* rank,
-                    uint32_t quota, float4* out);
+                      const uint32_t* off, uint32_t cnt);
+// Round `round` of deciding the batch's off[cnt] points in seed order (a no-op
+// once an earlier round left none open); st->open[round] counts those open.
+int launch_gen_resolve(cudaStream_t st, const GenGrid& g, const uint32_t* off, uint32_t cnt, int round);
+// The batch's end, each a no-op while points are open: flags of the accepted
+// points (cnt + 1 entries, zero past the batch's), then, with their ranks,
+// the accepted points out to out[st->placed + rank] below target, and onto the
+// accepted lists; the batch's cells are emptied, and st moves on.
+int launch_gen_accept_flags(cudaStream_t st, const GenGrid& g, const uint32_t* off, uint32_t cnt, uint32_t* flags);
+int launch_gen_emit(cudaStream_t st, const GenGrid& g, const uint32_t* off, uint32_t cnt, const uint32_t* rank,
+                    uint32_t target, float4* out);
+int launch_gen_advance(cudaStream_t st, const GenGrid& g, const uint32_t* off, uint32_t cnt, const uint32_t* rank,
+                       uint32_t target);
 
 // ---- clusters (formfactor.rs:91-147) ----
 void launch_cluster_keys(cudaStream_t st, const float4* p, const float4* n, uint32_t count, SceneConsts sc,
