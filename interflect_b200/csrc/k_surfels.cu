@@ -6,13 +6,18 @@ namespace ifx {
 // surfel.rs:190-211: Halton seed i (bases 2, 3, 5) across the scene bounds,
 // Newton projection onto the zero level set (at most 10 steps), then the
 // on-surface and in-bounds tests. Writes the projected point with w = 1 if
-// the seed survives, w = 0 otherwise. The Poisson-disc thinning that follows
-// (below) keeps the reference's seed-order semantics.
+// the seed survives, w = 0 otherwise. (The reference tests the distance of an
+// accepted point once more, which at the same point is the same.) The
+// Poisson-disc thinning that follows (below) keeps the reference's seed-order
+// semantics.
 //
 // Consecutive Halton points lie far apart, points whose indices differ by a
 // multiple of 32 * 9 * 25 in the same 1/32 x 1/9 x 1/25 box of the bounds:
 // lanes take the chunk's seeds in that stride, so that a warp's points meet
-// the same objects and take similar numbers of steps.
+// the same objects. Each lane is a state machine over its seeds with one
+// query site for the distance and the four normal taps, all lanes querying
+// together: with the taps unrolled the code outgrew the instruction cache
+// (23 of 28 stall cycles per instruction; 627 us a chunk of 2^18 seeds).
 static constexpr uint32_t kGenStride = 32u * 9u * 25u;
 __global__ void __launch_bounds__(128) k_gen_project(BlobRef blob, SceneConsts sc, uint32_t seed0,
                                                       uint32_t count, float eps, float4* out, uint32_t* status) {
@@ -21,25 +26,50 @@ __global__ void __launch_bounds__(128) k_gen_project(BlobRef blob, SceneConsts s
     const V lo{sc.lo[0], sc.lo[1], sc.lo[2]}, hi{sc.hi[0], sc.hi[1], sc.hi[2]};
     const float diag = sc.diag;
     const uint32_t per = (count + kGenStride - 1u) / kGenStride, total = per * kGenStride;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
-        const uint32_t j = (k % per) * kGenStride + k / per;
-        if (j >= count) continue;
-        uint32_t i = seed0 + j;
-        V s{radical_inverse(i + 1, 2), radical_inverse(i + 1, 3), radical_inverse(i + 1, 5)};
-        V p = lo + (hi - lo) * s;
-        bool ok = false;
-        for (int it = 0; it < 10; ++it) {
-            float d = scene_dist(sv, p, nc);
-            if (fabsf(d) < eps) {
-                ok = true;
-                break;
-            }
-            if (!isfinite(d) || fabsf(d) > diag) break;
-            p = p - scene_normal(sv, p, nc) * d;
+    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x, j = 0;
+    bool live = false;
+    int it = 0, tap = -1;
+    V p{}, n{};
+    float d = 0.0f;
+    while (true) {
+        while (!live && k < total) {
+            j = (k % per) * kGenStride + k / per;
+            k += gridDim.x * blockDim.x;
+            if (j >= count) continue;
+            const uint32_t i = seed0 + j;
+            p = lo + (hi - lo) * V{radical_inverse(i + 1, 2), radical_inverse(i + 1, 3), radical_inverse(i + 1, 5)};
+            live = true;
+            it = 0;
+            tap = -1;
         }
-        if (ok && fabsf(scene_dist(sv, p, nc)) >= eps) ok = false;
-        if (ok && (p.x < lo.x || p.y < lo.y || p.z < lo.z || p.x > hi.x || p.y > hi.y || p.z > hi.z)) ok = false;
-        out[j] = make_float4(p.x, p.y, p.z, ok ? 1.0f : 0.0f);
+        if (!__any_sync(kFull, live)) break;
+        // scene.rs:218-236 tap offsets, in the order scene_normal() sums them.
+        const V o{(tap == 0 || tap == 3) ? 1.0f : -1.0f, (tap >= 2) ? 1.0f : -1.0f,
+                  (tap == 1 || tap == 3) ? 1.0f : -1.0f};
+        const float v = dist_warp<false>(sv, tap < 0 ? p : p + o * 5e-4f, live, nc).d;
+        if (!live) continue;
+        bool ok = false, done = false;
+        if (tap < 0) {
+            d = v;
+            ok = fabsf(d) < eps;
+            done = ok || !isfinite(d) || fabsf(d) > diag;
+            n = V{0.0f, 0.0f, 0.0f};
+            tap = 0;
+        } else {
+            n = n + o * v;
+            if (++tap == 4) {
+                const float l = len(n);
+                n = l > 1e-12f ? n / l : V{0.0f, 1.0f, 0.0f};
+                p = p - n * d;
+                tap = -1;
+                done = ++it == 10;
+            }
+        }
+        if (done) {
+            if (p.x < lo.x || p.y < lo.y || p.z < lo.z || p.x > hi.x || p.y > hi.y || p.z > hi.z) ok = false;
+            out[j] = make_float4(p.x, p.y, p.z, ok ? 1.0f : 0.0f);
+            live = false;
+        }
     }
 }
 
@@ -52,7 +82,7 @@ __global__ void __launch_bounds__(128) k_gen_finalize(BlobRef blob, const float4
         V p = mk4(pts[i]);
         DistHit h = dist_mat(sv, p, nc);
         const DMaterial& m = sv.mat(h.mat);
-        V nn = scene_normal(sv, p, nc);
+        V nn = scene_normal_rolled(sv, p, nc);
         s.p[i] = f4(p, area);
         s.n[i] = f4(nn, 0.0f);
         s.albedo[i] = make_float4(m.kd[0], m.kd[1], m.kd[2], 0.0f);
@@ -249,7 +279,7 @@ int launch_gen_advance(cudaStream_t st, const GenGrid& g, const uint32_t* off, u
 
 void launch_gen_project(cudaStream_t st, BlobRef blob, SceneConsts sc, uint32_t seed0, uint32_t count, float eps,
                         float4* out, uint32_t* status) {
-    k_gen_project<<<grid_for(count, 128), 128, blob_smem(blob, 128), st>>>(blob, sc, seed0, count, eps, out, status);
+    k_gen_project<<<grid_for(count, 128, 9), 128, blob_smem(blob, 128), st>>>(blob, sc, seed0, count, eps, out, status);
 }
 void launch_gen_finalize(cudaStream_t st, BlobRef blob, const float4* pts, uint32_t n, float area, SurfelArrays s,
                          uint32_t* status) {
