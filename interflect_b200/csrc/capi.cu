@@ -820,8 +820,12 @@ extern "C" int ifx_surfels_generate(ifx_ctx* ctx, uint64_t target, uint64_t* pla
 
     // Seeds are projected and thinned on the GPU in batches of consecutive
     // indices (k_surfels.cu); the host only reads each batch's counts.
-    const uint32_t kChunk = 1u << 18;       // seeds projected at a time
+    // Seeds projected at a time: as many as before them, within these bounds,
+    // so that a scene that reaches its target early projects at most twice
+    // what it needs and a long run has few tails of half-empty warps.
+    const uint32_t kMinChunk = 1u << 18, kMaxChunk = 1u << 20;
     const uint32_t kFirstBatch = 1u << 12;  // seeds thinned in the first batch
+    const uint32_t kChunk = seeds < kMaxChunk ? seeds : kMaxChunk;
     const size_t ncells = (size_t)dim[0] * (size_t)dim[1] * (size_t)dim[2];
     ENSURE(ctx->gen_cand, (size_t)kChunk * sizeof(float4));
     ENSURE(ctx->gen_keep, ((size_t)kChunk + 1) * 4);
@@ -858,8 +862,8 @@ extern "C" int ifx_surfels_generate(ifx_ctx* ctx, uint64_t target, uint64_t* pla
     uint32_t* off = (uint32_t*)ctx->gen_off.p;
     uint32_t* rank = (uint32_t*)ctx->gen_rank.p;
     uint32_t placed_n = 0;
-    for (uint32_t s0 = 0; s0 < seeds && placed_n < target; s0 += kChunk) {
-        const uint32_t chunk = seeds - s0 < kChunk ? seeds - s0 : kChunk;
+    for (uint32_t s0 = 0, chunk = 0; s0 < seeds && placed_n < target; s0 += chunk) {
+        chunk = std::min(seeds - s0, std::min(kMaxChunk, std::max(kMinChunk, s0)));
         launch_gen_project(ctx->st, ctx->blobref, ctx->sc, s0, chunk, eps, (float4*)ctx->gen_cand.p,
                            (uint32_t*)ctx->status.p);
         ctx->launches++;
