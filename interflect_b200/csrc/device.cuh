@@ -340,12 +340,19 @@ __device__ __forceinline__ float prim_dist(const DPrim& pr, V p, C& cnt) {
 // counting kernels evaluate everything, as the reference does.
 template <class C>
 __device__ __forceinline__ float obj_dist(const SceneView& sv, const DObject& o, V p, C& cnt, float best = kMaxF) {
-    float d = prim_dist(sv.prim(o.prim), p, cnt);
-    if constexpr (sizeof(C) == 1) {
-        if (o.nsub > 0 && d >= best + (o.smooth > 0.0f ? 1e-5f * (1.0f + fabsf(best) + o.smooth) : 0.0f)) return d;
-    }
-    for (int s = 1; s <= o.nsub; ++s) {
-        float sd = prim_dist(sv.prim(o.prim + s), p, cnt);
+    float d = 0.0f;
+    // The base is the loop's first turn, so that prim_dist has one site.
+#pragma unroll 1
+    for (int s = 0; s <= o.nsub; ++s) {
+        const float sd = prim_dist(sv.prim(o.prim + s), p, cnt);
+        if (s == 0) {
+            d = sd;
+            if constexpr (sizeof(C) == 1) {
+                if (o.nsub > 0 && d >= best + (o.smooth > 0.0f ? 1e-5f * (1.0f + fabsf(best) + o.smooth) : 0.0f))
+                    return d;
+            }
+            continue;
+        }
         cnt.add(o.smooth > 0.0f ? CN_SMOOTH : CN_HARD);
         if (o.smooth > 0.0f) {
             float k = o.smooth;
@@ -373,104 +380,169 @@ struct DistHit {
     uint32_t mat;
 };
 
-// scene.rs:191-208 with bvh.rs:100-150 (query) or bvh.rs:155-163 (linear):
-// the reference's own traversal.
+// ------------------------------------------------- the reference query ----
+// scene.rs:191-208 with bvh.rs:100-150 (query) or bvh.rs:155-163 (linear) as a
+// sequence of object ranges: the planes, then the leaves the pruned near-first
+// traversal reaches (or all objects in parse order). Every range is evaluated
+// at one place in the code, which the kernels' instruction cache needs.
+//
+// A node's box distance is a pure function of p and the node, so the value
+// computed when it was pushed (bvh.rs:135-136) is the one the reference
+// recomputes when it pops it (:116); it is kept on the stack and counted as
+// the reference's test. The stack holds squared box distances (see sq_ge /
+// sq_lt). Trees of a root and two leaves keep their two pending leaves in
+// registers instead: the same box tests, pruning decisions, visit order and
+// counts (kernels for such scenes, C::kTree3, compile only that form).
+struct RefQuery {
+    int k, end;         // pending range of stored objects; empty when k == end
+    int leaf;           // the pending leaf, or a range every lane shares: kRefPlanes, kRefLinear
+    int next, last;     // three-node trees: leaves still to pop, in order
+    float dnext, dlast;
+    int sp;
+    bool first;
+};
+enum : int { kRefPlanes = -1, kRefLinear = -2, kRefNone = -3 };
+
 template <class C>
-__device__ __forceinline__ DistHit dist_mat_ref(const SceneView& sv, V p, C& cnt) {
-    DistHit best{kMaxF, 0u};
-    for (int i = 0; i < sv.n_planes; ++i) {
-        const DObject o = sv.obj(i);
-        float d = obj_dist(sv, o, p, cnt, best.d);
-        if (d < best.d) best = DistHit{d, o.mat};
+__device__ __forceinline__ bool ref_three(const SceneView& sv) {
+    if constexpr (C::kTree3) return true;
+    return sv.use_bvh && sv.n_nodes == 3;
+}
+
+__device__ __forceinline__ RefQuery ref_begin(const SceneView& sv, bool active) {
+    return RefQuery{0, active ? sv.n_planes : 0, active ? kRefPlanes : kRefNone, -1, -1, 0.0f, 0.0f, 0, true};
+}
+
+// After the planes: the root (not counted when it is popped, as its distance
+// is computed here).
+template <class C>
+__device__ __forceinline__ void ref_root(const SceneView& sv, RefQuery& q, V p, const DistHit& best, C& cnt) {
+    if (ref_three<C>(sv)) {
+        const float d0 = aabb_dist2(p, sv.node(0), cnt);
+        if (sq_ge(d0, best.d)) return;
+        const int l = 1, r = sv.node(0).link;
+        const float dl = aabb_dist2(p, sv.node(l), cnt), dr = aabb_dist2(p, sv.node(r), cnt);
+        const bool left = sq_lt(dl, dr);
+        q.next = left ? l : r, q.dnext = left ? dl : dr;
+        q.last = left ? r : l, q.dlast = left ? dr : dl;
+        return;
     }
-    if constexpr (C::kTree3) {
-        // bvh.rs:100-150 on a root and two leaves: the same tests, prunes and
-        // visit order as the stack traversal below.
-        if (sq_ge(aabb_dist2(p, sv.node(0), cnt), best.d)) return best;
-        const int r = sv.node(0).link;
-        const float dl = aabb_dist2(p, sv.node(1), cnt), dr = aabb_dist2(p, sv.node(r), cnt);
-        const bool lfirst = sq_lt(dl, dr);
-#pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass) {
-            const bool left = (pass == 0) == lfirst;
-            if (sq_ge(left ? dl : dr, best.d)) continue;
-            const DNode& nd = sv.node(left ? 1 : r);
-            for (int k = nd.link; k < nd.link + nd.count; ++k) {
-                const DObject o = sv.obj(k);
-                const float d = obj_dist(sv, o, p, cnt, best.d);
-                if (d < best.d) {
-                    best.d = d;
-                    best.mat = o.mat;
-                }
-            }
+    if (!sv.use_bvh) {
+        q.k = 0, q.end = sv.n_objects, q.leaf = kRefLinear;
+        return;
+    }
+    if (sv.n_nodes == 0) return;
+    sv.stk[0] = 0;
+    sv.stkd[0] = aabb_dist2(p, sv.node(0), cnt);
+    q.sp = 1;
+}
+
+// Pops nodes until one is a leaf to evaluate (the new pending range) or none
+// is left.
+template <class C>
+__device__ __forceinline__ void ref_advance(const SceneView& sv, RefQuery& q, V p, const DistHit& best, C& cnt) {
+    if (q.leaf == kRefPlanes) {
+        q.leaf = kRefNone;
+        ref_root(sv, q, p, best, cnt);
+        if (q.leaf == kRefLinear) return;
+    }
+    q.leaf = kRefNone;
+    if (ref_three<C>(sv)) {
+        while (q.next >= 0 && q.leaf == kRefNone) {
+            cnt.add(CN_NODE);
+            if (!sq_ge(q.dnext, best.d)) q.leaf = q.next;
+            q.next = q.last, q.dnext = q.dlast, q.last = -1;
         }
-        return best;
-    }
-    if (sv.use_bvh) {
-        if (sv.n_nodes == 0) return best;
-        // bvh.rs:100-150. A node's box distance is a pure function of p and
-        // the node, so the value computed when it was pushed (bvh.rs:135-136)
-        // is the one the reference recomputes when it pops it (:116); it is
-        // kept on the stack and counted as the reference's test.
-        // The stack holds squared box distances (see sq_ge / sq_lt).
+    } else if constexpr (!C::kTree3) {
         uint32_t* const stack = sv.stk;
         float* const stackd = sv.stkd;
         const int stride = sv.stk_stride;
-        int sp = 0;
-        stack[0] = 0;
-        stackd[0] = aabb_dist2(p, sv.node(0), cnt);
-        sp = 1;
-        bool first = true;
-        while (sp > 0) {
-            --sp;
-            const int ni = (int)stack[sp * stride];
+        while (q.sp > 0) {
+            --q.sp;
+            const int ni = (int)stack[q.sp * stride];
             const DNode nd = sv.node(ni);
-            if (!first) cnt.add(CN_NODE);
-            first = false;
-            if (sq_ge(stackd[sp * stride], best.d)) continue;
+            if (!q.first) cnt.add(CN_NODE);
+            q.first = false;
+            if (sq_ge(stackd[q.sp * stride], best.d)) continue;
             if (nd.count > 0) {
-                for (int k = nd.link; k < nd.link + nd.count; ++k) {
-                    const DObject o = sv.obj(k);
-                    float d = obj_dist(sv, o, p, cnt, best.d);
-                    if (d < best.d) {
-                        best.d = d;
-                        best.mat = o.mat;
-                    }
-                }
-            } else {
-                const int l = ni + 1, r = nd.link;
-                float dl = aabb_dist2(p, sv.node(l), cnt);
-                float dr = aabb_dist2(p, sv.node(r), cnt);
-                // Near-first DFS holds at most depth + 1 entries; the host
-                // sizes the stack to depth + 2 (and rejects trees deeper
-                // than the reference's 64-entry stack). The guard keeps an
-                // unexpected overflow inside the stack: traversal stops.
-                if (sp + 2 > sv.stk_depth) break;
-                if (sq_lt(dl, dr)) {
-                    stack[sp * stride] = (uint32_t)r;
-                    stackd[sp * stride] = dr;
-                    stack[(sp + 1) * stride] = (uint32_t)l;
-                    stackd[(sp + 1) * stride] = dl;
-                } else {
-                    stack[sp * stride] = (uint32_t)l;
-                    stackd[sp * stride] = dl;
-                    stack[(sp + 1) * stride] = (uint32_t)r;
-                    stackd[(sp + 1) * stride] = dr;
-                }
-                sp += 2;
+                q.leaf = ni;
+                break;
             }
-        }
-    } else {
-        for (int k = 0; k < sv.n_objects; ++k) {
-            const DObject o = sv.obj(sv.lin(k));
-            float d = obj_dist(sv, o, p, cnt, best.d);
-            if (d < best.d) {
-                best.d = d;
-                best.mat = o.mat;
+            const int l = ni + 1, r = nd.link;
+            const float dl = aabb_dist2(p, sv.node(l), cnt), dr = aabb_dist2(p, sv.node(r), cnt);
+            // Near-first DFS holds at most depth + 1 entries; the host sizes
+            // the stack to depth + 2 (and rejects trees deeper than the
+            // reference's 64-entry stack). The guard keeps an unexpected
+            // overflow inside the stack: traversal stops.
+            if (q.sp + 2 > sv.stk_depth) {
+                q.sp = 0;
+                break;
             }
+            const bool left = sq_lt(dl, dr);
+            stack[q.sp * stride] = (uint32_t)(left ? r : l);
+            stackd[q.sp * stride] = left ? dr : dl;
+            stack[(q.sp + 1) * stride] = (uint32_t)(left ? l : r);
+            stackd[(q.sp + 1) * stride] = left ? dl : dr;
+            q.sp += 2;
         }
     }
-    return best;
+    if (q.leaf >= 0) {
+        const DNode& nd = sv.node(q.leaf);
+        q.k = nd.link;
+        q.end = nd.link + nd.count;
+    }
+}
+
+// One object of the pending range.
+template <class C>
+__device__ __forceinline__ void ref_eval(const SceneView& sv, RefQuery& q, V p, DistHit& best, C& cnt) {
+    const DObject o = sv.obj(q.leaf == kRefLinear ? (int)sv.lin(q.k) : q.k);
+    ++q.k;
+    const float d = obj_dist(sv, o, p, cnt, best.d);
+    if (d < best.d) {
+        best.d = d;
+        best.mat = o.mat;
+    }
+}
+
+template <class C>
+__device__ __forceinline__ DistHit dist_mat_ref(const SceneView& sv, V p, C& cnt) {
+    DistHit best{kMaxF, 0u};
+    RefQuery q = ref_begin(sv, true);
+    while (true) {
+        while (q.k < q.end) ref_eval(sv, q, p, best, cnt);
+        if (q.leaf == kRefNone || q.leaf == kRefLinear) return best;
+        ref_advance(sv, q, p, best, cnt);
+    }
+}
+
+// dist_mat_ref for a whole warp (all 32 lanes call it; lanes with !active only
+// take part in the votes). Each active lane runs its own near-first traversal
+// with the reference's pruning, but leaves are evaluated in warp-synchronous
+// rounds: once every lane has either a pending range or finished, either the
+// lanes sharing the first waiting lane's leaf evaluate it together (the
+// primitive code runs converged) or, in trees of more than four leaves when
+// fewer than 7/8 of the waiting lanes share that leaf, every waiting lane
+// evaluates its own leaf in the same round (lanes at different leaves then
+// diverge only by primitive kind, instead of waiting a round per leaf). A
+// lane's sequence of node tests, object evaluations and best-distance updates
+// is exactly the one dist_mat_ref() makes.
+template <class C>
+__device__ __forceinline__ DistHit dist_mat_ref_warp(const SceneView& sv, V p, bool active, C& cnt) {
+    DistHit best{kMaxF, 0u};
+    RefQuery q = ref_begin(sv, active);
+    while (true) {
+        while (q.k >= q.end && q.leaf != kRefNone)
+            if (q.leaf == kRefLinear) q.leaf = kRefNone;
+            else ref_advance(sv, q, p, best, cnt);
+        const unsigned waiting = __ballot_sync(0xffffffffu, q.leaf != kRefNone);
+        if (!waiting) return best;
+        const int leaf = __shfl_sync(0xffffffffu, q.leaf, __ffs(waiting) - 1);
+        const bool shared = C::kTree3 || sv.n_nodes <= 7 ||
+                            8 * __popc(__ballot_sync(0xffffffffu, q.leaf == leaf)) >= 7 * __popc(waiting);
+        if (q.leaf != kRefNone && (q.leaf == leaf || !shared))
+            while (q.k < q.end) ref_eval(sv, q, p, best, cnt);
+    }
 }
 
 // obj_dist of stored object o from its packed form: the operations of
@@ -567,160 +639,6 @@ __device__ __forceinline__ DistHit dist_mat(const SceneView& sv, V p, C& cnt) {
 template <class C>
 __device__ __forceinline__ float scene_dist(const SceneView& sv, V p, C& cnt) {
     return dist_mat(sv, p, cnt).d;
-}
-
-// Evaluates leaf `leaf`'s objects into `best` (bvh.rs:118-126).
-template <class C>
-__device__ __forceinline__ void leaf_eval(const SceneView& sv, int leaf, V p, DistHit& best, C& cnt) {
-    const DNode nd = sv.node(leaf);
-    for (int k = nd.link; k < nd.link + nd.count; ++k) {
-        const DObject o = sv.obj(k);
-        const float d = obj_dist(sv, o, p, cnt, best.d);
-        if (d < best.d) {
-            best.d = d;
-            best.mat = o.mat;
-        }
-    }
-}
-
-// dist_mat_warp's traversal for a three-node tree (a root and two leaves):
-// the same box tests, pruning decisions, visit order and counts, with the two
-// pending leaves held in registers instead of the shared-memory stack. The
-// root is popped first (not counted, as in dist_mat), then the nearer leaf,
-// then the other; leaves are evaluated in warp rounds of one leaf each.
-template <class C>
-__device__ __forceinline__ DistHit dist_mat_warp3(const SceneView& sv, V p, bool active, DistHit best, C& cnt) {
-    int next = -1, last = -1;  // leaves still to pop, in order
-    float dnext = 0.0f, dlast = 0.0f;
-    if (active) {
-        const float d0 = aabb_dist2(p, sv.node(0), cnt);
-        if (!sq_ge(d0, best.d)) {
-            const int l = 1, r = sv.node(0).link;
-            const float dl = aabb_dist2(p, sv.node(l), cnt);
-            const float dr = aabb_dist2(p, sv.node(r), cnt);
-            if (sq_lt(dl, dr)) {
-                next = l, dnext = dl, last = r, dlast = dr;
-            } else {
-                next = r, dnext = dr, last = l, dlast = dl;
-            }
-        }
-    }
-    int pending = -1;
-    while (true) {
-        while (pending < 0 && next >= 0) {
-            cnt.add(CN_NODE);
-            if (!sq_ge(dnext, best.d)) pending = next;
-            next = last, dnext = dlast, last = -1;
-        }
-        const unsigned waiting = __ballot_sync(0xffffffffu, pending >= 0);
-        if (!waiting) break;
-        const int leaf = __shfl_sync(0xffffffffu, pending, __ffs(waiting) - 1);
-        if (pending == leaf) {
-            leaf_eval(sv, leaf, p, best, cnt);
-            pending = -1;
-        }
-    }
-    return best;
-}
-
-// dist_mat_ref for a whole warp (all 32 lanes call it; lanes with !active only
-// take part in the votes). Each active lane runs its own near-first BVH
-// traversal with the reference's pruning, but leaves are evaluated in
-// warp-synchronous rounds: a lane advances through interior nodes until it
-// reaches a leaf that passes the AABB test; then, once every lane has either
-// found one or finished, either the lanes sharing the first waiting lane's
-// leaf evaluate it together (the primitive code runs converged) or, in trees
-// of more than four leaves when fewer than 7/8 of the waiting lanes share
-// that leaf, every waiting lane evaluates its own leaf in the same round
-// (lanes at different leaves then diverge only by primitive kind, instead of
-// waiting a round per leaf). A lane's sequence of node
-// tests, object evaluations and best-distance updates is exactly the one
-// dist_mat() makes.
-template <class C>
-__device__ __forceinline__ DistHit dist_mat_ref_warp(const SceneView& sv, V p, bool active, C& cnt) {
-    DistHit best{kMaxF, 0u};
-    if (active) {
-        for (int i = 0; i < sv.n_planes; ++i) {
-            const DObject o = sv.obj(i);
-            float d = obj_dist(sv, o, p, cnt, best.d);
-            if (d < best.d) best = DistHit{d, o.mat};
-        }
-    }
-    if constexpr (C::kTree3) return dist_mat_warp3(sv, p, active, best, cnt);
-    if (!sv.use_bvh) {
-        if (active) {
-            for (int k = 0; k < sv.n_objects; ++k) {
-                const DObject o = sv.obj(sv.lin(k));
-                float d = obj_dist(sv, o, p, cnt, best.d);
-                if (d < best.d) {
-                    best.d = d;
-                    best.mat = o.mat;
-                }
-            }
-        }
-        return best;
-    }
-    if (sv.n_nodes == 0) return best;
-    if (sv.n_nodes == 3) return dist_mat_warp3(sv, p, active, best, cnt);
-    uint32_t* const stack = sv.stk;
-    float* const stackd = sv.stkd;
-    const int stride = sv.stk_stride;
-    int sp = 0;
-    bool first = true;
-    if (active) {
-        stack[0] = 0;
-        stackd[0] = aabb_dist2(p, sv.node(0), cnt);
-        sp = 1;
-    }
-    int pending = -1;
-    while (true) {
-        while (pending < 0 && sp > 0) {
-            --sp;
-            const int ni = (int)stack[sp * stride];
-            const DNode nd = sv.node(ni);
-            // The box distance stored at push time (see dist_mat).
-            if (!first) cnt.add(CN_NODE);
-            first = false;
-            if (sq_ge(stackd[sp * stride], best.d)) continue;
-            if (nd.count > 0) {
-                pending = ni;
-                break;
-            }
-            const int l = ni + 1, r = nd.link;
-            float dl = aabb_dist2(p, sv.node(l), cnt);
-            float dr = aabb_dist2(p, sv.node(r), cnt);
-            if (sp + 2 > sv.stk_depth) {
-                sp = 0;
-                break;
-            }
-            if (sq_lt(dl, dr)) {
-                stack[sp * stride] = (uint32_t)r;
-                stackd[sp * stride] = dr;
-                stack[(sp + 1) * stride] = (uint32_t)l;
-                stackd[(sp + 1) * stride] = dl;
-            } else {
-                stack[sp * stride] = (uint32_t)l;
-                stackd[sp * stride] = dl;
-                stack[(sp + 1) * stride] = (uint32_t)r;
-                stackd[(sp + 1) * stride] = dr;
-            }
-            sp += 2;
-        }
-        const unsigned waiting = __ballot_sync(0xffffffffu, pending >= 0);
-        if (!waiting) break;
-        const int leaf = __shfl_sync(0xffffffffu, pending, __ffs(waiting) - 1);
-        // Trees of at most four leaves: one leaf per round, converged. Larger
-        // trees: the first waiting lane's leaf is evaluated alone when at
-        // least 7/8 of the waiting lanes share it; otherwise every waiting
-        // lane evaluates its own leaf in this round.
-        const bool shared = sv.n_nodes <= 7 || 8 * __popc(__ballot_sync(0xffffffffu, pending == leaf)) >=
-                                                   7 * __popc(waiting);
-        if (pending >= 0 && (pending == leaf || !shared)) {
-            leaf_eval(sv, pending, p, best, cnt);
-            pending = -1;
-        }
-    }
-    return best;
 }
 
 // dist_mat for a whole warp (all 32 lanes call it; lanes with !active get

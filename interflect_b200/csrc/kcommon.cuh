@@ -107,7 +107,12 @@ static inline unsigned grid_for(unsigned long long items, int block, int per_sm_
     return (unsigned)(need < cap ? need : cap);
 }
 
-// Persistent kernels: one wave of CTAs, as many as are co-resident.
+// Persistent kernels: one wave of CTAs, as many as are co-resident. Few items
+// are spread thinly (WarpQueue then leaves lanes of every warp empty) until
+// there are kSpreadCtas per SM: a warp issues at most every fourth cycle or so
+// along a ray's dependent chain, so a scheduler needs about five warps to
+// stay busy, and a warp of fewer rays takes fewer divergent turns per step.
+static constexpr unsigned kSpreadCtas = 5;
 template <class K>
 static inline unsigned persistent_grid(K kernel, int block, size_t smem, unsigned long long items) {
     int per_sm = 0;
@@ -115,6 +120,9 @@ static inline unsigned persistent_grid(K kernel, int block, size_t smem, unsigne
     if (per_sm < 1) per_sm = 1;
     unsigned long long cap = (unsigned long long)sm_count() * (unsigned long long)per_sm;
     unsigned long long need = (items + (unsigned long long)block - 1) / (unsigned long long)block;
+    const unsigned long long thin = (items * 32ull + (unsigned long long)block - 1) / (unsigned long long)block;
+    const unsigned long long spread = (unsigned long long)sm_count() * kSpreadCtas;
+    need = need > spread ? need : (thin < spread ? thin : spread);
     if (need < 1) need = 1;
     return (unsigned)(need < cap ? need : cap);
 }
@@ -127,21 +135,26 @@ static inline unsigned persistent_grid(K kernel, int block, size_t smem, unsigne
 // written to a slot fixed by its index.
 struct WarpQueue {
     uint32_t cur, end;  // warp-uniform private range [cur, end)
-    uint32_t kChunk;    // items taken per atomic: about 1/8 of a fair share per warp, 32..256
+    uint32_t kChunk;    // items taken per atomic: about 1/8 of a fair share per warp, 32..256, or
+                        // the whole share where it is less than a warp
+    uint32_t lanes;     // lanes that take items: all, or a fair share where there are few items
     bool drained;
 
-    __device__ __forceinline__ WarpQueue() : cur(0), end(0), kChunk(32), drained(false) {}
     __device__ __forceinline__ explicit WarpQueue(unsigned long long total) : cur(0), end(0), drained(false) {
         const unsigned long long warps = (unsigned long long)gridDim.x * blockDim.x / 32u;
         unsigned long long c = total / (warps * 8ull + 1ull);
         c = c < 32ull ? 32ull : (c > 256ull ? 256ull : c);
-        kChunk = (uint32_t)(c & ~31ull);
+        const unsigned long long share = (total + warps - 1ull) / warps;
+        // At least one, of an empty queue too: some lane has to find it drained.
+        lanes = share < 1ull ? 1u : (share < 32ull ? (uint32_t)share : 32u);
+        kChunk = lanes < 32u ? lanes : (uint32_t)(c & ~31ull);
     }
 
     // Returns the item for this lane (or ~0u) when it is idle; `idle` says
     // whether this lane needs an item. Must be called by all 32 lanes.
     __device__ __forceinline__ uint32_t refill(bool idle, unsigned long long total, unsigned long long* cursor) {
         const int lane = threadIdx.x & 31;
+        idle = idle && (uint32_t)lane < lanes;
         unsigned need = __ballot_sync(kFull, idle);
         uint32_t item = ~0u;
         if (!need) return item;
