@@ -613,11 +613,7 @@ static int objgrid_build(ifx_ctx* ctx, const std::vector<uint8_t>& blob) {
     if (!ctx->objgrid_on || !bh->use_bvh || bh->n_nodes == 0 || nobj > kOgMaxObjects) return IFX_OK;
     const float* lo = ctx->sc.lo;
     const float* hi = ctx->sc.hi;
-    double ext = 0.0, scale = 0.0;
-    for (int a = 0; a < 3; ++a) {
-        ext = std::max(ext, (double)hi[a] - (double)lo[a]);
-        scale = std::max(scale, std::max(std::fabs((double)lo[a]), std::fabs((double)hi[a])));
-    }
+    double scale = 0.0;
     const DPrim* prims = reinterpret_cast<const DPrim*>(blob.data() + bh->off_prims);
     for (int i = 0; i < bh->n_prims; ++i)
         if (!og_admits(prims[i], scale)) return IFX_OK;
@@ -626,27 +622,24 @@ static int objgrid_build(ifx_ctx* ctx, const std::vector<uint8_t>& blob) {
         if (!std::isfinite(objs[i].smooth)) return IFX_OK;
         scale = std::max(scale, std::fabs((double)objs[i].smooth));
     }
-    scale += (double)ctx->sc.diag;
-    if (!(ext > 0.0) || !std::isfinite(scale)) return IFX_OK;
     const bool masks = nobj <= kOgMaskObjects;
-    const int kCells = masks ? 64 : 96;
-    const double cs = ext / kCells;
+    const double diag = (double)ctx->sc.diag;
     ObjGrid g{};
-    g.delta = (float)(scale / 65536.0);
+    float from[2][3];
+    const double side = og_level(g.fine, lo, hi, masks ? 64 : 96, 1.0, scale, diag, 0, from[0]);
+    const uint32_t fine = g.fine.dim[0] * g.fine.dim[1] * g.fine.dim[2];
+    const double side2 =
+        og_level(g.coarse, lo, hi, kOgCoarseCells, kOgCoarseExtent, scale, diag, fine, from[1]);
+    const size_t ncells = (size_t)fine + (size_t)g.coarse.dim[0] * g.coarse.dim[1] * g.coarse.dim[2];
     // A scene whose coordinates dwarf its extent: the margins would list everything.
-    if ((double)g.delta > 0.25 * cs) return IFX_OK;
-    g.inv = (float)(1.0 / cs);
-    size_t ncells = 1;
-    for (int a = 0; a < 3; ++a) {
-        g.bias[a] = (float)(-(double)lo[a] / cs - 0.5);
-        g.dim[a] = (uint32_t)std::min(kCells, std::max(1, (int)std::ceil(((double)hi[a] - (double)lo[a]) / cs)));
-        ncells *= g.dim[a];
-    }
+    if (!(side > 0.0) || !(g.fine.delta <= 0.25 * side) || !(g.coarse.delta <= 0.25 * side2)) return IFX_OK;
     ENSURE(ctx->og_cells, ncells * (masks ? 4 : 16));
     g.mode = masks ? kOgMask : kOgList;
-    launch_og_build(ctx->st, ctx->blobref, g, lo, (float)cs, masks ? (uint32_t*)ctx->og_cells.p : nullptr,
-                    masks ? nullptr : (uint4*)ctx->og_cells.p, (uint32_t*)ctx->status.p);
-    ctx->launches++;
+    uint32_t* mask = masks ? (uint32_t*)ctx->og_cells.p : nullptr;
+    uint4* list = masks ? nullptr : (uint4*)ctx->og_cells.p;
+    launch_og_build(ctx->st, ctx->blobref, g, g.fine, from[0], (float)side, mask, list, (uint32_t*)ctx->status.p);
+    launch_og_build(ctx->st, ctx->blobref, g, g.coarse, from[1], (float)side2, mask, list, (uint32_t*)ctx->status.p);
+    ctx->launches += 2;
     CKL();
     g.mask = g.list = (const uint32_t*)ctx->og_cells.p;
     ctx->blobref.og = g;

@@ -583,18 +583,19 @@ __device__ __forceinline__ float fast_dist(const SceneView& sv, int o, V p, floa
 struct OgBest {
     float d1, d2;
     int o1;
-    __device__ __forceinline__ OgBest() : d1(kMaxF), d2(kMaxF), o1(0) {}
+    float delta;
+    __device__ __forceinline__ OgBest() : d1(kMaxF), d2(kMaxF), o1(0), delta(0.0f) {}
     // An object that cannot come within delta of the nearest needs no exact
     // value (obj_dist's `best`), so its subtractions are skipped.
     __device__ __forceinline__ void eval(const SceneView& sv, int o, V p) {
-        const float d = fast_dist(sv, o, p, fmaxf(d1, 0.0f) + 2.0f * sv.og.delta);
+        const float d = fast_dist(sv, o, p, fmaxf(d1, 0.0f) + 2.0f * delta);
         o1 = d < d1 ? o : o1;
         d2 = fminf(d2, fmaxf(d, d1));
         d1 = fminf(d1, d);
     }
     // Whether the reference's query returns d1 (and, unless dist_only, o1).
     __device__ __forceinline__ bool exact(const SceneView& sv, V p, bool dist_only) const {
-        if (og_exact(d1, d2, sv.og.delta, dist_only)) return true;
+        if (og_exact(d1, d2, delta, dist_only)) return true;
         const int leaf = sv.fobj(o1).leaf;
         if (leaf < 0) return dist_only || d2 > d1;
         NoCount nc;
@@ -622,8 +623,8 @@ __device__ __forceinline__ DistHit dist_mat(const SceneView& sv, V p, C& cnt) {
     cnt.add(CN_SDF);
     if constexpr (sizeof(C) == 1) {
         uint32_t cell;
-        if (sv.og.mode != kOgOff && og_cell(sv.og, p.x, p.y, p.z, cell)) {
-            OgBest b;
+        OgBest b;
+        if (sv.og.mode != kOgOff && og_cell(sv.og, p.x, p.y, p.z, cell, b.delta)) {
             if (C::kTree3 || sv.og.mode == kOgMask) {
                 for (uint32_t m = __ldg(&sv.og.mask[cell]); m; m &= m - 1u) b.eval(sv, __ffs((int)m) - 1, p);
             } else {
@@ -656,16 +657,20 @@ __device__ __forceinline__ float scene_dist(const SceneView& sv, V p, C& cnt) {
 // leaves (a 512-object scene's visibility ran 10 of 32 lanes). Whole frames,
 // traversal -> grid with open_steps: Cornell box 5.61 -> 3.76 ms, 1920 x 1080
 // product scene 7.06 -> 5.66 ms, 512 objects at 961 x 541 97.8 -> 30.1 ms.
-template <bool kDistOnly, class C>
+// kUnion = false walks each lane's own mask instead, for warps whose lanes are
+// in unrelated places (the path tracer's states: 39.2 -> 35.0 ms; the product
+// frame's coherent rays, the other way: 5.50 -> 5.88 ms).
+template <bool kDistOnly, bool kUnion = true, class C>
 __device__ __forceinline__ DistHit dist_warp(const SceneView& sv, V p, bool active, C& cnt) {
     if (active) cnt.add(CN_SDF);
     if constexpr (sizeof(C) == 1) {
         if (sv.og.mode != kOgOff) {
             uint32_t cell = 0;
-            bool ok = active && og_cell(sv.og, p.x, p.y, p.z, cell);
             OgBest b;
+            bool ok = active && og_cell(sv.og, p.x, p.y, p.z, cell, b.delta);
             if (C::kTree3 || sv.og.mode == kOgMask) {
-                uint32_t m = __reduce_or_sync(0xffffffffu, ok ? __ldg(&sv.og.mask[cell]) : 0u);
+                uint32_t m = ok ? __ldg(&sv.og.mask[cell]) : 0u;
+                if constexpr (kUnion) m = __reduce_or_sync(0xffffffffu, m);
                 for (; m; m &= m - 1u) b.eval(sv, __ffs((int)m) - 1, p);
             } else if (ok) {
                 OgList l{__ldg(reinterpret_cast<const uint4*>(sv.og.list) + cell)};
@@ -884,7 +889,7 @@ __device__ __forceinline__ bool shadow_step_w(const SceneView& sv, ShadowRay& s,
     s.ph = h;
     s.t += clampr(h, 0.006f, 0.12f);
     if (!(s.steps < kShadowSteps && s.t < s.tmax) ||
-        (kSkips && sv.og.mode != kOgOff && open_steps(s, h, sv.og.delta))) {
+        (kSkips && sv.og.mode != kOgOff && open_steps(s, h, sv.og.coarse.delta))) {
         vis = clampr(s.res, 0.0f, 1.0f);
         return true;
     }

@@ -11,9 +11,9 @@ namespace ifx {
 // converged. A 512-object scene keeps some 30 objects per block.
 static constexpr int kOgBlock = 64;
 
-__global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, float lox, float loy, float loz,
-                                                       float cell, uint32_t nbx, uint32_t nby, uint32_t* mask,
-                                                       uint4* list, uint32_t* status) {
+__global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, OgLevel l, float lox, float loy,
+                                                       float loz, float cell, uint32_t nbx, uint32_t nby,
+                                                       uint32_t* mask, uint4* list, uint32_t* status) {
     IFX_SCENE_PROLOGUE(blob, status, sv);
     __shared__ uint32_t keep[kOgMaxObjects / 32];
     __shared__ float wmin[kOgBlock / 32];
@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, 
     const uint32_t nobj = (uint32_t)(sv.n_planes + sv.n_objects), words = (nobj + 31u) / 32u;
     const uint32_t b = blockIdx.x, t = threadIdx.x;
     const uint32_t bx = (b % nbx) * 4u, by = ((b / nbx) % nby) * 4u, bz = (b / (nbx * nby)) * 4u;
-    const float half = og_half(cell, g.delta), bhalf = og_half(4.0f * cell, g.delta);
+    const float half = og_half(cell, l.delta), bhalf = og_half(4.0f * cell, l.delta);
     {
         const V c{lox + (float)(bx + 2u) * cell, loy + (float)(by + 2u) * cell, loz + (float)(bz + 2u) * cell};
         float m = kMaxF;
@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, 
         if ((t & 31u) == 0) wmin[t >> 5] = m;
         __syncthreads();
         m = fminf(wmin[0], wmin[1]);
-        const float margin = og_margin(bhalf, g.delta) + og_margin(half, g.delta);
+        const float margin = og_margin(bhalf, l.delta) + og_margin(half, l.delta);
         for (uint32_t w = t >> 5; w < words; w += kOgBlock / 32) {
             const uint32_t i = w * 32u + (t & 31u);
             const bool in = i < nobj && og_listed(obj_dist(sv, sv.obj((int)(i < nobj ? i : 0u)), c, nc), m, margin);
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, 
     for (uint32_t w = 0; w < words; ++w)
         for (uint32_t v = keep[w]; v; v &= v - 1u)
             m = fminf(m, obj_dist(sv, sv.obj((int)(w * 32u) + __ffs((int)v) - 1), p, nc));
-    const float margin = og_margin(half, g.delta);
+    const float margin = og_margin(half, l.delta);
     uint32_t bits = 0, n = 0;
     float key[kOgListLen];
     uint32_t id[kOgListLen];
@@ -70,8 +70,8 @@ __global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, 
             }
             ++n;
         }
-    if (x >= g.dim[0] || y >= g.dim[1] || z >= g.dim[2]) return;
-    const uint32_t c = x + g.dim[0] * (y + g.dim[1] * z);
+    if (x >= l.dim[0] || y >= l.dim[1] || z >= l.dim[2]) return;
+    const uint32_t c = l.base + x + l.dim[0] * (y + l.dim[1] * z);
     if (g.mode == kOgMask) {
         mask[c] = bits;
     } else {
@@ -80,16 +80,16 @@ __global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, 
     }
 }
 
-void launch_og_build(cudaStream_t st, const BlobRef& blob, const ObjGrid& g, const float lo[3], float cell,
-                     uint32_t* mask, uint4* list, uint32_t* status) {
-    const uint32_t nbx = (g.dim[0] + 3u) / 4u, nby = (g.dim[1] + 3u) / 4u, nbz = (g.dim[2] + 3u) / 4u;
+void launch_og_build(cudaStream_t st, const BlobRef& blob, const ObjGrid& g, const OgLevel& l, const float lo[3],
+                     float cell, uint32_t* mask, uint4* list, uint32_t* status) {
+    const uint32_t nbx = (l.dim[0] + 3u) / 4u, nby = (l.dim[1] + 3u) / 4u, nbz = (l.dim[2] + 3u) / 4u;
     // The scene is read in place: nothing here waits, so no poll budget can
     // leave a grid half built, and the traversal stacks (at most 33 KiB) are
     // all its dynamic shared memory.
     BlobRef b = blob;
     b.staged = 0;
-    k_og_build<<<nbx * nby * nbz, kOgBlock, blob_smem(b, kOgBlock), st>>>(b, g, lo[0], lo[1], lo[2], cell, nbx, nby,
-                                                                         mask, list, status);
+    k_og_build<<<nbx * nby * nbz, kOgBlock, blob_smem(b, kOgBlock), st>>>(b, g, l, lo[0], lo[1], lo[2], cell, nbx,
+                                                                         nby, mask, list, status);
 }
 
 }  // namespace ifx

@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(128) k_path(ShadeParams P, uint32_t spp, const
         const float kx = (tap == 0 || tap == 3) ? 1.0f : -1.0f, ky = tap >= 2 ? 1.0f : -1.0f,
                     kz = (tap == 1 || tap == 3) ? 1.0f : -1.0f;
         const V qp = phase == kPhTap ? hp + V{kx, ky, kz} * 5e-4f : ray.ro + ray.rd * ray.t;
-        const DistHit h = dist_warp<false>(sv, qp, active, cnt);
+        const DistHit h = dist_warp<false, false>(sv, qp, active, cnt);
         if (!active) continue;
 
         // Where the lane goes after this query.

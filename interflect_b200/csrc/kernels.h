@@ -375,10 +375,10 @@ void configure_solve_kernels(int max_dyn_smem);
 void configure_shade_kernels(int max_dyn_smem);
 void configure_diff_kernels(int max_dyn_smem);
 void configure_path_kernels(int max_dyn_smem);
-// The object grid (objgrid.h) of the staged scene: lo is the grid's corner,
-// cell its cells' side; g.mode picks which of mask and list is written.
-void launch_og_build(cudaStream_t st, const BlobRef& blob, const ObjGrid& g, const float lo[3], float cell,
-                     uint32_t* mask, uint4* list, uint32_t* status);
+// Level l of the scene's object grid (objgrid.h): lo is its corner, cell its
+// cells' side; g.mode picks which of mask and list is written.
+void launch_og_build(cudaStream_t st, const BlobRef& blob, const ObjGrid& g, const OgLevel& l, const float lo[3],
+                     float cell, uint32_t* mask, uint4* list, uint32_t* status);
 // The path-traced reference mode (k_path.cu): p.film / p.out8 receive the
 // frame; sincos holds (sinf, cosf) of the 2^24 sampler angles.
 int launch_path(cudaStream_t st, const ShadeParams& p, uint32_t spp, const float2* sincos,

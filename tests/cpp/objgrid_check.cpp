@@ -41,26 +41,20 @@ int main(int argc, char** argv) {
         for (uint32_t k = 0; k < sc.bvh.nodes[n].count; ++k)
             leaf[sc.planes.size() + sc.bvh.nodes[n].start + k] = (int)n;
     const float lo[3] = {sc.lo.x, sc.lo.y, sc.lo.z}, hi[3] = {sc.hi.x, sc.hi.y, sc.hi.z};
-    double ext = 0.0, scale = 0.0;
-    for (int a = 0; a < 3; ++a) {
-        ext = std::max(ext, (double)hi[a] - (double)lo[a]);
-        scale = std::max(scale, std::max(std::fabs((double)lo[a]), std::fabs((double)hi[a])));
-    }
-    scale += (double)sc.diag();
     ifx::ObjGrid g{};
-    const double cs = ext / cells;
-    g.delta = (float)(scale / 65536.0);
-    g.inv = (float)(1.0 / cs);
-    for (int a = 0; a < 3; ++a) {
-        g.bias[a] = (float)(-(double)lo[a] / cs - 0.5);
-        g.dim[a] = (uint32_t)std::min(cells, std::max(1, (int)std::ceil(((double)hi[a] - (double)lo[a]) / cs)));
-    }
+    float from[2][3];
+    const double diag = sc.diag(), side[2] = {
+        ifx::og_level(g.fine, lo, hi, cells, 1.0, 0.0, diag, 0, from[0]),
+        ifx::og_level(g.coarse, lo, hi, ifx::kOgCoarseCells, ifx::kOgCoarseExtent, 0.0, diag,
+                      g.fine.dim[0] * g.fine.dim[1] * g.fine.dim[2], from[1])};
     std::unordered_map<uint32_t, std::vector<uint32_t>> lists;
     auto list_of = [&](uint32_t c) -> const std::vector<uint32_t>& {
         auto it = lists.find(c);
         if (it != lists.end()) return it->second;
-        const uint32_t x = c % g.dim[0], y = c / g.dim[0] % g.dim[1], z = c / (g.dim[0] * g.dim[1]);
-        const float s = (float)cs;
+        const int k = c >= g.coarse.base;
+        const ifx::OgLevel& l = k ? g.coarse : g.fine;
+        const uint32_t i = c - l.base, x = i % l.dim[0], y = i / l.dim[0] % l.dim[1], z = i / (l.dim[0] * l.dim[1]);
+        const float s = (float)side[k], *lo = from[k];
         const V3 p(lo[0] + ((float)x + 0.5f) * s, lo[1] + ((float)y + 0.5f) * s, lo[2] + ((float)z + 0.5f) * s);
         float m = 3.4028235e38f;
         std::vector<float> d;
@@ -70,7 +64,7 @@ int main(int argc, char** argv) {
         }
         std::vector<uint32_t> v;
         for (uint32_t i = 0; i < objs.size(); ++i)
-            if (ifx::og_listed(d[i], m, ifx::og_margin(ifx::og_half(s, g.delta), g.delta))) v.push_back(i);
+            if (ifx::og_listed(d[i], m, ifx::og_margin(ifx::og_half(s, l.delta), l.delta))) v.push_back(i);
         return lists.emplace(c, v).first->second;
     };
     std::mt19937 rng(7);
@@ -80,7 +74,8 @@ int main(int argc, char** argv) {
         const DistHit ref = sc.dist_mat(p);
         ++q;
         uint32_t c;
-        if (!ifx::og_cell(g, p.x, p.y, p.z, c)) {
+        float delta;
+        if (!ifx::og_cell(g, p.x, p.y, p.z, c, delta)) {
             ++outside;
             return ref.d;
         }
@@ -99,7 +94,7 @@ int main(int argc, char** argv) {
         }
         bool wrong = false;
         for (bool dist_only : {false, true}) {
-            bool ok = ifx::og_exact(d1, d2, g.delta, dist_only);
+            bool ok = ifx::og_exact(d1, d2, delta, dist_only);
             if (!ok) {
                 if (dist_only) ++ties;
                 if (leaf[o1] < 0) {
@@ -138,7 +133,7 @@ int main(int argc, char** argv) {
             }
             t += d;
         }
-        float h = sc.dist(p), lower = ifx::og_open_first(h, g.delta);
+        float h = sc.dist(p), lower = ifx::og_open_first(h, g.coarse.delta);
         t = 0.0f;
         for (int s = 0; s < 60; ++s) {
             t += ifx::kOpenStep;
@@ -151,7 +146,7 @@ int main(int argc, char** argv) {
                 }
                 lower = ifx::og_open_next(lower);
             } else {
-                lower = ifx::og_open_first(d, g.delta);
+                lower = ifx::og_open_first(d, g.coarse.delta);
             }
         }
     }
