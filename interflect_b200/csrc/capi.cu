@@ -631,10 +631,13 @@ static int objgrid_build(ifx_ctx* ctx, const std::vector<uint8_t>& blob) {
     const double side2 =
         og_level(g.coarse, lo, hi, kOgCoarseCells, kOgCoarseExtent, scale, diag, fine, from[1]);
     const size_t ncells = (size_t)fine + (size_t)g.coarse.dim[0] * g.coarse.dim[1] * g.coarse.dim[2];
-    // A scene whose coordinates dwarf its extent: the margins would list everything.
-    if (!(side > 0.0) || !(g.fine.delta <= 0.25 * side) || !(g.coarse.delta <= 0.25 * side2)) return IFX_OK;
+    // A scene whose coordinates dwarf its extent: the margins would list
+    // everything. (And at 1e9 squares of lengths are still far from overflow:
+    // no distance is NaN.)
+    if (!(scale < 1e9) || !(diag < 1e9) || !(side > 0.0) || !(g.fine.delta <= 0.25 * side) || !(g.coarse.delta <= 0.25 * side2)) return IFX_OK;
     ENSURE(ctx->og_cells, ncells * (masks ? 4 : 16));
     g.mode = masks ? kOgMask : kOgList;
+    g.id_bits = nobj <= kOgKeyObjects ? 12 : 16;
     uint32_t* mask = masks ? (uint32_t*)ctx->og_cells.p : nullptr;
     uint4* list = masks ? nullptr : (uint4*)ctx->og_cells.p;
     launch_og_build(ctx->st, ctx->blobref, g, g.fine, from[0], (float)side, mask, list, (uint32_t*)ctx->status.p);

@@ -7,6 +7,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include "layout.h"
@@ -584,7 +585,7 @@ struct OgBest {
     float d1, d2;
     int o1;
     float delta;
-    __device__ __forceinline__ OgBest() : d1(kMaxF), d2(kMaxF), o1(0), delta(0.0f) {}
+    __device__ __forceinline__ explicit OgBest(float delta_) : d1(kMaxF), d2(kMaxF), o1(0), delta(delta_) {}
     // An object that cannot come within delta of the nearest needs no exact
     // value (obj_dist's `best`), so its subtractions are skipped.
     __device__ __forceinline__ void eval(const SceneView& sv, int o, V p) {
@@ -603,17 +604,25 @@ struct OgBest {
     }
 };
 
-// The 16-bit entries of a cell's list, taken one by one.
-struct OgList {
-    uint4 e;
-    __device__ __forceinline__ uint32_t head() const { return e.x & 0xffffu; }
-    __device__ __forceinline__ void pop() {
+// Evaluates the objects of a cell's list, as far as they matter at p; false
+// if objects that the list leaves out can matter.
+__device__ __forceinline__ bool og_walk_list(const SceneView& sv, OgBest& b, uint32_t cell, bool coarse, V p) {
+    const OgLevel& l = coarse ? sv.og.coarse : sv.og.fine;
+    uint4 e = __ldg(reinterpret_cast<const uint4*>(sv.og.list) + cell);
+    const float base = __half2float(__ushort_as_half((unsigned short)(e.x & 0xffffu)));
+    const float off = og_from_centre(l, p.x, p.y, p.z);
+    const uint32_t ids = (1u << sv.og.id_bits) - 1u;
+    while (true) {
         e.x = __funnelshift_r(e.x, e.y, 16);
         e.y = __funnelshift_r(e.y, e.z, 16);
         e.z = __funnelshift_r(e.z, e.w, 16);
-        e.w = (e.w >> 16) | 0xffff0000u;
+        e.w = (e.w >> 16) | (kOgNone << 16);
+        const uint32_t word = e.x & 0xffffu;
+        if (word == kOgNone || og_beyond(word >> sv.og.id_bits, l.key_step, base, off, b.d1, l.delta)) return true;
+        if ((word & ids) == og_more(sv.og.id_bits)) return false;
+        b.eval(sv, (int)(word & ids), p);
     }
-};
+}
 
 // scene.rs:191-208 for one lane: the object grid's answer where it is the
 // reference's (objgrid.h), the reference's traversal elsewhere. The counting
@@ -623,15 +632,16 @@ __device__ __forceinline__ DistHit dist_mat(const SceneView& sv, V p, C& cnt) {
     cnt.add(CN_SDF);
     if constexpr (sizeof(C) == 1) {
         uint32_t cell;
-        OgBest b;
-        if (sv.og.mode != kOgOff && og_cell(sv.og, p.x, p.y, p.z, cell, b.delta)) {
+        bool coarse;
+        if (sv.og.mode != kOgOff && og_cell(sv.og, p.x, p.y, p.z, cell, coarse)) {
+            OgBest b(coarse ? sv.og.coarse.delta : sv.og.fine.delta);
+            bool ok = true;
             if (C::kTree3 || sv.og.mode == kOgMask) {
                 for (uint32_t m = __ldg(&sv.og.mask[cell]); m; m &= m - 1u) b.eval(sv, __ffs((int)m) - 1, p);
             } else {
-                OgList l{__ldg(reinterpret_cast<const uint4*>(sv.og.list) + cell)};
-                for (uint32_t o = l.head(); o < kOgOverflow; l.pop(), o = l.head()) b.eval(sv, (int)o, p);
+                ok = og_walk_list(sv, b, cell, coarse, p);
             }
-            if (b.d1 < kMaxF && b.exact(sv, p, false)) return DistHit{b.d1, sv.obj(b.o1).mat};
+            if (ok && b.d1 < kMaxF && b.exact(sv, p, false)) return DistHit{b.d1, sv.obj(b.o1).mat};
         }
     }
     return dist_mat_ref(sv, p, cnt);
@@ -666,15 +676,15 @@ __device__ __forceinline__ DistHit dist_warp(const SceneView& sv, V p, bool acti
     if constexpr (sizeof(C) == 1) {
         if (sv.og.mode != kOgOff) {
             uint32_t cell = 0;
-            OgBest b;
-            bool ok = active && og_cell(sv.og, p.x, p.y, p.z, cell, b.delta);
+            bool coarse = false;
+            bool ok = active && og_cell(sv.og, p.x, p.y, p.z, cell, coarse);
+            OgBest b(coarse ? sv.og.coarse.delta : sv.og.fine.delta);
             if (C::kTree3 || sv.og.mode == kOgMask) {
                 uint32_t m = ok ? __ldg(&sv.og.mask[cell]) : 0u;
                 if constexpr (kUnion) m = __reduce_or_sync(0xffffffffu, m);
                 for (; m; m &= m - 1u) b.eval(sv, __ffs((int)m) - 1, p);
             } else if (ok) {
-                OgList l{__ldg(reinterpret_cast<const uint4*>(sv.og.list) + cell)};
-                for (uint32_t o = l.head(); o < kOgOverflow; l.pop(), o = l.head()) b.eval(sv, (int)o, p);
+                ok = og_walk_list(sv, b, cell, coarse, p);
             }
             DistHit h{b.d1, 0u};
             ok = ok && b.d1 < kMaxF && b.exact(sv, p, kDistOnly);

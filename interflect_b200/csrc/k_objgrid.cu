@@ -2,6 +2,8 @@
 // counterpart in the reference, which traverses its BVH for every query.
 #include "kcommon.cuh"
 
+#include <cuda_fp16.h>
+
 namespace ifx {
 
 // One CTA per block of 4 x 4 x 4 cells, a thread per cell. The CTA first
@@ -49,7 +51,7 @@ __global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, 
     uint32_t bits = 0, n = 0;
     float key[kOgListLen];
     uint32_t id[kOgListLen];
-    for (uint32_t k = 0; k < kOgListLen; ++k) id[k] = kOgNone, key[k] = 0.0f;
+    for (uint32_t k = 0; k < kOgListLen; ++k) id[k] = 0, key[k] = 0.0f;
     for (uint32_t w = 0; w < words; ++w)
         for (uint32_t v = keep[w]; v; v &= v - 1u) {
             const uint32_t i = w * 32u + (uint32_t)__ffs((int)v) - 1u;
@@ -59,12 +61,13 @@ __global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, 
                 bits |= 1u << (i & 31u);
                 continue;
             }
-            if (n < kOgListLen) {
-                uint32_t j = n;
-                for (; j > 0 && key[j - 1] > d; --j) {
-                    key[j] = key[j - 1];
-                    id[j] = id[j - 1];
-                }
+            uint32_t j = n < kOgListLen ? n : kOgListLen;
+            for (; j > 0 && key[j - 1] > d; --j) {
+                if (j == kOgListLen) continue;
+                key[j] = key[j - 1];
+                id[j] = id[j - 1];
+            }
+            if (j < kOgListLen) {
                 key[j] = d;
                 id[j] = i;
             }
@@ -74,10 +77,19 @@ __global__ void __launch_bounds__(kOgBlock) k_og_build(BlobRef blob, ObjGrid g, 
     const uint32_t c = l.base + x + l.dim[0] * (y + l.dim[1] * z);
     if (g.mode == kOgMask) {
         mask[c] = bits;
-    } else {
-        if (n > kOgListLen) id[0] = kOgOverflow;
-        list[c] = make_uint4(id[0] | id[1] << 16, id[2] | id[3] << 16, id[4] | id[5] << 16, id[6] | id[7] << 16);
+        return;
     }
+    const __half h = __float2half_rd(fminf(fmaxf(m, -60000.0f), 60000.0f));
+    const float base = __half2float(h);
+    uint32_t e[kOgListLen];
+    for (uint32_t k = 0; k < kOgListLen; ++k) {
+        e[k] = kOgNone;
+        if (k >= n) continue;
+        e[k] = n > kOgListLen && k == kOgListLen - 1 ? og_more(g.id_bits) : id[k];
+        if (g.id_bits < 16) e[k] |= og_key(key[k], base, l.key_step) << g.id_bits;
+    }
+    list[c] = make_uint4((uint32_t)__half_as_ushort(h) | e[0] << 16, e[1] | e[2] << 16, e[3] | e[4] << 16,
+                         e[5] | e[6] << 16);
 }
 
 void launch_og_build(cudaStream_t st, const BlobRef& blob, const ObjGrid& g, const OgLevel& l, const float lo[3],

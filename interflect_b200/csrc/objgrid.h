@@ -18,6 +18,11 @@
 //    max(the nearest distance there, 0) + og_margin. An object that is not
 //    listed is then, everywhere in the cell, farther than max(G, 0) + 3 delta,
 //    G being the nearest distance at that point.
+//  * A list carries a lower bound of each object's distance at the cell's
+//    centre (og_key), and is sorted by it: a query stops at the first object
+//    that cannot come within max(d1, 0) + delta of its point. A list too long
+//    for its cell keeps the nearest objects and ends with the key of the next:
+//    a query that gets there without stopping knows no answer.
 //  * The query returns the smallest listed distance d1, its object o1, and d2,
 //    the second smallest. If d2 > max(d1, 0) + delta/4, the reference's query
 //    (bvh.rs:100-150: prune a node when its box distance >= the best so far,
@@ -53,7 +58,7 @@
 namespace ifx {
 
 // Two levels: the fine one over the scene's bounds, and one of coarse cells
-// over four times their extent, for the rays of a camera outside the bounds
+// over eight times their extent, for the rays of a camera outside the bounds
 // and those that leave them.
 struct OgLevel {
     float inv;      // cells per unit length
@@ -61,22 +66,29 @@ struct OgLevel {
     uint32_t dim[3];
     uint32_t base;  // the level's first cell
     float delta;
+    float side, key_step;  // the cells' side; what one unit of og_key stands for
 };
 struct ObjGrid {
     const uint32_t* mask;  // kOgMask: per cell, bit i = stored object i is listed
-    const uint32_t* list;  // kOgList: per cell, eight 16-bit stored-object indices, nearest first, kOgNone-padded
+    // kOgList: per cell eight 16-bit words, the nearest distance at the centre
+    // (half precision, rounded down), then up to kOgListLen objects, nearest
+    // first: the stored-object index in the low id_bits, its og_key above.
+    const uint32_t* list;
     OgLevel fine, coarse;
+    int id_bits;           // 12, or 16 (and no keys) above kOgKeyObjects
     int mode;              // kOgOff, kOgMask, kOgList
 };
-static constexpr int kOgCoarseCells = 32;
-static constexpr float kOgCoarseExtent = 4.0f;
+static constexpr int kOgCoarseCells = 64;
+static constexpr float kOgCoarseExtent = 8.0f;
 enum : int { kOgOff = 0, kOgMask = 1, kOgList = 2 };
 // Scenes of at most this many stored objects (planes and bounded) use masks.
 static constexpr uint32_t kOgMaskObjects = 32;
 static constexpr uint32_t kOgMaxObjects = 32768;
-static constexpr uint32_t kOgListLen = 8;
-static constexpr uint32_t kOgNone = 0xffffu;      // end of a list
-static constexpr uint32_t kOgOverflow = 0xfffeu;  // first entry of a cell with more than kOgListLen objects
+static constexpr uint32_t kOgKeyObjects = 4094;
+static constexpr uint32_t kOgListLen = 7;
+static constexpr uint32_t kOgNone = 0xffffu;  // end of a list
+// The object index of a list's last word that stands for all that were left out: 2^id_bits - 2.
+IFX_OG_FN uint32_t og_more(int id_bits) { return (1u << id_bits) - 2u; }
 
 IFX_OG_FN uint32_t og_bits(float x) {
 #ifdef __CUDA_ARCH__
@@ -95,6 +107,32 @@ IFX_OG_FN uint32_t og_axis(float p, float inv, float bias) {
     return og_bits(fmaf(p, inv, bias) + 8388608.0f) - 0x4B000000u;
 }
 
+// At least the distance of a point from its cell's centre: the parts of the
+// cell index that og_axis rounds away, in cells' sides.
+IFX_OG_FN float og_off_axis(float p, float inv, float bias) {
+    const float f = fmaf(p, inv, bias);
+    return f - ((f + 8388608.0f) - 8388608.0f);
+}
+IFX_OG_FN float og_from_centre(const OgLevel& l, float x, float y, float z) {
+    const float a = og_off_axis(x, l.inv, l.bias[0]), b = og_off_axis(y, l.inv, l.bias[1]),
+                c = og_off_axis(z, l.inv, l.bias[2]);
+    return l.side * sqrtf(a * a + b * b + c * c) + 0.25f * l.delta;
+}
+
+// The key of an object at distance d from the centre of a cell whose nearest
+// distance there is at least `base`: d is at least base + key * key_step.
+IFX_OG_FN uint32_t og_key(float d, float base, float key_step) {
+    const float k = (d - base) / key_step * (1.0f - 1e-6f);
+    return k >= 15.0f ? 15u : (k > 0.0f ? (uint32_t)k : 0u);
+}
+
+// Whether an object of that key cannot come within max(d1, 0) + delta of a
+// point `off` from the centre (an object's distance there is at least its
+// distance at the centre less `off`).
+IFX_OG_FN bool og_beyond(uint32_t key, float key_step, float base, float off, float d1, float delta) {
+    return (float)key * key_step > fmaxf(d1, 0.0f) + 1.5f * delta + off - base;
+}
+
 IFX_OG_FN bool og_level_cell(const OgLevel& l, float x, float y, float z, uint32_t& cell) {
     const uint32_t i = og_axis(x, l.inv, l.bias[0]), j = og_axis(y, l.inv, l.bias[1]),
                    k = og_axis(z, l.inv, l.bias[2]);
@@ -102,12 +140,22 @@ IFX_OG_FN bool og_level_cell(const OgLevel& l, float x, float y, float z, uint32
     return i < l.dim[0] && j < l.dim[1] && k < l.dim[2];
 }
 
-IFX_OG_FN bool og_cell(const ObjGrid& g, float x, float y, float z, uint32_t& cell, float& delta) {
-    delta = g.fine.delta;
+// The cell of a point and which level it is of; false outside the grid.
+IFX_OG_FN bool og_cell(const ObjGrid& g, float x, float y, float z, uint32_t& cell, bool& coarse) {
+    coarse = false;
     if (og_level_cell(g.fine, x, y, z, cell)) return true;
-    delta = g.coarse.delta;
+    coarse = true;
     return og_level_cell(g.coarse, x, y, z, cell);
 }
+
+// Half-diagonal of a cube of side `side`, with room for the rounding of the
+// cell index and of the centre.
+IFX_OG_FN float og_half(float side, float delta) { return side * 0.8660255f + delta; }
+
+// The listing margin over a cell of half-diagonal `half`: the nearest distance
+// and an object's distance can each change by `half` between the centre and a
+// point of the cell.
+IFX_OG_FN float og_margin(float half, float delta) { return 2.0f * half + 4.0f * delta; }
 
 // A level of `cells` cells along the longest side of [lo, hi] grown by `grow`
 // about its centre; `scale` is the largest coordinate, length or radius of the
@@ -129,17 +177,10 @@ inline double og_level(OgLevel& l, const float lo[3], const float hi[3], int cel
         l.dim[a] = (uint32_t)(n < 1 ? 1 : (n > cells ? cells : n));
     }
     l.delta = (float)((scale + diag) / 65536.0);
+    l.side = (float)side;
+    l.key_step = og_margin(og_half(l.side, l.delta), l.delta) / 16.0f;
     return side;
 }
-
-// Half-diagonal of a cube of side `side`, with room for the rounding of the
-// cell index and of the centre.
-IFX_OG_FN float og_half(float side, float delta) { return side * 0.8660255f + delta; }
-
-// The listing margin over a cell of half-diagonal `half`: the nearest distance
-// and an object's distance can each change by `half` between the centre and a
-// point of the cell.
-IFX_OG_FN float og_margin(float half, float delta) { return 2.0f * half + 4.0f * delta; }
 
 IFX_OG_FN bool og_listed(float d, float nearest, float margin) { return !(d > fmaxf(nearest, 0.0f) + margin); }
 

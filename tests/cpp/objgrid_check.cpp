@@ -47,8 +47,13 @@ int main(int argc, char** argv) {
         ifx::og_level(g.fine, lo, hi, cells, 1.0, 0.0, diag, 0, from[0]),
         ifx::og_level(g.coarse, lo, hi, ifx::kOgCoarseCells, ifx::kOgCoarseExtent, 0.0, diag,
                       g.fine.dim[0] * g.fine.dim[1] * g.fine.dim[2], from[1])};
-    std::unordered_map<uint32_t, std::vector<uint32_t>> lists;
-    auto list_of = [&](uint32_t c) -> const std::vector<uint32_t>& {
+    // Per cell: its objects and their keys, nearest first, and the nearest distance at the centre.
+    struct Cell {
+        std::vector<std::pair<uint32_t, uint32_t>> items;
+        float base;
+    };
+    std::unordered_map<uint32_t, Cell> lists;
+    auto list_of = [&](uint32_t c) -> const Cell& {
         auto it = lists.find(c);
         if (it != lists.end()) return it->second;
         const int k = c >= g.coarse.base;
@@ -62,28 +67,44 @@ int main(int argc, char** argv) {
             d.push_back(o->dist(p));
             m = std::fmin(m, d.back());
         }
-        std::vector<uint32_t> v;
+        Cell v;
+        v.base = m - std::fabs(m) * 1e-3f;  // as much lower as half precision can round
         for (uint32_t i = 0; i < objs.size(); ++i)
-            if (ifx::og_listed(d[i], m, ifx::og_margin(ifx::og_half(s, l.delta), l.delta))) v.push_back(i);
+            if (ifx::og_listed(d[i], m, ifx::og_margin(ifx::og_half(s, l.delta), l.delta)))
+                v.items.push_back({i, ifx::og_key(d[i], v.base, l.key_step)});
+        std::stable_sort(v.items.begin(), v.items.end(),
+                         [&](auto& a, auto& b) { return d[a.first] < d[b.first]; });
         return lists.emplace(c, v).first->second;
     };
     std::mt19937 rng(7);
     std::uniform_real_distribution<float> U(0.0f, 1.0f);
-    long q = 0, bad = 0, outside = 0, ties = 0, unsure = 0, listed = 0, open = 0;
+    long q = 0, bad = 0, outside = 0, ties = 0, unsure = 0, unknown = 0, listed = 0, evaluated = 0, open = 0;
     auto check = [&](V3 p) {
         const DistHit ref = sc.dist_mat(p);
         ++q;
         uint32_t c;
-        float delta;
-        if (!ifx::og_cell(g, p.x, p.y, p.z, c, delta)) {
+        bool coarse;
+        if (!ifx::og_cell(g, p.x, p.y, p.z, c, coarse)) {
             ++outside;
             return ref.d;
         }
         float d1 = 3.4028235e38f, d2 = d1;
         uint32_t o1 = 0;
-        for (uint32_t i : list_of(c)) {
-            const float d = objs[i]->dist(p);
+        const ifx::OgLevel& l = coarse ? g.coarse : g.fine;
+        const float delta = l.delta, off = ifx::og_from_centre(l, p.x, p.y, p.z);
+        const Cell& cell = list_of(c);
+        const bool capped = cell.items.size() > ifx::kOgListLen;
+        bool known = true;
+        for (size_t n = 0; n < cell.items.size(); ++n) {
+            const auto [i, key] = cell.items[n];
             ++listed;
+            if (ifx::og_beyond(key, l.key_step, cell.base, off, d1, delta)) break;
+            if (capped && n == ifx::kOgListLen - 1) {
+                known = false;
+                break;
+            }
+            const float d = objs[i]->dist(p);
+            ++evaluated;
             if (d < d1) {
                 d2 = d1;
                 d1 = d;
@@ -91,6 +112,10 @@ int main(int argc, char** argv) {
             } else if (d < d2) {
                 d2 = d;
             }
+        }
+        if (!known) {
+            ++unknown;
+            return ref.d;
         }
         bool wrong = false;
         for (bool dist_only : {false, true}) {
@@ -150,9 +175,9 @@ int main(int argc, char** argv) {
             }
         }
     }
-    std::printf("objects %zu, queries %ld, mean listed %.2f, outside %ld, near ties %ld (unsure %ld), open steps %ld, "
+    std::printf("objects %zu, queries %ld, mean listed %.2f evaluated %.2f, outside %ld, unknown %ld, near ties %ld (unsure %ld), open steps %ld, "
                 "disagreements %ld\n",
-                objs.size(), q, (double)listed / q, outside, ties, unsure, open, bad);
+                objs.size(), q, (double)listed / q, (double)evaluated / q, outside, unknown, ties, unsure, open, bad);
     if (bad) return 1;
     std::printf("every accepted answer equals the reference traversal\n");
     return 0;
