@@ -1371,10 +1371,9 @@ extern "C" int ifx_transfer_upload(ifx_ctx* ctx, const uint32_t* starts, uint64_
 
 // solve.rs:27-39 on ctx->st: direct = rad = E and irr = 0 for every
 // surfel, the SDF evaluations added to *evals_dev, per-light factors into
-// `terms` (nullable, n x nl). Few (surfel, light) slots leave most lanes of
-// the GPU idle: there each surfel's marches run as one independent thread
-// (latency-bound, so warp-synchronous rounds would only add waiting); many
-// slots go through a queue to the lane-refilling shadow kernel.
+// `terms` (nullable, n x nl). Few surfels of one light run as one independent
+// thread each; the others' (surfel, light) slots go through a queue to the
+// lane-refilling shadow kernel (kLightSlotsQueued).
 // The light stage on stream st, its errors in *status.
 static int light_surfels_run(ifx_ctx* ctx, cudaStream_t st, uint32_t* status, unsigned long long* evals_dev,
                              unsigned long long* counts, float* terms) {
@@ -1382,7 +1381,7 @@ static int light_surfels_run(ifx_ctx* ctx, cudaStream_t st, uint32_t* status, un
     if (n == 0) return IFX_OK;
     const int nl = (int)(ctx->scene.lights.size() + ctx->scene.sphere_lights.size());
     const size_t slots = (size_t)n * (size_t)(nl > 0 ? nl : 1);
-    if (slots < kLightSlotsQueued) {
+    if (nl <= 1 && slots < kLightSlotsQueued) {
         launch_light_surfels(st, ctx->blobref, ctx->sarr(), n, evals_dev, status, counts, terms);
         ctx->launches++;
         CKL();
