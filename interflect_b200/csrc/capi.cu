@@ -1448,9 +1448,9 @@ static void solve_graph_drop(ifx_ctx* ctx) {
     ctx->solve_graph = nullptr;
 }
 
-// Enqueues the control-block reset and max_bounces bounces (three launches
-// each) on ctx->st; bounces after convergence return at once on the
-// device-side flag.
+// Enqueues bounces [first, end) (two launches each) and the stop test after
+// them on ctx->st; bounces after convergence return at once on the device-side
+// flag.
 static void solve_enqueue(ifx_ctx* ctx, uint32_t first, uint32_t end) {
     SolveCtl* ctl = (SolveCtl*)ctx->ctl.p;
     for (uint32_t it = first; it < end; ++it) {
@@ -1461,6 +1461,9 @@ static void solve_enqueue(ifx_ctx* ctx, uint32_t first, uint32_t end) {
                             &l, 0, ctx->sell_ready ? &ctx->sellm : nullptr);
         ctx->launches += (uint64_t)l;
     }
+    int l = 0;
+    launch_solve_end(ctx->st, ctl, end, &l);
+    ctx->launches += (uint64_t)l;
 }
 
 extern "C" int ifx_solve(ifx_ctx* ctx, uint32_t max_bounces, ifx_solve_stats* out) {
@@ -1475,7 +1478,7 @@ extern "C" int ifx_solve(ifx_ctx* ctx, uint32_t max_bounces, ifx_solve_stats* ou
     SolveCtl h{};
     // Up to kSolveGraphBounces the whole sequence (the bounces after
     // convergence are no-ops) is one graph launch: the host neither issues
-    // three launches per bounce nor looks at the flag in between.
+    // two launches per bounce nor looks at the flag in between.
     const uint32_t kSolveGraphBounces = 64;
     bool graphed = false;
     if (max_bounces > 0 && max_bounces <= kSolveGraphBounces) {
@@ -2339,7 +2342,7 @@ struct ifx_multiscene {
     };
     std::vector<Member> members;
     bool valid = true;  // false once a member context was destroyed
-    DBuf scenes, bases, ctl, live, bar, status, srgb_t;
+    DBuf scenes, bases, ctl, bar, status, srgb_t;
     MsParams params{};
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -2432,7 +2435,7 @@ extern "C" void ifx_multiscene_destroy(ifx_multiscene* ms) {
             o.erase(std::remove(o.begin(), o.end(), ms), o.end());
         }
     ms_drop_graph(ms);
-    for (DBuf* b : {&ms->scenes, &ms->bases, &ms->ctl, &ms->live, &ms->bar, &ms->status, &ms->srgb_t}) free_buf(*b);
+    for (DBuf* b : {&ms->scenes, &ms->bases, &ms->ctl, &ms->bar, &ms->status, &ms->srgb_t}) free_buf(*b);
     if (ms->e0) cudaEventDestroy(ms->e0);
     if (ms->e1) cudaEventDestroy(ms->e1);
     if (ms->st) cudaStreamDestroy(ms->st);
@@ -2586,7 +2589,6 @@ extern "C" int ifx_multiscene_build(ifx_multiscene* ms, int autotune, int* grid_
     MSENSURE(ms->scenes, table.size() * sizeof(MsScene));
     MSENSURE(ms->bases, bases.size() * 4);
     MSENSURE(ms->ctl, (size_t)S * sizeof(SolveCtl));
-    MSENSURE(ms->live, 16);
     MSENSURE(ms->bar, sizeof(MsBarrier));
     MSENSURE(ms->status, 16);
     MSCK(cudaMemcpyAsync(ms->scenes.p, table.data(), table.size() * sizeof(MsScene), cudaMemcpyHostToDevice, ms->st));
@@ -2604,7 +2606,6 @@ extern "C" int ifx_multiscene_build(ifx_multiscene* ms, int autotune, int* grid_
     p.total_pix = (uint32_t)tp;
     p.max_bounces = maxb;
     p.ctl = (SolveCtl*)ms->ctl.p;
-    p.live = (uint32_t*)ms->live.p;
     p.bar = (MsBarrier*)ms->bar.p;
     p.status = (uint32_t*)ms->status.p;
     p.srgb_t = (const float*)ms->srgb_t.p;

@@ -42,8 +42,7 @@ __global__ void __launch_bounds__(256) k_multi_frame(MsParams M) {
     const MsScene* sc = M.scenes;
 
     // Relight, and reset the per-scene solve controls.
-    for (uint32_t s = tid; s < (uint32_t)M.S; s += stride) M.ctl[s] = SolveCtl{0u, 0u, 0u, 0u};
-    if (tid == 0) M.live[0] = (uint32_t)M.S;
+    for (uint32_t s = tid; s < (uint32_t)M.S; s += stride) M.ctl[s] = SolveCtl{};
     for (uint32_t item = tid; item < M.total_surf; item += stride) {
         const MsScene& S = sc[scene_of(M.surf_base, M.S, item)];
         const uint32_t i = item - S.surf_base;
@@ -60,16 +59,41 @@ __global__ void __launch_bounds__(256) k_multi_frame(MsParams M) {
     }
     if (!grid_barrier(M.bar, M.status, M.polls)) return;
 
-    for (uint32_t it = 0; it < M.max_bounces; ++it) {
+    // The stop test of each bounce (solve.rs:93-101, with each scene's own
+    // bounce cap) is part of the next one's first phase: every CTA forms it
+    // from the residuals, CTA 0 also notes the scenes' statistics. `it` runs
+    // one past the last bounce for that.
+    for (uint32_t it = 0; it <= M.max_bounces; ++it) {
+        auto stopped = [&](int s) { return solve_stopped(M.ctl[s], it, 0) || it >= sc[s].max_bounces; };
+        int live = 0;
+        for (int s = (int)threadIdx.x; s < M.S; s += (int)blockDim.x) {
+            const bool stop = stopped(s);
+            live |= !stop;
+            if (blockIdx.x == 0) solve_note(M.ctl[s], it, stop);
+        }
+        if (!__syncthreads_or(live)) break;
         // solve.rs:61-73: cluster means, members summed in member order.
         for (uint32_t item = tid; item < M.total_clus; item += stride) {
             const int s = scene_of(M.clus_base, M.S, item);
-            if (M.ctl[s].done) continue;
+            if (stopped(s)) continue;
             const MsScene& S = sc[s];
             const uint32_t c = item - S.clus_base;
             const uint2 r = S.crange[c];
             V acc{0.0f, 0.0f, 0.0f};
-            for (uint32_t k = r.x; k < r.y; ++k) {
+            uint32_t k = r.x;
+            for (; k + 4 <= r.y; k += 4) {  // four members' loads in flight
+                float4 v[4];
+                float a[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint32_t m = S.members[k + q];
+                    v[q] = S.rad[m];
+                    a[q] = S.sp[m].w;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc = acc + V{v[q].x * a[q], v[q].y * a[q], v[q].z * a[q]};
+            }
+            for (; k < r.y; ++k) {
                 const uint32_t m = S.members[k];
                 const float4 v = S.rad[m];
                 const float a = S.sp[m].w;
@@ -85,9 +109,7 @@ __global__ void __launch_bounds__(256) k_multi_frame(MsParams M) {
             if (!M.ctl[s].done) {
                 const MsScene& S = sc[s];
                 const uint32_t i = item - S.surf_base;
-                V irr{0.0f, 0.0f, 0.0f};
-                const uint32_t e = S.starts[i + 1];
-                for (uint32_t k = S.starts[i]; k < e; ++k) irr = irr + mk4(S.crad[S.idx[k]]) * S.w[k];
+                const V irr = jacobi_row(S.crad, S.idx, S.w, S.starts[i], S.starts[i + 1], 1);
                 V nr = mk4(S.direct[i]) + mk4(S.albedo[i]) * irr;
                 V diff = vabs(nr - mk4(S.rad[i]));
                 float d = fmaxf(diff.x, fmaxf(diff.y, diff.z));
@@ -98,29 +120,9 @@ __global__ void __launch_bounds__(256) k_multi_frame(MsParams M) {
             // One atomic per (warp, scene): the lanes of a scene reduce first.
             const unsigned grp = __match_any_sync(__activemask(), s);
             bits = __reduce_max_sync(grp, bits);
-            if ((int)(threadIdx.x & 31) == __ffs(grp) - 1 && bits) atomicMax(&M.ctl[s].residual_bits, bits);
+            if ((int)(threadIdx.x & 31) == __ffs(grp) - 1 && bits) atomicMax(&M.ctl[s].res[it & 1], bits);
         }
         if (!grid_barrier(M.bar, M.status, M.polls)) return;
-        // solve.rs:93-101 per scene, with each scene's own bounce cap.
-        if (blockIdx.x == 0) {
-            __shared__ uint32_t live;
-            if (threadIdx.x == 0) live = 0;
-            __syncthreads();
-            for (int s = threadIdx.x; s < M.S; s += blockDim.x) {
-                SolveCtl& c = M.ctl[s];
-                if (c.done) continue;
-                const float res = __uint_as_float(c.residual_bits);
-                c.iterations = it + 1;
-                c.last_residual = c.residual_bits;
-                c.residual_bits = 0;
-                if (res < 1e-4f || it + 1 >= sc[s].max_bounces) c.done = 1;
-                else atomicAdd(&live, 1u);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) M.live[0] = live;
-        }
-        if (!grid_barrier(M.bar, M.status, M.polls)) return;
-        if (*(volatile uint32_t*)&M.live[0] == 0) break;
     }
 
     // The grid's irradiance copy.

@@ -1,9 +1,10 @@
 // Direct light on surfels (solve.rs:27-39; for many (surfel, light) slots
 // the light stage uses launch_light_slots in k_shade.cu instead) and the
 // Jacobi bounce solve (solve.rs:47-108). The bounce loop runs without host round trips: every
-// bounce kernel first reads a device-side `done` flag, so the host enqueues
-// max_bounces bounces at once and the ones after convergence return
-// immediately.
+// bounce kernel first reads a device-side control block, so the host enqueues
+// many bounces at once and the ones after convergence return immediately. A
+// bounce is two launches, the cluster means and the rows: the stop test is
+// part of the next bounce's first kernel (SolveCtl).
 #include "kcommon.cuh"
 
 namespace ifx {
@@ -102,91 +103,158 @@ __device__ __forceinline__ void cluster_mean(const float4* rad, const float4* sp
 static constexpr int kAggBlock = 128;
 __global__ void __launch_bounds__(kAggBlock) k_cluster_agg(const float4* rad, const float4* sp, const float4* cp,
                                                             const uint2* crange, const uint32_t* members,
-                                                            uint32_t nc, float4* cluster_rad, const SolveCtl* ctl) {
+                                                            uint32_t nc, float4* cluster_rad, SolveCtl* ctl,
+                                                            uint32_t it, int no_exit) {
     pdl_wait();
-    if (ctl->done) return;
+    const bool stop = solve_stopped(*ctl, it, no_exit);
+    if (blockIdx.x == 0 && threadIdx.x == 0) solve_note(*ctl, it, stop);
+    if (stop) return;
     __shared__ float4 buf[2][kAggBlock];
     for (uint32_t c = blockIdx.x; c < nc; c += gridDim.x)
         cluster_mean<kAggBlock>(rad, sp, cp, crange, members, c, cluster_rad, buf);
     pdl_trigger();
 }
 
-// solve.rs:76-102: one Jacobi row per thread, its links added in CSR order
-// (the reference's sum). Each iteration of the row loop issues the index and
-// weight loads of 8 links as two 128-bit loads each, then the 8 cluster
-// gathers, before the first add, so a thread keeps 12 loads in flight; the
-// products crad[idx] * w and their left-to-right sum round exactly as the
-// scalar loop does. `vec` is 0 when idx or w is not 16-byte aligned (caller-
-// provided arrays), which keeps every load scalar. The bounce residual is the
-// maximum change over rows, an order-free reduction kept as the bits of a
-// non-negative f32 (NaN ignored, as the reference's f32::max fold does).
+// solve.rs:76-102, one row per thread. The bounce residual is the maximum
+// change over rows, an order-free reduction kept as the bits of a non-negative
+// f32 (NaN ignored, as the reference's f32::max fold does).
 static constexpr int kJacBlock = 256;
-__device__ __forceinline__ V jacobi_row(const float4* crad, const uint32_t* __restrict__ idx,
-                                        const float* __restrict__ w, uint32_t k, uint32_t e, int vec) {
-    V irr{0.0f, 0.0f, 0.0f};
-    if (vec) {
-        for (; k < e && (k & 3u); ++k) irr = irr + mk4(__ldg(&crad[__ldg(&idx[k])])) * __ldg(&w[k]);
-        for (; k + 8 <= e; k += 8) {
-            const uint4 i0 = __ldg(reinterpret_cast<const uint4*>(idx + k));
-            const uint4 i1 = __ldg(reinterpret_cast<const uint4*>(idx + k + 4));
-            const float4 w0 = __ldg(reinterpret_cast<const float4*>(w + k));
-            const float4 w1 = __ldg(reinterpret_cast<const float4*>(w + k + 4));
-            const float4 c0 = __ldg(&crad[i0.x]), c1 = __ldg(&crad[i0.y]),
-                         c2 = __ldg(&crad[i0.z]), c3 = __ldg(&crad[i0.w]),
-                         c4 = __ldg(&crad[i1.x]), c5 = __ldg(&crad[i1.y]),
-                         c6 = __ldg(&crad[i1.z]), c7 = __ldg(&crad[i1.w]);
-            irr = irr + mk4(c0) * w0.x;
-            irr = irr + mk4(c1) * w0.y;
-            irr = irr + mk4(c2) * w0.z;
-            irr = irr + mk4(c3) * w0.w;
-            irr = irr + mk4(c4) * w1.x;
-            irr = irr + mk4(c5) * w1.y;
-            irr = irr + mk4(c6) * w1.z;
-            irr = irr + mk4(c7) * w1.w;
-        }
-    }
-    for (; k < e; ++k) irr = irr + mk4(__ldg(&crad[__ldg(&idx[k])])) * __ldg(&w[k]);
-    return irr;
+__device__ __forceinline__ void note_residual(float dmax, SolveCtl* ctl, uint32_t it) {
+    for (int o = 16; o >= 1; o >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(kFull, dmax, o));
+    if ((threadIdx.x & 31) == 0 && dmax > 0.0f) atomicMax(&ctl->res[it & 1], __float_as_uint(dmax));
 }
 
-// The CSR row i of one bounce: irradiance, new radiosity, |change|.
-__device__ __forceinline__ float csr_row_update(float4* direct, float4* albedo, float4* irr_out, float4* rad,
-                                                const uint32_t* starts, const uint32_t* idx, const float* w,
-                                                const float4* cluster_rad, int vec, uint32_t i) {
-    const V irr = jacobi_row(cluster_rad, idx, w, starts[i], starts[i + 1], vec);
-    V nr = mk4(__ldg(&direct[i])) + mk4(__ldg(&albedo[i])) * irr;
-    V diff = vabs(nr - mk4(rad[i]));
+// The end of row i: irradiance, new radiosity, |change|.
+__device__ __forceinline__ float row_update(const float4* direct, const float4* albedo, float4* irr_out, float4* rad,
+                                            uint32_t i, V irr) {
+    const V nr = mk4(__ldg(&direct[i])) + mk4(__ldg(&albedo[i])) * irr;
+    const V diff = vabs(nr - mk4(rad[i]));
     irr_out[i] = f4(irr, 0.0f);
     rad[i] = f4(nr, 0.0f);
-    return fmaxf(diff.x, fmaxf(diff.y, diff.z));
+    const float d = fmaxf(diff.x, fmaxf(diff.y, diff.z));
+    return isnan(d) ? 0.0f : d;
 }
 
-__global__ void __launch_bounds__(kJacBlock) k_jacobi(float4* direct, float4* albedo, float4* irr_out, float4* rad,
-                                                       uint32_t n, const uint32_t* starts, const uint32_t* idx,
-                                                       const float* w, const float4* cluster_rad, SolveCtl* ctl,
-                                                       int vec) {
+__global__ void __launch_bounds__(kJacBlock) k_jacobi(const float4* direct, const float4* albedo, float4* irr_out,
+                                                       float4* rad, uint32_t n, const uint32_t* starts,
+                                                       const uint32_t* idx, const float* w, const float4* crad,
+                                                       SolveCtl* ctl, uint32_t it, int vec) {
     pdl_wait();
     if (ctl->done) return;
     float dmax = 0.0f;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float d = csr_row_update(direct, albedo, irr_out, rad, starts, idx, w, cluster_rad, vec, i);
-        if (!isnan(d)) dmax = fmaxf(dmax, d);
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        dmax = fmaxf(dmax, row_update(direct, albedo, irr_out, rad, i,
+                                      jacobi_row(crad, idx, w, starts[i], starts[i + 1], vec)));
     pdl_trigger();
-    for (int o = 16; o >= 1; o >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(kFull, dmax, o));
-    if ((threadIdx.x & 31) == 0 && dmax > 0.0f) atomicMax(&ctl->residual_bits, __float_as_uint(dmax));
+    note_residual(dmax, ctl, it);
 }
 
-// solve.rs:454-462; no_exit keeps every bounce running (fixed bounce count).
-__global__ void k_bounce_end(SolveCtl* ctl, uint32_t it, int no_exit) {
+// The same for many rows, whose CSR arrays stream from memory. A thread's own
+// loads of its row touch a cache line each, and so do its gathers: 1.5 L1
+// cycles a link, twice the time the arrays take to arrive. Here a warp fetches
+// the next 32 links of each of its 32 rows together, one coalesced copy per
+// row and array straight into shared memory (double-buffered, rows padded to
+// 33 words so that the lanes read their own rows without conflicts), and the
+// cluster radiosities are gathered from a copy in shared memory where they
+// fit (kShared). Each lane still adds its row's links in order.
+static constexpr int kTileWarps = 8;
+static constexpr uint32_t kTileWords = 32u * 33u;  // one array of one tile
+static constexpr size_t kTileBytes = (size_t)kTileWarps * 2u * 2u * kTileWords * 4u;
+static constexpr uint32_t kTileMinRows = 65536;
+// Cluster radiosities gathered from shared memory: up to 4,096 clusters.
+static constexpr size_t kSharedRadMax = 64u * 1024u;
+
+__device__ __forceinline__ void copy4_async(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+template <bool kShared>
+__global__ void __launch_bounds__(kTileWarps * 32) k_jacobi_tiles(const float4* direct, const float4* albedo,
+                                                                  float4* irr_out, float4* rad, uint32_t n,
+                                                                  const uint32_t* starts, const uint32_t* idx,
+                                                                  const float* w, const float4* crad, uint32_t nc,
+                                                                  SolveCtl* ctl, uint32_t it) {
+    extern __shared__ __align__(16) uint8_t tile_smem[];
     pdl_wait();
-    pdl_trigger();
     if (ctl->done) return;
-    float res = __uint_as_float(ctl->residual_bits);
-    ctl->iterations = it + 1;
-    ctl->last_residual = ctl->residual_bits;
-    ctl->residual_bits = 0;
-    if (res < 1e-4f && !no_exit) ctl->done = 1;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    float4* cs = reinterpret_cast<float4*>(tile_smem + kTileBytes);
+    if constexpr (kShared) {
+        for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x) cs[c] = crad[c];
+        __syncthreads();
+    }
+    uint32_t* tiles = reinterpret_cast<uint32_t*>(tile_smem) + (size_t)warp * 4u * kTileWords;
+    const uint32_t tiles_at = (uint32_t)__cvta_generic_to_shared(tiles);
+    const uint32_t groups = (n + 31u) / 32u, stride = gridDim.x * kTileWarps;
+    // Links [32 t, 32 t + 32) of the group's rows into stage st.
+    auto fetch = [&](uint32_t s, uint32_t len, uint32_t t, uint32_t st) {
+        const uint32_t at = tiles_at + (st * 2u * kTileWords + lane) * 4u, j = 32u * t + lane;
+#pragma unroll 8
+        for (uint32_t r = 0; r < 32u; ++r) {
+            const uint32_t sr = __shfl_sync(kFull, s, r), lr = __shfl_sync(kFull, len, r);
+            if (j < lr) {
+                copy4_async(at + r * 132u, idx + (size_t)sr + j);
+                copy4_async(at + r * 132u + kTileWords * 4u, w + (size_t)sr + j);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto row_of = [&](uint32_t g, uint32_t& s, uint32_t& len) {
+        const uint32_t row = g * 32u + lane;
+        s = len = 0;
+        if (g < groups && row < n) {
+            s = starts[row];
+            len = starts[row + 1] - s;
+        }
+    };
+    uint32_t g = blockIdx.x * kTileWarps + warp, s, len, st = 0;
+    float dmax = 0.0f;
+    row_of(g, s, len);
+    if (g < groups) fetch(s, len, 0, 0);
+    for (; g < groups; g += stride) {
+        uint32_t s2, len2;
+        row_of(g + stride, s2, len2);
+        const uint32_t most = __reduce_max_sync(kFull, len), turns = most > 32u ? (most + 31u) / 32u : 1u;
+        V irr{0.0f, 0.0f, 0.0f};
+        for (uint32_t t = 0; t < turns; ++t, st ^= 1u) {
+            // The next tile of this group, or the first of the next.
+            if (t + 1u < turns) fetch(s, len, t + 1u, st ^ 1u);
+            else fetch(s2, len2, 0, st ^ 1u);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            const uint32_t* ti = tiles + st * 2u * kTileWords + lane * 33u;
+            const float* tw = reinterpret_cast<const float*>(ti + kTileWords);
+            const uint32_t cnt = len > 32u * t ? min(len - 32u * t, 32u) : 0u;
+            uint32_t j = 0;
+            for (; j + 4u <= cnt; j += 4u) {
+                float4 c[4];
+                float v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    v[k] = tw[j + k];
+                    c[k] = kShared ? cs[ti[j + k]] : crad[ti[j + k]];
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) irr = irr + mk4(c[k]) * v[k];
+            }
+            for (; j < cnt; ++j) irr = irr + mk4(kShared ? cs[ti[j]] : crad[ti[j]]) * tw[j];
+            __syncwarp();
+        }
+        const uint32_t row = g * 32u + lane;
+        if (row < n) dmax = fmaxf(dmax, row_update(direct, albedo, irr_out, rad, row, irr));
+        s = s2;
+        len = len2;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    pdl_trigger();
+    note_residual(dmax, ctl, it);
+}
+
+// solve.rs:93-101 after the last bounce that was launched.
+__global__ void k_solve_end(SolveCtl* ctl, uint32_t it) {
+    pdl_wait();
+    const bool stop = solve_stopped(*ctl, it, 0);
+    solve_note(*ctl, it, stop);
 }
 
 void launch_light_surfels(cudaStream_t st, BlobRef blob, SurfelArrays s, uint32_t n, unsigned long long* evals,
@@ -205,80 +273,88 @@ void launch_light_surfels(cudaStream_t st, BlobRef blob, SurfelArrays s, uint32_
 // from the interleaved layout (a warp's loads are one contiguous 512-byte
 // block) and added in CSR order, exactly as k_jacobi; a lane stops at its own
 // row's length, so padding is never read. Outputs go to the original row.
-__device__ __forceinline__ float sell_row_update(float4* direct, float4* albedo, float4* irr_out, float4* rad,
-                                                 const SellMatrix& m, const float4* crad, uint32_t sp) {
-    const uint32_t row = m.perm[sp], len = m.len[sp];
-    const uint32_t* ip = m.idx + m.slice_off[sp >> 5] + (sp & 31u) * 4u;
-    const float* wp = m.w + m.slice_off[sp >> 5] + (sp & 31u) * 4u;
+// The next 8 links' indices and weights are loaded while the current ones are
+// gathered and added: with few rows the kernel is one such chain per row.
+__device__ __forceinline__ V sell_row(const SellMatrix& m, const float4* crad, uint32_t sp, uint32_t len) {
+    const uint4* ip = reinterpret_cast<const uint4*>(m.idx + m.slice_off[sp >> 5] + (sp & 31u) * 4u);
+    const float4* wp = reinterpret_cast<const float4*>(m.w + m.slice_off[sp >> 5] + (sp & 31u) * 4u);
     V irr{0.0f, 0.0f, 0.0f};
-    uint32_t j = 0;
-    for (; j + 8 <= len; j += 8, ip += 256, wp += 256) {
-        const uint4 i0 = __ldg(reinterpret_cast<const uint4*>(ip));
-        const uint4 i1 = __ldg(reinterpret_cast<const uint4*>(ip + 128));
-        const float4 w0 = __ldg(reinterpret_cast<const float4*>(wp));
-        const float4 w1 = __ldg(reinterpret_cast<const float4*>(wp + 128));
-        const float4 c0 = __ldg(&crad[i0.x]), c1 = __ldg(&crad[i0.y]),
-                     c2 = __ldg(&crad[i0.z]), c3 = __ldg(&crad[i0.w]),
-                     c4 = __ldg(&crad[i1.x]), c5 = __ldg(&crad[i1.y]),
-                     c6 = __ldg(&crad[i1.z]), c7 = __ldg(&crad[i1.w]);
-        irr = irr + mk4(c0) * w0.x;
-        irr = irr + mk4(c1) * w0.y;
-        irr = irr + mk4(c2) * w0.z;
-        irr = irr + mk4(c3) * w0.w;
-        irr = irr + mk4(c4) * w1.x;
-        irr = irr + mk4(c5) * w1.y;
-        irr = irr + mk4(c6) * w1.z;
-        irr = irr + mk4(c7) * w1.w;
-    }
-    if (j < len) {
-        const uint4 i0 = __ldg(reinterpret_cast<const uint4*>(ip));
-        const float4 w0 = __ldg(reinterpret_cast<const float4*>(wp));
-        const uint32_t ia[4] = {i0.x, i0.y, i0.z, i0.w};
-        const float wa[4] = {w0.x, w0.y, w0.z, w0.w};
-        const uint32_t r4 = len - j < 4u ? len - j : 4u;
-        for (uint32_t t = 0; t < r4; ++t) irr = irr + mk4(__ldg(&crad[ia[t]])) * wa[t];
-        j += r4;
-        if (j < len) {
-            ip += 128;
-            wp += 128;
-            const uint4 i1 = __ldg(reinterpret_cast<const uint4*>(ip));
-            const float4 w1 = __ldg(reinterpret_cast<const float4*>(wp));
-            const uint32_t ib[4] = {i1.x, i1.y, i1.z, i1.w};
-            const float wb[4] = {w1.x, w1.y, w1.z, w1.w};
-            for (uint32_t t = 0; t < len - j; ++t) irr = irr + mk4(__ldg(&crad[ib[t]])) * wb[t];
+    if (len == 0) return irr;
+    // Entries [0, 4 * ceil(len / 4)) of the row exist (padding included).
+    uint4 i0 = __ldg(ip), i1 = len > 4u ? __ldg(ip + 32) : i0;
+    float4 w0 = __ldg(wp), w1 = len > 4u ? __ldg(wp + 32) : w0;
+    for (uint32_t j = 0;; j += 8) {
+        const uint32_t left = len - j;
+        const uint4 a0 = i0, a1 = i1;
+        const float4 b0 = w0, b1 = w1;
+        ip += 64;
+        wp += 64;
+        if (left > 8u) {
+            i0 = __ldg(ip);
+            w0 = __ldg(wp);
+        }
+        if (left > 12u) {
+            i1 = __ldg(ip + 32);
+            w1 = __ldg(wp + 32);
+        }
+        if (left >= 8u) {
+            const float4 c0 = crad[a0.x], c1 = crad[a0.y], c2 = crad[a0.z], c3 = crad[a0.w], c4 = crad[a1.x],
+                         c5 = crad[a1.y], c6 = crad[a1.z], c7 = crad[a1.w];
+            irr = irr + mk4(c0) * b0.x;
+            irr = irr + mk4(c1) * b0.y;
+            irr = irr + mk4(c2) * b0.z;
+            irr = irr + mk4(c3) * b0.w;
+            irr = irr + mk4(c4) * b1.x;
+            irr = irr + mk4(c5) * b1.y;
+            irr = irr + mk4(c6) * b1.z;
+            irr = irr + mk4(c7) * b1.w;
+            if (left == 8u) return irr;
+        } else {
+            const uint32_t ia[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const float wa[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+            for (uint32_t t = 0; t < 7u; ++t)
+                if (t < left) irr = irr + mk4(crad[ia[t]]) * wa[t];
+            return irr;
         }
     }
-    V nr = mk4(__ldg(&direct[row])) + mk4(__ldg(&albedo[row])) * irr;
-    V diff = vabs(nr - mk4(rad[row]));
-    irr_out[row] = f4(irr, 0.0f);
-    rad[row] = f4(nr, 0.0f);
-    return fmaxf(diff.x, fmaxf(diff.y, diff.z));
 }
 
-__global__ void __launch_bounds__(kJacBlock) k_jacobi_sell(float4* direct, float4* albedo, float4* irr_out,
-                                                            float4* rad, uint32_t n, SellMatrix m,
-                                                            const float4* __restrict__ crad, SolveCtl* ctl) {
+// kShared: many rows gather the cluster radiosities from shared memory, where
+// a warp's 32 scattered 16-byte reads take some 10 cycles, a third of what
+// they take in L1 (a cache line each).
+template <bool kShared>
+__global__ void __launch_bounds__(kJacBlock) k_jacobi_sell(const float4* direct, const float4* albedo,
+                                                            float4* irr_out, float4* rad, uint32_t n, SellMatrix m,
+                                                            const float4* __restrict__ crad, uint32_t nc,
+                                                            SolveCtl* ctl, uint32_t it) {
+    extern __shared__ __align__(16) uint8_t sell_smem[];
     pdl_wait();
     if (ctl->done) return;
+    float4* cs = reinterpret_cast<float4*>(sell_smem);
+    if constexpr (kShared) {
+        for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x) cs[c] = crad[c];
+        __syncthreads();
+    }
     float dmax = 0.0f;
     for (uint32_t sp = blockIdx.x * blockDim.x + threadIdx.x; sp < n; sp += gridDim.x * blockDim.x) {
-        const float d = sell_row_update(direct, albedo, irr_out, rad, m, crad, sp);
-        if (!isnan(d)) dmax = fmaxf(dmax, d);
+        const uint32_t row = m.perm[sp];
+        const V irr = kShared ? sell_row(m, cs, sp, m.len[sp]) : sell_row(m, crad, sp, m.len[sp]);
+        dmax = fmaxf(dmax, row_update(direct, albedo, irr_out, rad, row, irr));
     }
     pdl_trigger();
-    for (int o = 16; o >= 1; o >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(kFull, dmax, o));
-    if ((threadIdx.x & 31) == 0 && dmax > 0.0f) atomicMax(&ctl->residual_bits, __float_as_uint(dmax));
+    note_residual(dmax, ctl, it);
 }
 
 // A bounce kernel launched with the programmatic-serialization attribute:
 // the stream (or the captured graph's edge) lets it start once the previous
 // kernel has triggered, and pdl_wait orders its work after that kernel.
 template <typename... K, typename... A>
-static void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+static void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -288,22 +364,48 @@ static void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, cuda
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// One wave of CTAs, as many as are co-resident.
+template <class K>
+static unsigned wave_grid(K kernel, int block, size_t smem, unsigned long long items) {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
+    return grid_for(items, block, per_sm < 1 ? 1 : per_sm);
+}
+
 void launch_solve_bounce(cudaStream_t st, SurfelArrays s, uint32_t n, const float4* cp, const uint2* crange,
                          const uint32_t* members, uint32_t nc, const uint32_t* starts, const uint32_t* idx,
                          const float* w, float4* cluster_rad, SolveCtl* ctl, uint32_t it, int* launches,
                          int no_exit, const SellMatrix* sell) {
-    launch_pdl(k_cluster_agg, nc < 4096u ? nc : 4096u, kAggBlock, st, (const float4*)s.rad, (const float4*)s.p, cp,
-               crange, members, nc, cluster_rad, (const SolveCtl*)ctl);
+    launch_pdl(k_cluster_agg, nc < 4096u ? nc : 4096u, kAggBlock, 0, st, (const float4*)s.rad, (const float4*)s.p, cp,
+               crange, members, nc, cluster_rad, ctl, it, no_exit);
+    const float4 *direct = s.direct, *albedo = s.albedo, *crad = cluster_rad;
+    const size_t cbytes = (size_t)nc * 16u;
     if (sell && sell->perm) {
-        launch_pdl(k_jacobi_sell, grid_for(n, kJacBlock), kJacBlock, st, s.direct, s.albedo, s.irr, s.rad, n, *sell,
-                   (const float4*)cluster_rad, ctl);
+        if (n >= kTileMinRows && cbytes <= kSharedRadMax)
+            launch_pdl(k_jacobi_sell<true>, wave_grid(k_jacobi_sell<true>, kJacBlock, cbytes, n), kJacBlock, cbytes, st,
+                       direct, albedo, s.irr, s.rad, n, *sell, crad, nc, ctl, it);
+        else
+            launch_pdl(k_jacobi_sell<false>, grid_for(n, kJacBlock), kJacBlock, 0, st, direct, albedo, s.irr, s.rad, n,
+                       *sell, crad, nc, ctl, it);
+    } else if (n >= kTileMinRows) {
+        const unsigned block = kTileWarps * 32u;
+        if (cbytes <= kSharedRadMax)
+            launch_pdl(k_jacobi_tiles<true>, wave_grid(k_jacobi_tiles<true>, block, kTileBytes + cbytes, n), block,
+                       kTileBytes + cbytes, st, direct, albedo, s.irr, s.rad, n, starts, idx, w, crad, nc, ctl, it);
+        else
+            launch_pdl(k_jacobi_tiles<false>, wave_grid(k_jacobi_tiles<false>, block, kTileBytes, n), block, kTileBytes,
+                       st, direct, albedo, s.irr, s.rad, n, starts, idx, w, crad, nc, ctl, it);
     } else {
         const int vec = (((uintptr_t)idx | (uintptr_t)w) & 15u) == 0 ? 1 : 0;
-        launch_pdl(k_jacobi, grid_for(n, kJacBlock), kJacBlock, st, s.direct, s.albedo, s.irr, s.rad, n, starts, idx,
-                   w, (const float4*)cluster_rad, ctl, vec);
+        launch_pdl(k_jacobi, grid_for(n, kJacBlock), kJacBlock, 0, st, direct, albedo, s.irr, s.rad, n, starts, idx, w,
+                   crad, ctl, it, vec);
     }
-    launch_pdl(k_bounce_end, 1u, 1u, st, ctl, it, no_exit);
-    *launches += 3;
+    *launches += 2;
+}
+
+void launch_solve_end(cudaStream_t st, SolveCtl* ctl, uint32_t it, int* launches) {
+    launch_pdl(k_solve_end, 1u, 1u, 0, st, ctl, it);
+    *launches += 1;
 }
 
 // ------------------------------------------------- sliced-ELL assembly ---
@@ -351,10 +453,19 @@ int launch_sell_fill(cudaStream_t st, const uint32_t* starts, const uint32_t* id
     return 1;
 }
 
+// Their own limits, which need no context (ifx_solve_noalloc has none).
+void configure_bounce_kernels() {
+    cudaFuncSetAttribute(k_jacobi_sell<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedRadMax);
+    cudaFuncSetAttribute(k_jacobi_tiles<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(kTileBytes + kSharedRadMax));
+    cudaFuncSetAttribute(k_jacobi_tiles<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileBytes);
+}
+
 void configure_solve_kernels(int max_dyn_smem) {
     cudaFuncSetAttribute(k_light_surfels<NoCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
     cudaFuncSetAttribute(k_light_surfels<NoCount3>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
     cudaFuncSetAttribute(k_light_surfels<Counts>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+    configure_bounce_kernels();
 }
 
 }  // namespace ifx

@@ -188,4 +188,56 @@ struct WarpQueue {
     __device__ __forceinline__ bool empty() const { return drained && cur >= end; }
 };
 
+// ------------------------------------------------------ Jacobi bounces ----
+// solve.rs:93-101: whether the solve has stopped before bounce `it`. Every
+// thread of a bounce's first phase decides the same, whether or not it sees
+// solve_note's writes.
+__device__ __forceinline__ bool solve_stopped(const SolveCtl& c, uint32_t it, int no_exit) {
+    const volatile SolveCtl& v = c;
+    return v.done || (!no_exit && it > 0 && __uint_as_float(v.res[(it - 1) & 1]) < 1e-4f);
+}
+// One thread's part before bounce `it`: the statistics of the bounces so far.
+__device__ __forceinline__ void solve_note(SolveCtl& c, uint32_t it, bool stop) {
+    if (c.done) return;
+    if (it > 0) {
+        c.iterations = it;
+        c.last_residual = c.res[(it - 1) & 1];
+    }
+    if (stop) c.done = 1;
+    else c.res[it & 1] = 0;
+}
+
+// solve.rs:76-102: the sum of a row's links [k, e) in CSR order (the
+// reference's sum). Each turn issues the index and weight loads of 8 links as
+// two 128-bit loads each, then the 8 cluster gathers, before the first add, so
+// a thread keeps 12 loads in flight; the products crad[idx] * w and their
+// left-to-right sum round exactly as the scalar loop does. `vec` is 0 when
+// idx or w is not 16-byte aligned (caller-provided arrays), which keeps every
+// load scalar.
+__device__ __forceinline__ V jacobi_row(const float4* crad, const uint32_t* __restrict__ idx,
+                                        const float* __restrict__ w, uint32_t k, uint32_t e, int vec) {
+    V irr{0.0f, 0.0f, 0.0f};
+    if (vec) {
+        for (; k < e && (k & 3u); ++k) irr = irr + mk4(crad[__ldg(&idx[k])]) * __ldg(&w[k]);
+        for (; k + 8 <= e; k += 8) {
+            const uint4 i0 = __ldg(reinterpret_cast<const uint4*>(idx + k));
+            const uint4 i1 = __ldg(reinterpret_cast<const uint4*>(idx + k + 4));
+            const float4 w0 = __ldg(reinterpret_cast<const float4*>(w + k));
+            const float4 w1 = __ldg(reinterpret_cast<const float4*>(w + k + 4));
+            const float4 c0 = crad[i0.x], c1 = crad[i0.y], c2 = crad[i0.z], c3 = crad[i0.w], c4 = crad[i1.x],
+                         c5 = crad[i1.y], c6 = crad[i1.z], c7 = crad[i1.w];
+            irr = irr + mk4(c0) * w0.x;
+            irr = irr + mk4(c1) * w0.y;
+            irr = irr + mk4(c2) * w0.z;
+            irr = irr + mk4(c3) * w0.w;
+            irr = irr + mk4(c4) * w1.x;
+            irr = irr + mk4(c5) * w1.y;
+            irr = irr + mk4(c6) * w1.z;
+            irr = irr + mk4(c7) * w1.w;
+        }
+    }
+    for (; k < e; ++k) irr = irr + mk4(crad[__ldg(&idx[k])]) * __ldg(&w[k]);
+    return irr;
+}
+
 }  // namespace ifx

@@ -160,7 +160,10 @@ void launch_sum_u64(cudaStream_t st, const unsigned long long* v, uint32_t n, un
 struct SolveCtl {
     uint32_t done;
     uint32_t iterations;
-    uint32_t residual_bits;  // max |delta| of the bounce in progress (non-negative f32 bits)
+    // max |delta| of bounce it in res[it & 1] (non-negative f32 bits): a
+    // bounce's first kernel reads the one before's while it clears its own, so
+    // that the stop test needs no launch (or grid barrier) of its own.
+    uint32_t res[2];
     uint32_t last_residual;  // residual of the last completed bounce
 };
 // solve.rs:27-39 with one thread per surfel walking its lights (k_solve.cu);
@@ -207,6 +210,8 @@ void launch_solve_bounce(cudaStream_t st, SurfelArrays s, uint32_t n, const floa
                          const uint32_t* members, uint32_t nc, const uint32_t* starts, const uint32_t* idx,
                          const float* w, float4* cluster_rad, SolveCtl* ctl, uint32_t it, int* launches,
                          int no_exit = 0, const SellMatrix* sell = nullptr);
+// After the last of `it` bounces: the stop test and the statistics in *ctl.
+void launch_solve_end(cudaStream_t st, SolveCtl* ctl, uint32_t it, int* launches);
 // Sliced-ELL construction: row link counts (keys) with the identity (vals);
 // after a stable descending sort of (keys, vals), the slice sizes, then the
 // interleaved copy of idx and w.
@@ -360,7 +365,6 @@ struct MsParams {
     uint32_t total_surf, total_clus, total_pix;
     uint32_t max_bounces;  // largest per-scene cap
     SolveCtl* ctl;         // S
-    uint32_t* live;        // scenes still bouncing
     MsBarrier* bar;
     uint32_t* status;
     const float* srgb_t;
@@ -376,6 +380,7 @@ int multi_frame_max_blocks(int block);
 void configure_surfel_kernels(int max_dyn_smem);
 void configure_transfer_kernels(int max_dyn_smem);
 void configure_solve_kernels(int max_dyn_smem);
+void configure_bounce_kernels();
 void configure_shade_kernels(int max_dyn_smem);
 void configure_diff_kernels(int max_dyn_smem);
 void configure_path_kernels(int max_dyn_smem);
