@@ -165,6 +165,7 @@ struct ifx_ctx {
     DBuf cub_tmp, small;  // small: 8 x u64 counters / results
     DBuf gen_cand, gen_keep, gen_off, gen_head, gen_pts, gen_next, gen_state, gen_out;  // surfel generation
     DBuf gen_head_acc, gen_next_acc, gen_rank, gen_st;
+    DBuf dlpack;  // the surfel download's packed arrays
 
     // measurement: per-kernel events, work counters (IFX_NUM_KERNELS x 21 u64), timer
     cudaEvent_t kv0 = nullptr, kv1 = nullptr, kc0 = nullptr, kc1 = nullptr, tm0 = nullptr, tm1 = nullptr;
@@ -477,7 +478,7 @@ extern "C" void ifx_ctx_destroy(ifx_ctx* ctx) {
                     &ctx->path_sincos, &ctx->shsc, &ctx->lff, &ctx->lvis, &ctx->lq, &ctx->lsc,
                     &ctx->vkey, &ctx->vkey_alt, &ctx->vval, &ctx->vval_alt, &ctx->ckey, &ctx->ckey_alt,
                     &ctx->cval, &ctx->cval_alt, &ctx->msum, &ctx->gen_head_acc, &ctx->gen_next_acc, &ctx->gen_rank, &ctx->gen_st,
-                    &ctx->og_cells};
+                    &ctx->og_cells, &ctx->dlpack};
     for (DBuf* b : bufs) free_buf(*b);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     for (cudaEvent_t ev : {ctx->ev0, ctx->ev1, ctx->kv0, ctx->kv1, ctx->kc0, ctx->kc1, ctx->tm0, ctx->tm1})
@@ -761,33 +762,30 @@ extern "C" int ifx_surfels_count(const ifx_ctx* ctx, uint64_t* n) {
     return IFX_OK;
 }
 
-static int download3(ifx_ctx* ctx, const DBuf& src, float* dst, bool w_only = false) {
-    if (!dst || ctx->n == 0) return IFX_OK;
-    std::vector<float4> h(ctx->n);
-    CK(cudaMemcpyAsync(h.data(), src.p, ctx->n * sizeof(float4), cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    for (uint32_t i = 0; i < ctx->n; ++i) {
-        if (w_only) {
-            dst[i] = h[i].w;
-        } else {
-            dst[3 * i] = h[i].x;
-            dst[3 * i + 1] = h[i].y;
-            dst[3 * i + 2] = h[i].z;
-        }
-    }
-    return IFX_OK;
-}
-
 extern "C" int ifx_surfels_download(ifx_ctx* ctx, float* p, float* nrm, float* albedo, float* area, float* direct,
                                     float* irr, float* rad) {
     if (!ctx) return IFX_ERR_INVALID;
     CK(cudaSetDevice(ctx->device));
-    int r;
-    if ((r = download3(ctx, ctx->sp, p)) || (r = download3(ctx, ctx->sn, nrm)) ||
-        (r = download3(ctx, ctx->salb, albedo)) || (r = download3(ctx, ctx->sp, area, true)) ||
-        (r = download3(ctx, ctx->sdir, direct)) || (r = download3(ctx, ctx->sirr, irr)) ||
-        (r = download3(ctx, ctx->srad, rad)))
-        return r;
+    const size_t n = ctx->n;
+    if (n == 0) return IFX_OK;
+    // The arrays are packed to the caller's layout on the device: the host
+    // unpacked 16-byte records by loops, 2.0 ms of 55,000 surfels' download.
+    ENSURE(ctx->dlpack, n * 19 * 4);
+    float* at = (float*)ctx->dlpack.p;
+    const std::pair<const DBuf*, float*> fields[] = {{&ctx->sp, p},     {&ctx->sn, nrm},  {&ctx->salb, albedo},
+                                                     {&ctx->sdir, direct}, {&ctx->sirr, irr}, {&ctx->srad, rad}};
+    for (const auto& f : fields) {
+        if (!f.second) continue;
+        ctx->launches += (uint64_t)launch_unpack3(ctx->st, (const float4*)f.first->p, (uint32_t)n, at);
+        CK(cudaMemcpyAsync(f.second, at, n * 12, cudaMemcpyDeviceToHost, ctx->st));
+        at += n * 3;
+    }
+    if (area) {
+        ctx->launches += (uint64_t)launch_unpack_w(ctx->st, (const float4*)ctx->sp.p, (uint32_t)n, at);
+        CK(cudaMemcpyAsync(area, at, n * 4, cudaMemcpyDeviceToHost, ctx->st));
+    }
+    CKL();
+    CK(cudaStreamSynchronize(ctx->st));
     return IFX_OK;
 }
 
@@ -998,13 +996,18 @@ static int build_clusters(ifx_ctx* ctx, int res) {
 
 // The transfer's sliced-ELL copy for the solve (kernels.h SellMatrix): rows
 // sorted by link count (stable, descending), 32-row slices, links
-// interleaved by 4 per lane. Left out (the solve reads the CSR arrays) when
-// its padded size could pass 2^32 entries.
-static int sell_build(ifx_ctx* ctx) {
+// interleaved by 4 per lane. Its padded size is bounded without a look at the
+// lengths: a slice is no longer than 32 times its first row, which no row of
+// the slice before it is shorter than, so the slices after the first hold at
+// most the links and the rounding up to 4. Left out (the solve reads the CSR
+// arrays) when that could pass 2^32 entries.
+static int sell_build(ifx_ctx* ctx, uint64_t longest) {
     ctx->sell_ready = false;
     const uint32_t n = ctx->n;
     if (n == 0 || ctx->links == 0) return IFX_OK;
     const uint32_t ns = (n + 31) / 32;
+    const uint64_t bound = 32ull * ((uint64_t)longest + 3ull) + ctx->links + 3ull * ns * 32ull;
+    if (bound >= 0xffffffffull) return IFX_OK;
     ENSURE(ctx->sell_len, (size_t)n * 4);
     ENSURE(ctx->sell_perm, (size_t)n * 4);
     ENSURE(ctx->sell_keys, (size_t)n * 4);
@@ -1020,20 +1023,13 @@ static int sell_build(ifx_ctx* ctx) {
     CUB([&](void* t, size_t& b) {
         return cub::DeviceRadixSort::SortPairsDescending(t, b, keys, len, rows, perm, (int)n, 0, 32, ctx->st);
     });
-    uint32_t maxlen = 0;
-    CK(cudaMemcpyAsync(&maxlen, len, 4, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    if ((uint64_t)ns * 32ull * (((uint64_t)maxlen + 3ull) & ~3ull) >= 0xffffffffull) return IFX_OK;
     uint32_t* sizes = (uint32_t*)ctx->sell_sizes.p;
     uint32_t* off = (uint32_t*)ctx->sell_off.p;
     ctx->launches += (uint64_t)launch_sell_sizes(ctx->st, len, n, sizes);
     CKL();
     CUB([&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveSum(t, b, sizes, off, (int)ns + 1, ctx->st); });
-    uint32_t total = 0;
-    CK(cudaMemcpyAsync(&total, off + ns, 4, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    ENSURE(ctx->sell_idx, (size_t)total * 4);
-    ENSURE(ctx->sell_w, (size_t)total * 4);
+    ENSURE(ctx->sell_idx, (size_t)bound * 4);
+    ENSURE(ctx->sell_w, (size_t)bound * 4);
     ctx->launches += (uint64_t)launch_sell_fill(ctx->st, (const uint32_t*)ctx->starts.p, (const uint32_t*)ctx->idx.p,
                                                 (const float*)ctx->w.p, n, perm, len, off,
                                                 (uint32_t*)ctx->sell_idx.p, (float*)ctx->sell_w.p);
@@ -1144,21 +1140,29 @@ static int transfer_build(ifx_ctx* ctx, int cluster_res, ifx_transfer_info* out,
     CK(cudaEventRecord(ctx->tev[1], ctx->st3));
     const uint32_t* vorder = nullptr;
     if (ncand > 1 && ncand <= 0x7fffffffull) {
-        ENSURE(ctx->vkey, ncand * 8);
-        ENSURE(ctx->vkey_alt, ncand * 8);
+        // 32-bit keys where they hold (nc + 1)^2: every scene of up to 65,534
+        // clusters. (64-bit keys moved 1.5 times the bytes.)
+        const unsigned long long kmax = (unsigned long long)nc * (nc + 1ull) + nc;
+        const bool narrow = kmax <= 0xffffffffull;
+        ENSURE(ctx->vkey, ncand * (narrow ? 4 : 8));
+        ENSURE(ctx->vkey_alt, ncand * (narrow ? 4 : 8));
         ENSURE(ctx->vval, ncand * 4);
         ENSURE(ctx->vval_alt, ncand * 4);
-        unsigned long long *kin = (unsigned long long*)ctx->vkey.p, *kout = (unsigned long long*)ctx->vkey_alt.p;
         uint32_t *vin = (uint32_t*)ctx->vval.p, *vout = (uint32_t*)ctx->vval_alt.p;
-        ctx->launches += (uint64_t)launch_vis_keys(ctx->st, ncand, (const uint32_t*)ctx->cand_c.p,
-                                                   (const uint32_t*)ctx->cand_row.p, (const uint32_t*)ctx->cid.p,
-                                                   nc, kin, vin);
-        const unsigned long long kmax = (unsigned long long)nc * (nc + 1ull) + nc;
         int end_bit = 1;
         while (end_bit < 64 && (kmax >> end_bit) != 0) ++end_bit;
-        CUB([&](void* t, size_t& b) {
-            return cub::DeviceRadixSort::SortPairs(t, b, kin, kout, vin, vout, (int)ncand, 0, end_bit, ctx->st);
-        });
+        auto sort = [&](auto* kin, auto* kout) -> int {
+            ctx->launches += (uint64_t)launch_vis_keys(ctx->st, ncand, (const uint32_t*)ctx->cand_c.p,
+                                                       (const uint32_t*)ctx->cand_row.p, (const uint32_t*)ctx->cid.p,
+                                                       nc, kin, vin);
+            CUB([&](void* t, size_t& b) {
+                return cub::DeviceRadixSort::SortPairs(t, b, kin, kout, vin, vout, (int)ncand, 0, end_bit, ctx->st);
+            });
+            return IFX_OK;
+        };
+        if ((r = narrow ? sort((uint32_t*)ctx->vkey.p, (uint32_t*)ctx->vkey_alt.p)
+                        : sort((unsigned long long*)ctx->vkey.p, (unsigned long long*)ctx->vkey_alt.p)))
+            return r;
         vorder = vout;
     }
     // Visibility (a persistent kernel).
@@ -1219,7 +1223,7 @@ static int transfer_build(ifx_ctx* ctx, int cluster_res, ifx_transfer_info* out,
                           (const uint2*)ctx->crange.p, (const uint32_t*)ctx->members.p, status);
     ctx->launches++;
 #endif
-    if ((r = sell_build(ctx))) {
+    if ((r = sell_build(ctx, nc))) {  // a row links each cluster once at most
         cudaStreamSynchronize(ctx->st3);
         ctx->mean_pending = false;
         return r;
@@ -1362,7 +1366,9 @@ extern "C" int ifx_transfer_upload(ifx_ctx* ctx, const uint32_t* starts, uint64_
     }
     CK(cudaStreamSynchronize(ctx->st));
     ctx->links = links;
-    int r = sell_build(ctx);
+    uint32_t longest = 0;
+    for (uint32_t i = 0; i < ctx->n; ++i) longest = std::max(longest, starts[i + 1] - starts[i]);
+    int r = sell_build(ctx, longest);
     if (r) return r;
     ctx->has_transfer = true;
     frame_changed(ctx);

@@ -419,6 +419,10 @@ __global__ void k_unpack3(const float4* in, uint32_t n, float* out) {
     }
 }
 
+__global__ void k_unpack_w(const float4* in, uint32_t n, float* out) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = in[i].w;
+}
+
 // ---------------------------------------------------------- launchers ----
 int launch_relight(cudaStream_t st, const float4* albedo, const float* terms, const float4* emit, int nl,
                    uint32_t n, float4* direct, float4* rad, float4* irr) {
@@ -507,6 +511,11 @@ int launch_emit_grad(cudaStream_t st, const float4* dpix, const float* gimg, uin
 
 int launch_unpack3(cudaStream_t st, const float4* in, uint32_t n, float* out) {
     k_unpack3<<<grid_for(n, 256), 256, 0, st>>>(in, n, out);
+    return 1;
+}
+
+int launch_unpack_w(cudaStream_t st, const float4* in, uint32_t n, float* out) {
+    k_unpack_w<<<grid_for(n, 256), 256, 0, st>>>(in, n, out);
     return 1;
 }
 

@@ -424,16 +424,46 @@ __global__ void k_sell_sizes(const uint32_t* sorted_len, uint32_t n, uint32_t* s
         sizes[k] = k < ns ? 32u * ((sorted_len[32 * k] + 3u) & ~3u) : 0u;
 }
 
-__global__ void k_sell_fill(const uint32_t* starts, const uint32_t* idx, const float* w, uint32_t n,
-                            const uint32_t* perm, const uint32_t* sorted_len, const uint32_t* slice_off,
-                            uint32_t* sidx, float* sw) {
-    for (uint32_t sp = blockIdx.x * blockDim.x + threadIdx.x; sp < n; sp += gridDim.x * blockDim.x) {
-        const uint32_t s0 = starts[perm[sp]], len = sorted_len[sp];
-        const uint32_t base = slice_off[sp >> 5] + (sp & 31u) * 4u;
-        for (uint32_t j = 0; j < len; ++j) {
-            const uint32_t q = base + (j >> 2) * 128u + (j & 3u);
-            sidx[q] = idx[s0 + j];
-            sw[q] = w[s0 + j];
+// A warp copies a slice, 32 links of each of its 32 rows at a time through
+// shared memory: rows are read and the interleaved blocks written as whole
+// lines. (A thread copying its own row touched a line per link on both sides:
+// 0.226 ms for the 2.36M links of the Cornell box.)
+static constexpr int kFillWarps = 4;
+__global__ void __launch_bounds__(kFillWarps * 32) k_sell_fill(const uint32_t* starts, const uint32_t* idx,
+                                                               const float* w, uint32_t n, const uint32_t* perm,
+                                                               const uint32_t* sorted_len, const uint32_t* slice_off,
+                                                               uint32_t* sidx, float* sw) {
+    __shared__ uint32_t ti[kFillWarps][32][33];
+    __shared__ float tw[kFillWarps][32][33];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t ns = (n + 31u) / 32u;
+    for (uint32_t k = blockIdx.x * kFillWarps + warp; k < ns; k += gridDim.x * kFillWarps) {
+        const uint32_t sp = k * 32u + lane;
+        const uint32_t len = sp < n ? sorted_len[sp] : 0u, s0 = sp < n ? starts[perm[sp]] : 0u;
+        const uint32_t base = slice_off[k], most = __shfl_sync(kFull, len, 0);
+        for (uint32_t t = 0; t < most; t += 32u) {
+#pragma unroll 8
+            for (uint32_t r = 0; r < 32u; ++r) {
+                const uint32_t sr = __shfl_sync(kFull, s0, r), lr = __shfl_sync(kFull, len, r);
+                if (t + lane < lr) {
+                    ti[warp][r][lane] = idx[(size_t)sr + t + lane];
+                    tw[warp][r][lane] = w[(size_t)sr + t + lane];
+                }
+            }
+            __syncwarp();
+            // Four links of each row make a block of 128 entries.
+            const uint32_t j0 = lane & 3u, blocks = min((most - t + 3u) / 4u, 8u);
+            for (uint32_t q = 0; q < blocks; ++q)
+#pragma unroll
+                for (uint32_t r0 = 0; r0 < 32u; r0 += 8u) {
+                    const uint32_t r = r0 + (lane >> 2), j = q * 4u + j0;
+                    const size_t o = (size_t)base + ((t >> 2) + q) * 128u + r * 4u + j0;
+                    if (t + j < __shfl_sync(kFull, len, r)) {
+                        sidx[o] = ti[warp][r][j];
+                        sw[o] = tw[warp][r][j];
+                    }
+                }
+            __syncwarp();
         }
     }
 }
@@ -449,7 +479,8 @@ int launch_sell_sizes(cudaStream_t st, const uint32_t* sorted_len, uint32_t n, u
 int launch_sell_fill(cudaStream_t st, const uint32_t* starts, const uint32_t* idx, const float* w, uint32_t n,
                      const uint32_t* perm, const uint32_t* sorted_len, const uint32_t* slice_off, uint32_t* sidx,
                      float* sw) {
-    k_sell_fill<<<grid_for(n, 256), 256, 0, st>>>(starts, idx, w, n, perm, sorted_len, slice_off, sidx, sw);
+    k_sell_fill<<<grid_for(n, kFillWarps * 32, 12), kFillWarps * 32, 0, st>>>(starts, idx, w, n, perm, sorted_len,
+                                                                             slice_off, sidx, sw);
     return 1;
 }
 

@@ -342,21 +342,31 @@ void launch_visibility(cudaStream_t st, BlobRef blob, SceneConsts sc, const floa
 
 // Sort keys of the visibility order: target cluster, then the source
 // surfel's cluster (nc when it has none); values: candidate indices.
+template <class K>
 __global__ void k_vis_keys(unsigned long long ncand, const uint32_t* cand_c, const uint32_t* cand_row,
-                           const uint32_t* cid, uint32_t nc, unsigned long long* keys, uint32_t* vals) {
+                           const uint32_t* cid, uint32_t nc, K* keys, uint32_t* vals) {
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < ncand; k += stride) {
         const uint32_t src = cid[cand_row[k]];
-        keys[k] = (unsigned long long)cand_c[k] * (nc + 1ull) + (src < nc ? src : nc);
+        keys[k] = (K)((K)cand_c[k] * (K)(nc + 1u) + (src < nc ? src : nc));
         vals[k] = (uint32_t)k;
     }
 }
 
-int launch_vis_keys(cudaStream_t st, unsigned long long ncand, const uint32_t* cand_c, const uint32_t* cand_row,
-                    const uint32_t* cid, uint32_t nc, unsigned long long* keys, uint32_t* vals) {
+template <class K>
+static int vis_keys(cudaStream_t st, unsigned long long ncand, const uint32_t* cand_c, const uint32_t* cand_row,
+                    const uint32_t* cid, uint32_t nc, K* keys, uint32_t* vals) {
     if (ncand == 0) return 0;
     k_vis_keys<<<grid_for(ncand, 256), 256, 0, st>>>(ncand, cand_c, cand_row, cid, nc, keys, vals);
     return 1;
+}
+int launch_vis_keys(cudaStream_t st, unsigned long long ncand, const uint32_t* cand_c, const uint32_t* cand_row,
+                    const uint32_t* cid, uint32_t nc, uint32_t* keys, uint32_t* vals) {
+    return vis_keys(st, ncand, cand_c, cand_row, cid, nc, keys, vals);
+}
+int launch_vis_keys(cudaStream_t st, unsigned long long ncand, const uint32_t* cand_c, const uint32_t* cand_row,
+                    const uint32_t* cid, uint32_t nc, unsigned long long* keys, uint32_t* vals) {
+    return vis_keys(st, ncand, cand_c, cand_row, cid, nc, keys, vals);
 }
 void launch_closure(cudaStream_t st, BlobRef blob, SceneConsts sc, const float4* sp, const float4* sn,
                     uint32_t n, const uint32_t* order, uint16_t* clo, uint32_t* status, unsigned long long* counts,

@@ -136,6 +136,8 @@ void launch_visibility(cudaStream_t st, BlobRef blob, SceneConsts sc, const floa
 // Keys (target cluster * (nc + 1) + source cluster) and candidate indices
 // for the stable sort that gives launch_visibility its order.
 int launch_vis_keys(cudaStream_t st, unsigned long long ncand, const uint32_t* cand_c, const uint32_t* cand_row,
+                    const uint32_t* cid, uint32_t nc, uint32_t* keys, uint32_t* vals);
+int launch_vis_keys(cudaStream_t st, unsigned long long ncand, const uint32_t* cand_c, const uint32_t* cand_row,
                     const uint32_t* cid, uint32_t nc, unsigned long long* keys, uint32_t* vals);
 // clo: per (row, ray) slot (open << 8) | steps, n * 16 entries.
 void launch_closure(cudaStream_t st, BlobRef blob, SceneConsts sc, const float4* sp, const float4* sn,
@@ -335,6 +337,7 @@ static constexpr uint32_t kEmitChunk = 4096;
 int launch_emit_grad(cudaStream_t st, const float4* dpix, const float* gimg, uint32_t npix, const float4* ebar,
                      const float4* albedo, const float* terms, uint32_t n, int nl, float* partials, float* out);
 int launch_unpack3(cudaStream_t st, const float4* in, uint32_t n, float* out);
+int launch_unpack_w(cudaStream_t st, const float4* in, uint32_t n, float* out);
 
 // ---- packed multi-scene frame (k_multi.cu) ----
 // One scene's device state, as its own context prepared it.
