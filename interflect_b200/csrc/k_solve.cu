@@ -161,8 +161,13 @@ static constexpr int kTileWarps = 8;
 static constexpr uint32_t kTileWords = 32u * 33u;  // one array of one tile
 static constexpr size_t kTileBytes = (size_t)kTileWarps * 2u * 2u * kTileWords * 4u;
 static constexpr uint32_t kTileMinRows = 65536;
-// Cluster radiosities gathered from shared memory: up to 4,096 clusters.
-static constexpr size_t kSharedRadMax = 64u * 1024u;
+// Cluster radiosities gathered from shared memory: up to 4,096 clusters. Few
+// rows take as long as the longest one's chain of gathers, each kernel with a
+// cold L1: small CTAs spread them over the SMs, and up to 1,024 clusters a copy
+// per CTA pays (20,000 rows, 793 clusters: 12 bounces 0.325 -> 0.258 ms; 50,000
+// rows, 2,504 clusters, 40 KiB a copy: 0.44 -> 0.47 ms).
+static constexpr size_t kSharedRadMax = 64u * 1024u, kSharedRadSmall = 16u * 1024u;
+static constexpr unsigned kFewRowsBlock = 128;
 
 __device__ __forceinline__ void copy4_async(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
@@ -384,9 +389,12 @@ void launch_solve_bounce(cudaStream_t st, SurfelArrays s, uint32_t n, const floa
         if (n >= kTileMinRows && cbytes <= kSharedRadMax)
             launch_pdl(k_jacobi_sell<true>, wave_grid(k_jacobi_sell<true>, kJacBlock, cbytes, n), kJacBlock, cbytes, st,
                        direct, albedo, s.irr, s.rad, n, *sell, crad, nc, ctl, it);
+        else if (cbytes <= kSharedRadSmall)
+            launch_pdl(k_jacobi_sell<true>, grid_for(n, kFewRowsBlock), kFewRowsBlock, cbytes, st, direct, albedo, s.irr,
+                       s.rad, n, *sell, crad, nc, ctl, it);
         else
-            launch_pdl(k_jacobi_sell<false>, grid_for(n, kJacBlock), kJacBlock, 0, st, direct, albedo, s.irr, s.rad, n,
-                       *sell, crad, nc, ctl, it);
+            launch_pdl(k_jacobi_sell<false>, grid_for(n, kFewRowsBlock, 16), kFewRowsBlock, 0, st, direct, albedo, s.irr,
+                       s.rad, n, *sell, crad, nc, ctl, it);
     } else if (n >= kTileMinRows) {
         const unsigned block = kTileWarps * 32u;
         if (cbytes <= kSharedRadMax)
