@@ -384,6 +384,7 @@ void configure_surfel_kernels(int max_dyn_smem);
 void configure_transfer_kernels(int max_dyn_smem);
 void configure_solve_kernels(int max_dyn_smem);
 void configure_bounce_kernels();
+void configure_batch_kernels();
 void configure_shade_kernels(int max_dyn_smem);
 void configure_diff_kernels(int max_dyn_smem);
 void configure_path_kernels(int max_dyn_smem);
@@ -399,6 +400,7 @@ inline void configure_kernels(int max_dyn_smem) {
     configure_surfel_kernels(max_dyn_smem);
     configure_transfer_kernels(max_dyn_smem);
     configure_solve_kernels(max_dyn_smem);
+    configure_batch_kernels();
     configure_shade_kernels(max_dyn_smem);
     configure_diff_kernels(max_dyn_smem);
     configure_path_kernels(max_dyn_smem);
