@@ -137,8 +137,9 @@ __device__ __forceinline__ float row_update(const float4* direct, const float4* 
 
 __global__ void __launch_bounds__(kJacBlock) k_jacobi(const float4* direct, const float4* albedo, float4* irr_out,
                                                        float4* rad, uint32_t n, const uint32_t* starts,
-                                                       const uint32_t* idx, const float* w, const float4* crad,
-                                                       SolveCtl* ctl, uint32_t it, int vec) {
+                                                       const uint32_t* idx, const float* w,
+                                                       const float4* __restrict__ crad, SolveCtl* ctl, uint32_t it,
+                                                       int vec) {
     pdl_wait();
     if (ctl->done) return;
     float dmax = 0.0f;
@@ -149,18 +150,11 @@ __global__ void __launch_bounds__(kJacBlock) k_jacobi(const float4* direct, cons
     note_residual(dmax, ctl, it);
 }
 
-// The same for many rows, whose CSR arrays stream from memory. A thread's own
-// loads of its row touch a cache line each, and so do its gathers: 1.5 L1
-// cycles a link, twice the time the arrays take to arrive. Here a warp fetches
-// the next 32 links of each of its 32 rows together, one coalesced copy per
-// row and array straight into shared memory (double-buffered, rows padded to
-// 33 words so that the lanes read their own rows without conflicts), and the
-// cluster radiosities are gathered from a copy in shared memory where they
-// fit (kShared). Each lane still adds its row's links in order.
-static constexpr int kTileWarps = 8;
-static constexpr uint32_t kTileWords = 32u * 33u;  // one array of one tile
-static constexpr size_t kTileBytes = (size_t)kTileWarps * 2u * 2u * kTileWords * 4u;
-static constexpr uint32_t kTileMinRows = 65536;
+// Many rows: from here on they fill the GPU's warps. The wide kernel's line is
+// lower where k_jacobi's loads bind and higher where its shorter chain per link
+// does (33,000 rows of 32 links, 9 bounces: 168 us wide, 159 us not; 60,000
+// rows of 97 links: 311 and 323 us).
+static constexpr uint32_t kManyRows = 65536, kWideRows = 49152;
 // Cluster radiosities gathered from shared memory: up to 4,096 clusters. Few
 // rows take as long as the longest one's chain of gathers, each kernel with a
 // cold L1: small CTAs spread them over the SMs, and up to 1,024 clusters a copy
@@ -169,88 +163,70 @@ static constexpr uint32_t kTileMinRows = 65536;
 static constexpr size_t kSharedRadMax = 64u * 1024u, kSharedRadSmall = 16u * 1024u;
 static constexpr unsigned kFewRowsBlock = 128;
 
-__device__ __forceinline__ void copy4_async(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+// Eight 32-bit words in one load; p is 32-byte aligned, its data constant.
+__device__ __forceinline__ void load8(const void* p, uint32_t v[8]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(p));
 }
 
+// The same where idx and w are 32-byte aligned, as allocations are. The rows
+// of a warp lie in 32 places, so each of its loads is 32 cache lines' worth of
+// L1 cycles however little it takes: links come eight at a time in 256-bit
+// loads of whole sectors, from the aligned place at or before the row's first
+// link to the one at or after its last, those of the neighbouring rows masked;
+// and the cluster radiosities, 32 lines to a gather, come from a copy in
+// shared memory where they fit (kShared), some 10 cycles. 800,000 rows of 97
+// links: 3.11 -> 2.33 ms for 10 bounces, 2.7 TB/s of the arrays; 150,000 such
+// rows, which L2 holds, 0.73 -> 0.65 ms for 12. (Tiles of 32 rows copied to
+// shared memory by cp.async first, so that every load is coalesced, took 2.78
+// and 0.82 ms: the shared-memory pipe then moves each link three times.)
 template <bool kShared>
-__global__ void __launch_bounds__(kTileWarps * 32) k_jacobi_tiles(const float4* direct, const float4* albedo,
-                                                                  float4* irr_out, float4* rad, uint32_t n,
-                                                                  const uint32_t* starts, const uint32_t* idx,
-                                                                  const float* w, const float4* crad, uint32_t nc,
-                                                                  SolveCtl* ctl, uint32_t it) {
-    extern __shared__ __align__(16) uint8_t tile_smem[];
+__global__ void __launch_bounds__(kJacBlock) k_jacobi_wide(const float4* direct, const float4* albedo,
+                                                            float4* irr_out, float4* rad, uint32_t n,
+                                                            const uint32_t* starts, const uint32_t* idx,
+                                                            const float* w, const float4* __restrict__ crad_g,
+                                                            uint32_t nc, SolveCtl* ctl, uint32_t it) {
+    extern __shared__ __align__(16) uint8_t wide_smem[];
     pdl_wait();
     if (ctl->done) return;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    float4* cs = reinterpret_cast<float4*>(tile_smem + kTileBytes);
+    float4* cs = reinterpret_cast<float4*>(wide_smem);
     if constexpr (kShared) {
-        for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x) cs[c] = crad[c];
+        for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x) cs[c] = crad_g[c];
         __syncthreads();
     }
-    uint32_t* tiles = reinterpret_cast<uint32_t*>(tile_smem) + (size_t)warp * 4u * kTileWords;
-    const uint32_t tiles_at = (uint32_t)__cvta_generic_to_shared(tiles);
-    const uint32_t groups = (n + 31u) / 32u, stride = gridDim.x * kTileWarps;
-    // Links [32 t, 32 t + 32) of the group's rows into stage st.
-    auto fetch = [&](uint32_t s, uint32_t len, uint32_t t, uint32_t st) {
-        const uint32_t at = tiles_at + (st * 2u * kTileWords + lane) * 4u, j = 32u * t + lane;
-#pragma unroll 8
-        for (uint32_t r = 0; r < 32u; ++r) {
-            const uint32_t sr = __shfl_sync(kFull, s, r), lr = __shfl_sync(kFull, len, r);
-            if (j < lr) {
-                copy4_async(at + r * 132u, idx + (size_t)sr + j);
-                copy4_async(at + r * 132u + kTileWords * 4u, w + (size_t)sr + j);
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    auto row_of = [&](uint32_t g, uint32_t& s, uint32_t& len) {
-        const uint32_t row = g * 32u + lane;
-        s = len = 0;
-        if (g < groups && row < n) {
-            s = starts[row];
-            len = starts[row + 1] - s;
-        }
-    };
-    uint32_t g = blockIdx.x * kTileWarps + warp, s, len, st = 0;
+    const uint32_t total = starts[n];
     float dmax = 0.0f;
-    row_of(g, s, len);
-    if (g < groups) fetch(s, len, 0, 0);
-    for (; g < groups; g += stride) {
-        uint32_t s2, len2;
-        row_of(g + stride, s2, len2);
-        const uint32_t most = __reduce_max_sync(kFull, len), turns = most > 32u ? (most + 31u) / 32u : 1u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t s = starts[i], e = starts[i + 1];
         V irr{0.0f, 0.0f, 0.0f};
-        for (uint32_t t = 0; t < turns; ++t, st ^= 1u) {
-            // The next tile of this group, or the first of the next.
-            if (t + 1u < turns) fetch(s, len, t + 1u, st ^ 1u);
-            else fetch(s2, len2, 0, st ^ 1u);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncwarp();
-            const uint32_t* ti = tiles + st * 2u * kTileWords + lane * 33u;
-            const float* tw = reinterpret_cast<const float*>(ti + kTileWords);
-            const uint32_t cnt = len > 32u * t ? min(len - 32u * t, 32u) : 0u;
-            uint32_t j = 0;
-            for (; j + 4u <= cnt; j += 4u) {
-                float4 c[4];
-                float v[4];
+        for (uint32_t k = s & ~7u; k < e; k += 8u) {
+            uint32_t a[8], b[8];
+            if (k + 8u <= total) {
+                load8(idx + k, a);
+                load8(w + k, b);
+            } else {  // the last links of the matrix
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    v[k] = tw[j + k];
-                    c[k] = kShared ? cs[ti[j + k]] : crad[ti[j + k]];
+                for (uint32_t t = 0; t < 8u; ++t) {
+                    a[t] = k + t < total ? __ldg(&idx[k + t]) : 0u;
+                    b[t] = k + t < total ? __float_as_uint(__ldg(&w[k + t])) : 0u;
                 }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) irr = irr + mk4(c[k]) * v[k];
             }
-            for (; j < cnt; ++j) irr = irr + mk4(kShared ? cs[ti[j]] : crad[ti[j]]) * tw[j];
-            __syncwarp();
+            if (k >= s && k + 8u <= e) {
+                float4 c[8];
+#pragma unroll
+                for (int t = 0; t < 8; ++t) c[t] = kShared ? cs[a[t]] : crad_g[a[t]];
+#pragma unroll
+                for (int t = 0; t < 8; ++t) irr = irr + mk4(c[t]) * __uint_as_float(b[t]);
+            } else {
+#pragma unroll
+                for (uint32_t t = 0; t < 8u; ++t)
+                    if (k + t >= s && k + t < e)
+                        irr = irr + mk4(kShared ? cs[a[t]] : crad_g[a[t]]) * __uint_as_float(b[t]);
+            }
         }
-        const uint32_t row = g * 32u + lane;
-        if (row < n) dmax = fmaxf(dmax, row_update(direct, albedo, irr_out, rad, row, irr));
-        s = s2;
-        len = len2;
+        dmax = fmaxf(dmax, row_update(direct, albedo, irr_out, rad, i, irr));
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
     pdl_trigger();
     note_residual(dmax, ctl, it);
 }
@@ -386,7 +362,7 @@ void launch_solve_bounce(cudaStream_t st, SurfelArrays s, uint32_t n, const floa
     const float4 *direct = s.direct, *albedo = s.albedo, *crad = cluster_rad;
     const size_t cbytes = (size_t)nc * 16u;
     if (sell && sell->perm) {
-        if (n >= kTileMinRows && cbytes <= kSharedRadMax)
+        if (n >= kManyRows && cbytes <= kSharedRadMax)
             launch_pdl(k_jacobi_sell<true>, wave_grid(k_jacobi_sell<true>, kJacBlock, cbytes, n), kJacBlock, cbytes, st,
                        direct, albedo, s.irr, s.rad, n, *sell, crad, nc, ctl, it);
         else if (cbytes <= kSharedRadSmall)
@@ -395,14 +371,13 @@ void launch_solve_bounce(cudaStream_t st, SurfelArrays s, uint32_t n, const floa
         else
             launch_pdl(k_jacobi_sell<false>, grid_for(n, kFewRowsBlock, 16), kFewRowsBlock, 0, st, direct, albedo, s.irr,
                        s.rad, n, *sell, crad, nc, ctl, it);
-    } else if (n >= kTileMinRows) {
-        const unsigned block = kTileWarps * 32u;
+    } else if (n >= kWideRows && (((uintptr_t)idx | (uintptr_t)w) & 31u) == 0) {
         if (cbytes <= kSharedRadMax)
-            launch_pdl(k_jacobi_tiles<true>, wave_grid(k_jacobi_tiles<true>, block, kTileBytes + cbytes, n), block,
-                       kTileBytes + cbytes, st, direct, albedo, s.irr, s.rad, n, starts, idx, w, crad, nc, ctl, it);
+            launch_pdl(k_jacobi_wide<true>, wave_grid(k_jacobi_wide<true>, kJacBlock, cbytes, n), kJacBlock, cbytes, st,
+                       direct, albedo, s.irr, s.rad, n, starts, idx, w, crad, nc, ctl, it);
         else
-            launch_pdl(k_jacobi_tiles<false>, wave_grid(k_jacobi_tiles<false>, block, kTileBytes, n), block, kTileBytes,
-                       st, direct, albedo, s.irr, s.rad, n, starts, idx, w, crad, nc, ctl, it);
+            launch_pdl(k_jacobi_wide<false>, grid_for(n, kJacBlock), kJacBlock, 0, st, direct, albedo, s.irr, s.rad, n,
+                       starts, idx, w, crad, nc, ctl, it);
     } else {
         const int vec = (((uintptr_t)idx | (uintptr_t)w) & 15u) == 0 ? 1 : 0;
         launch_pdl(k_jacobi, grid_for(n, kJacBlock), kJacBlock, 0, st, direct, albedo, s.irr, s.rad, n, starts, idx, w,
@@ -495,9 +470,7 @@ int launch_sell_fill(cudaStream_t st, const uint32_t* starts, const uint32_t* id
 // Their own limits, which need no context (ifx_solve_noalloc has none).
 void configure_bounce_kernels() {
     cudaFuncSetAttribute(k_jacobi_sell<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedRadMax);
-    cudaFuncSetAttribute(k_jacobi_tiles<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(kTileBytes + kSharedRadMax));
-    cudaFuncSetAttribute(k_jacobi_tiles<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileBytes);
+    cudaFuncSetAttribute(k_jacobi_wide<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedRadMax);
 }
 
 void configure_solve_kernels(int max_dyn_smem) {

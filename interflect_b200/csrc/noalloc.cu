@@ -126,12 +126,11 @@ extern "C" int ifx_solve_noalloc(int device, void* stream, uint32_t n, uint32_t 
     ifx::SurfelArrays s{(float4*)p_area4, nullptr, (float4*)albedo4, (float4*)direct4, (float4*)irr4,
                         (float4*)rad4};
     ifx::SolveCtl h{};
-    // Bounces queued before the host looks at the flag: the first 6, then 8 at
-    // a time. A look costs some 10 us, a bounce queued past convergence two
-    // launches (5 us); solves take 5 to 14 bounces.
-    uint32_t batch = 6;
-    for (uint32_t it = 0; it < max_bounces; batch = 8) {
-        uint32_t end = it + batch < max_bounces ? it + batch : max_bounces;
+    // Bounces queued before the host looks at the flag. A look leaves the GPU
+    // idle for some 15 us, as long as five bounces queued past convergence.
+    const uint32_t kBatch = 16;
+    for (uint32_t it = 0; it < max_bounces;) {
+        uint32_t end = it + kBatch < max_bounces ? it + kBatch : max_bounces;
         int l = 0;
         for (; it < end; ++it) {
             ifx::launch_solve_bounce(st, s, n, (const float4*)cluster_p_area4, (const uint2*)cluster_ranges, members,

@@ -1,7 +1,7 @@
 """The device-buffer solve's row kernels against the same f32 sums formed by
-numpy in CSR order: from 65,536 rows on a warp stages its rows' links in
-shared memory, with the cluster radiosities there too up to 4,096 clusters.
-Rows of 0, 1, 31, 32, 33, 64, 65 and other lengths, at every alignment, and
+numpy in CSR order: from 49,152 rows on links are read eight at a time from
+aligned places, with the cluster radiosities in shared memory up to 4,096
+clusters. Rows of 0, 1, 31, 32, 33, 64, 65 and other lengths, at every alignment, and
 row counts around the switch and off a warp's multiple. Products and sums
 round the same way, so the results are equal to the bit."""
 import numpy as np
@@ -23,7 +23,7 @@ def row_sums(starts, idx, w, crad):
     return irr
 
 
-@pytest.mark.parametrize("n,nc", [(1000, 300), (65535, 300), (65536, 300), (65536 + 37, 4096), (70001, 4097)])
+@pytest.mark.parametrize("n,nc", [(1000, 300), (49151, 300), (49152, 300), (49152 + 37, 4096), (70001, 4097)])
 def test_rows_equal_the_ordered_sums(n, nc):
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(n + nc)
