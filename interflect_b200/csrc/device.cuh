@@ -335,32 +335,33 @@ __device__ __forceinline__ float prim_dist(const DPrim& pr, V p, C& cnt) {
 // with a strict `<`. A subtraction never lowers the base primitive's
 // distance: max(d, -s) >= d exactly, and the smooth form is above max(d, -s)
 // but for rounding (a few ulps of its operands, far below the margin here).
-// So in the uncounted kernels, a base at or beyond `best` (plus that margin
-// for the smooth form) cannot win the comparison, and its subtractions are
-// not evaluated; the returned value is then the base's, itself >= best. The
-// counting kernels evaluate everything, as the reference does.
+// So in the uncounted kernels, once the distance is at or beyond `best` (plus
+// that margin for the smooth form) it cannot win the comparison, and the
+// subtractions left are not evaluated; the returned value is then itself >=
+// best. The counting kernels evaluate everything, as the reference does.
 template <class C>
 __device__ __forceinline__ float obj_dist(const SceneView& sv, const DObject& o, V p, C& cnt, float best = kMaxF) {
     float d = 0.0f;
+    const float limit = best + (o.smooth > 0.0f ? 1e-5f * (1.0f + fabsf(best) + o.smooth) : 0.0f);
     // The base is the loop's first turn, so that prim_dist has one site.
 #pragma unroll 1
     for (int s = 0; s <= o.nsub; ++s) {
         const float sd = prim_dist(sv.prim(o.prim + s), p, cnt);
+        if (s > 0) cnt.add(o.smooth > 0.0f ? CN_SMOOTH : CN_HARD);
         if (s == 0) {
             d = sd;
-            if constexpr (sizeof(C) == 1) {
-                if (o.nsub > 0 && d >= best + (o.smooth > 0.0f ? 1e-5f * (1.0f + fabsf(best) + o.smooth) : 0.0f))
-                    return d;
-            }
-            continue;
-        }
-        cnt.add(o.smooth > 0.0f ? CN_SMOOTH : CN_HARD);
-        if (o.smooth > 0.0f) {
+        } else if (o.smooth > 0.0f) {
             float k = o.smooth;
-            float hk = clampr(0.5f - 0.5f * (d + sd) / k, 0.0f, 1.0f);
-            d = d * (1.0f - hk) + (-sd) * hk + k * hk * (1.0f - hk);
+            // Where d + sd >= k the weight hk is 0 and the blend is d.
+            if (sizeof(C) > 1 || !(d + sd >= 1.00001f * k && sd < 1e30f)) {
+                float hk = clampr(0.5f - 0.5f * (d + sd) / k, 0.0f, 1.0f);
+                d = d * (1.0f - hk) + (-sd) * hk + k * hk * (1.0f - hk);
+            }
         } else {
             d = fmaxf(d, -sd);
+        }
+        if constexpr (sizeof(C) == 1) {
+            if (s < o.nsub && d >= limit) return d;
         }
     }
     return d;

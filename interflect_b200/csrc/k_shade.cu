@@ -260,9 +260,14 @@ __global__ void __launch_bounds__(128) k_setup2(ShadeParams P) {
 
 // main.rs:289-358: the pixel's colour from the stored hits, form factors and
 // visibilities, in the reference's order of operations, then film.rs encode.
+// Bound by the gather's loads: 64 registers keep 8 CTAs on an SM, no geometry
+// is staged (only lights and materials are read), and CTAs are handed out as
+// they finish, since gathers differ in length.
+static constexpr int kComposeCtas = 64;
 template <class C>
-__global__ void __launch_bounds__(128) k_compose(ShadeParams P) {
-    IFX_SCENE_PROLOGUE(P.blob, P.status, sv);
+__global__ void __launch_bounds__(128, 8) k_compose(ShadeParams P) {
+    SceneView sv = make_view(P.blob.ptr);
+    sv.status = P.status;
     C cnt;
     __shared__ float t8[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) t8[i] = P.srgb_t[i];
@@ -318,7 +323,7 @@ static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, i
     if (part & kShadeCompose) {
         rec(12);
         const unsigned long long cpx = p.pix1 ? (unsigned long long)(p.pix1 - p.pix0) : px;
-        k_compose<C><<<grid_for(cpx, 128, 16), 128, sm, st>>>(with(4));
+        k_compose<C><<<grid_for(cpx, 128, kComposeCtas), 128, 0, st>>>(with(4));
         rec(13);
     }
 }
@@ -406,13 +411,12 @@ int launch_light_slots(cudaStream_t st, const ShadeParams& p, const SurfelArrays
 }
 
 int launch_compose(cudaStream_t st, const ShadeParams& p) {
-    const size_t sm = blob_smem(p.blob, 128);
     ShadeParams q = p;
     q.counts = nullptr;
     if (p.blob.tree3)
-        k_compose<NoCount3><<<grid_for((unsigned long long)p.w * p.h, 128, 16), 128, sm, st>>>(q);
+        k_compose<NoCount3><<<grid_for((unsigned long long)p.w * p.h, 128, kComposeCtas), 128, 0, st>>>(q);
     else
-        k_compose<NoCount><<<grid_for((unsigned long long)p.w * p.h, 128, 16), 128, sm, st>>>(q);
+        k_compose<NoCount><<<grid_for((unsigned long long)p.w * p.h, 128, kComposeCtas), 128, 0, st>>>(q);
     return 1;
 }
 
@@ -423,7 +427,6 @@ static void configure_one(int max_dyn_smem) {
     cudaFuncSetAttribute(k_shadow<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
     cudaFuncSetAttribute(k_reflect<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
     cudaFuncSetAttribute(k_setup2<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_compose<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
 }
 
 void configure_shade_kernels(int max_dyn_smem) {
