@@ -1838,8 +1838,15 @@ static int render_impl(ifx_ctx* ctx, const ifx_camera* cam, int mode, uint32_t w
     CK(cudaMemsetAsync(ctx->qlen.p, 0, 16, ctx->st));
     CK(cudaMemsetAsync(ctx->qcur.p, 0, 16 * 8, ctx->st));
     CK(cudaEventRecord(ctx->ev0, ctx->st));
-    ctx->launches += (uint64_t)launch_shade(ctx->st, P, ctx->shev);
-    CKL();
+    // The primary shadow rays beside the mirror passes, each too few to fill
+    // the GPU to its end (853 x 479: 2.25 -> 1.98 ms a view). ifx_frame has the
+    // GI stages beside them instead, and is slower with this too.
+    const SideStream side{ctx->st3, ctx->tev[0], ctx->tev[1]};
+    ctx->launches += (uint64_t)launch_shade(ctx->st, P, ctx->shev, kShadeAll, &side);
+    if (cudaError_t le = cudaGetLastError(); le != cudaSuccess) {
+        cudaStreamSynchronize(ctx->st3);  // nothing stays in flight once the call returns
+        return fail(ctx, IFX_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(le));
+    }
     CK(cudaEventRecord(ctx->ev1, ctx->st));
     unsigned long long e = 0;
     CK(cudaMemcpyAsync(&e, &small[3], 8, cudaMemcpyDeviceToHost, ctx->st));

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(128, 8) k_compose(ShadeParams P) {
 // slots (kNumCounters u64 each) 0 primary, 1 shadow, 2 reflect, 3 shadow2,
 // 4 the rest.
 template <class C>
-static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, int part) {
+static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, int part, const SideStream* side) {
     const size_t sm = blob_smem(p.blob, 128);
     const unsigned long long px = (unsigned long long)p.w * p.h;
     const unsigned long long slots = px * (unsigned long long)(p.nl > 0 ? p.nl : 1);
@@ -294,9 +294,10 @@ static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, i
         q.counts = p.counts ? p.counts + (size_t)slot * kNumCounters : nullptr;
         return q;
     };
-    auto rec = [&](int i) {
-        if (ev) cudaEventRecord(ev[i], st);
+    auto rec_on = [&](int i, cudaStream_t on) {
+        if (ev) cudaEventRecord(ev[i], on);
     };
+    auto rec = [&](int i) { rec_on(i, st); };
     if (part & kShadeFront) {
         rec(0);
         k_primary<C><<<persistent_grid(k_primary<C>, 128, sm, px), 128, sm, st>>>(with(0));
@@ -304,10 +305,17 @@ static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, i
         rec(8);
         k_setup<C><<<grid_for(px, 128, 16), 128, sm, st>>>(with(4));
         rec(9);
-        rec(2);
-        k_shadow<C><<<persistent_grid(k_shadow<C>, 128, sm, slots), 128, sm, st>>>(
+        const bool fork = side && p.has_gi;
+        const cudaStream_t st1 = fork ? side->st : st;
+        if (fork) {
+            cudaEventRecord(side->fork, st);
+            cudaStreamWaitEvent(st1, side->fork, 0);
+        }
+        rec_on(2, st1);
+        k_shadow<C><<<persistent_grid(k_shadow<C>, 128, sm, slots), 128, sm, st1>>>(
             with(1), p.hp1, p.hn1, p.q1, &p.qlen[0], p.vis1, &p.cursors[2]);
-        rec(3);
+        rec_on(3, st1);
+        if (fork) cudaEventRecord(side->join, st1);
         rec(4);
         if (p.has_gi) k_reflect<C><<<persistent_grid(k_reflect<C>, 128, sm, px), 128, sm, st>>>(with(2));
         rec(5);
@@ -319,6 +327,7 @@ static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, i
             k_shadow<C><<<persistent_grid(k_shadow<C>, 128, sm, slots), 128, sm, st>>>(
                 with(3), p.hp2, p.hn2, p.q2, &p.qlen[2], p.vis2, &p.cursors[3]);
         rec(7);
+        if (fork) cudaStreamWaitEvent(st, side->join, 0);
     }
     if (part & kShadeCompose) {
         rec(12);
@@ -328,10 +337,10 @@ static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, i
     }
 }
 
-int launch_shade(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, int part) {
-    if (p.counts) launch_all<Counts>(st, p, ev, part);
-    else if (p.blob.tree3) launch_all<NoCount3>(st, p, ev, part);
-    else launch_all<NoCount>(st, p, ev, part);
+int launch_shade(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, int part, const SideStream* side) {
+    if (p.counts) launch_all<Counts>(st, p, ev, part, side);
+    else if (p.blob.tree3) launch_all<NoCount3>(st, p, ev, part, side);
+    else launch_all<NoCount>(st, p, ev, part, side);
     return ((part & kShadeFront) ? (p.has_gi ? 6 : 3) : 0) + ((part & kShadeCompose) ? 1 : 0);
 }
 

@@ -280,7 +280,15 @@ struct ShadeParams {
 // the composition, or both.
 static constexpr int kShadeEvents = 14;
 enum : int { kShadeFront = 1, kShadeCompose = 2, kShadeAll = 3 };
-int launch_shade(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, int part = kShadeAll);
+// `side` (nullable, with two untimed events of its own): the primary hits'
+// shadow rays run there while the mirror rays and their shadow rays, which
+// need nothing of them, run on st; st waits for them.
+struct SideStream {
+    cudaStream_t st;
+    cudaEvent_t fork, join;
+};
+int launch_shade(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, int part = kShadeAll,
+                 const SideStream* side = nullptr);
 // k_compose alone over the hits, form factors and visibilities a previous
 // launch_shade with the same parameters left in the wavefront buffers.
 int launch_compose(cudaStream_t st, const ShadeParams& p);
