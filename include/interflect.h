@@ -393,8 +393,8 @@ int ifx_diff_forward(ifx_ctx* ctx, const float* rho, const float* emit, float* i
 int ifx_diff_backward(ifx_ctx* ctx, const float* grad_image, float* grad_rho, float* grad_emit);
 
 /* ------------------------------------------------- packed multi-scene --- */
-/* Many independent scenes solved and shaded in ONE persistent cooperative
- * kernel launch, replayed from a captured CUDA graph. No counterpart in the
+/* Many independent scenes solved in ONE persistent cooperative kernel launch
+ * and shaded in a second, replayed from a captured CUDA graph. No counterpart in the
  * reference (one scene per process). Each scene keeps its own context; the
  * packed frame re-lights its surfels from the stored light factors (the
  * result of solve::light_surfels for the context's current albedo and

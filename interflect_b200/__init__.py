@@ -661,7 +661,7 @@ def solve_noalloc(device: int, stream: int, n: int, nc: int, p_area4: int, direc
 
 
 class MultiScene:
-    """Many scenes' solve + shade in one persistent launch replayed from a
+    """Many scenes' solve (one persistent launch) and shade, replayed from a
     CUDA graph (ifx_multiscene_* in interflect.h). Member contexts must stay
     alive, and unused for other rendering, while they belong to it."""
 

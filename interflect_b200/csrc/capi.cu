@@ -2488,6 +2488,7 @@ extern "C" int ifx_multiscene_add(ifx_multiscene* ms, ifx_ctx* ctx, const ifx_ca
     P.recompose = 1;
     P.evals = nullptr;
     MsScene s{};
+    if (ctx->sell_ready) s.sell = ctx->sellm;
     s.sp = (const float4*)ctx->sp.p;
     s.albedo = (const float4*)ctx->salb.p;
     s.direct = (float4*)ctx->sdir.p;

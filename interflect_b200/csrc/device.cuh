@@ -702,49 +702,9 @@ __device__ __forceinline__ DistHit dist_warp(const SceneView& sv, V p, bool acti
     return dist_mat_ref_warp(sv, p, active, cnt);
 }
 
-// scene.rs:218-236: tetrahedron taps K = (1,-1,-1), (-1,-1,1), (-1,1,-1), (1,1,1).
-template <class C>
-__device__ __forceinline__ V scene_normal(const SceneView& sv, V p, C& cnt) {
-    const float H = 5e-4f;
-    V n{0.0f, 0.0f, 0.0f};
-    const V K[4] = {V{1.0f, -1.0f, -1.0f}, V{-1.0f, -1.0f, 1.0f}, V{-1.0f, 1.0f, -1.0f}, V{1.0f, 1.0f, 1.0f}};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) n = n + K[i] * scene_dist(sv, p + K[i] * H, cnt);
-    float l = len(n);
-    if (l > 1e-12f) return n / l;
-    return V{0.0f, 1.0f, 0.0f};
-}
-
 // ------------------------------------------------------------ trace.rs ----
 static constexpr uint32_t kMaxSteps = 128;    // trace.rs:10
 static constexpr uint32_t kShadowSteps = 96;  // trace.rs:11
-
-struct TraceHit {
-    bool hit;
-    float t;
-    V p;
-    uint32_t mat;
-    uint32_t steps;  // includes the +4 normal taps on a hit (trace.rs:48)
-};
-
-// trace.rs:27-58 without the normal; callers that need it call
-// scene_normal(hit.p), which costs exactly the four counted taps.
-template <class C>
-__device__ __forceinline__ TraceHit trace(const SceneView& sv, V ro, V rd, float tmin, float tmax, C& cnt) {
-    float t = tmin;
-    uint32_t steps = 0;
-    while (steps < kMaxSteps) {
-        V p = ro + rd * t;
-        DistHit h = dist_mat(sv, p, cnt);
-        cnt.add(CN_TSTEP);
-        steps += 1;
-        float eps = 1e-4f * fmaxf(t, 1.0f);
-        if (h.d < eps) return TraceHit{true, t, p, h.mat, steps + 4};
-        t += h.d;
-        if (t > tmax) break;
-    }
-    return TraceHit{false, 0.0f, V{0.0f, 0.0f, 0.0f}, 0u, steps};
-}
 
 // True when this step's cone term X = k * d / max(t - y, 1e-4)
 // (trace.rs:84-124) is provably >= res, so that res = min(res, X) leaves res
@@ -1087,75 +1047,6 @@ __device__ __forceinline__ void add_specular(V& out, V p, V n, V v, V rep, float
     float vis_s = v_smith(n_dot_v, n_dot_l, wide);
     V f = fresnel_schlick(fmaxf(dot(l, h), 0.0f), f0);
     out = out + f * (d * vis_s * energy * n_dot_l) * radiance;
-}
-
-// shade.rs:50-125
-template <class C>
-__device__ __forceinline__ V direct(const SceneView& sv, V p, V n, V v, const DMaterial& m, uint32_t& steps_out,
-                                    C& cnt) {
-    V out{0.0f, 0.0f, 0.0f};
-    uint32_t steps = 0;
-    V tan, bit;
-    frame(n, tan, bit);
-    float n_dot_v = fmaxf(dot(n, v), 1e-4f);
-    float alpha = m.kd[3];
-    V f0{m.f0[0], m.f0[1], m.f0[2]};
-    V kd{m.kd[0], m.kd[1], m.kd[2]};
-    for (int li = 0; li < sv.n_lights; ++li) {
-        const DQuadLight& L = sv.light(li);
-        V lc{L.center[0], L.center[1], L.center[2]};
-        V ln{L.normal[0], L.normal[1], L.normal[2]};
-        V to_light = lc - p;
-        if (dot(ln, -nrm(to_light)) <= 0.0f) continue;
-        float ff = quad_light_ff(L, p, tan, bit, n, cnt);
-        if (ff <= 1e-6f) continue;
-        cnt.add(CN_LIGHT);
-        float dist = len(to_light);
-        float radius = L.center[3];
-        float k = clampr(dist / radius, 1.5f, 96.0f);
-        V ldir = to_light / dist;
-        float shadow_end = fmaxf(dist - radius * 1.25f, 0.05f);
-        uint32_t s;
-        float vis = soft_shadow(sv, p + n * 3e-3f, ldir, 0.015f, shadow_end, k, s, cnt);
-        steps += s;
-        if (vis <= 1e-4f) continue;
-        V radiance = V{L.emit[0], L.emit[1], L.emit[2]} * vis;
-        out = out + kd * radiance * ff;
-        V r = (-v) - n * (2.0f * dot(n, -v));
-        float denom = dot(r, ln);
-        V rep = lc;
-        if (fabsf(denom) > 1e-6f) {
-            float t = dot(V{L.v[0][0], L.v[0][1], L.v[0][2]} - p, ln) / denom;
-            if (t > 0.0f) rep = closest_on_quad(L, p + r * t);
-        }
-        add_specular(out, p, n, v, rep, radius, alpha, n_dot_v, f0, radiance, cnt);
-    }
-    for (int li = 0; li < sv.n_slights; ++li) {  // extension: sphere lights
-        const DSphereLight& L = sv.slight(li);
-        V c{L.c[0], L.c[1], L.c[2]};
-        V to_light = c - p;
-        float ff = sphere_light_ff(p, n, c, L.c[3]);
-        if (ff <= 1e-6f) continue;
-        cnt.add(CN_LIGHT);
-        float dist = len(to_light);
-        float radius = fmaxf(L.c[3], 1e-4f);
-        float k = clampr(dist / radius, 1.5f, 96.0f);
-        V ldir = to_light / dist;
-        float shadow_end = fmaxf(dist - radius * 1.25f, 0.05f);
-        uint32_t s;
-        float vis = soft_shadow(sv, p + n * 3e-3f, ldir, 0.015f, shadow_end, k, s, cnt);
-        steps += s;
-        if (vis <= 1e-4f) continue;
-        V radiance = V{L.emit[0], L.emit[1], L.emit[2]} * vis;
-        out = out + kd * radiance * ff;
-        V r = (-v) - n * (2.0f * dot(n, -v));
-        V ctr = r * dot(to_light, r) - to_light;
-        float cl = len(ctr);
-        V rep = p + to_light + ctr * clampr(radius / fmaxf(cl, 1e-9f), 0.0f, 1.0f);
-        add_specular(out, p, n, v, rep, radius, alpha, n_dot_v, f0, radiance, cnt);
-    }
-    steps_out = steps;
-    return out;
 }
 
 // shade.rs:133-164

@@ -362,6 +362,7 @@ struct MsScene {
     const uint32_t* members;
     const uint32_t *starts, *idx;
     const float* w;
+    SellMatrix sell;        // the same transfer in sliced-ELL form; perm null: CSR only
     float4* crad;
     const uint32_t* gitems;  // grid slot -> surfel
     float4* girr;
@@ -381,8 +382,8 @@ struct MsParams {
     const float* srgb_t;
     uint32_t polls;        // poll budget of each grid barrier
 };
-// Cooperative launch (every CTA resident); capturable in a CUDA graph.
-// Returns 1, or -1 if the launch was refused.
+// A cooperative launch (every CTA resident) and the composition's; capturable
+// in a CUDA graph. Returns 2, or -1 if the first was refused.
 int launch_multi_frame(cudaStream_t st, const MsParams& p, int grid, int block);
 // Largest cooperative grid for this block size on the current device.
 int multi_frame_max_blocks(int block);
