@@ -240,4 +240,56 @@ __device__ __forceinline__ V jacobi_row(const float4* crad, const uint32_t* __re
     return irr;
 }
 
+// solve.rs:76-102 over the sliced-ELL copy: one thread per sorted position
+// (its warp is its slice), the row's links read 4 at a time as 128-bit loads
+// from the interleaved layout (a warp's loads are one contiguous 512-byte
+// block) and added in CSR order, exactly as k_jacobi; a lane stops at its own
+// row's length, so padding is never read. Outputs go to the original row.
+// The next 8 links' indices and weights are loaded while the current ones are
+// gathered and added: with few rows the kernel is one such chain per row.
+__device__ __forceinline__ V sell_row(const SellMatrix& m, const float4* crad, uint32_t sp, uint32_t len) {
+    const uint4* ip = reinterpret_cast<const uint4*>(m.idx + m.slice_off[sp >> 5] + (sp & 31u) * 4u);
+    const float4* wp = reinterpret_cast<const float4*>(m.w + m.slice_off[sp >> 5] + (sp & 31u) * 4u);
+    V irr{0.0f, 0.0f, 0.0f};
+    if (len == 0) return irr;
+    // Entries [0, 4 * ceil(len / 4)) of the row exist (padding included).
+    uint4 i0 = __ldg(ip), i1 = len > 4u ? __ldg(ip + 32) : i0;
+    float4 w0 = __ldg(wp), w1 = len > 4u ? __ldg(wp + 32) : w0;
+    for (uint32_t j = 0;; j += 8) {
+        const uint32_t left = len - j;
+        const uint4 a0 = i0, a1 = i1;
+        const float4 b0 = w0, b1 = w1;
+        ip += 64;
+        wp += 64;
+        if (left > 8u) {
+            i0 = __ldg(ip);
+            w0 = __ldg(wp);
+        }
+        if (left > 12u) {
+            i1 = __ldg(ip + 32);
+            w1 = __ldg(wp + 32);
+        }
+        if (left >= 8u) {
+            const float4 c0 = crad[a0.x], c1 = crad[a0.y], c2 = crad[a0.z], c3 = crad[a0.w], c4 = crad[a1.x],
+                         c5 = crad[a1.y], c6 = crad[a1.z], c7 = crad[a1.w];
+            irr = irr + mk4(c0) * b0.x;
+            irr = irr + mk4(c1) * b0.y;
+            irr = irr + mk4(c2) * b0.z;
+            irr = irr + mk4(c3) * b0.w;
+            irr = irr + mk4(c4) * b1.x;
+            irr = irr + mk4(c5) * b1.y;
+            irr = irr + mk4(c6) * b1.z;
+            irr = irr + mk4(c7) * b1.w;
+            if (left == 8u) return irr;
+        } else {
+            const uint32_t ia[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const float wa[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+            for (uint32_t t = 0; t < 7u; ++t)
+                if (t < left) irr = irr + mk4(crad[ia[t]]) * wa[t];
+            return irr;
+        }
+    }
+}
+
 }  // namespace ifx
