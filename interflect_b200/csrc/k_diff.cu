@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(256) k_gather_t(const uint32_t* gstarts, const
 static constexpr int kFtBlock = 256;
 __global__ void __launch_bounds__(kFtBlock) k_ft_spmv(const uint32_t* ftstarts, const uint2* ft, const float4* t,
                                                       uint32_t nc, float4* y) {
+    pdl_wait();
     __shared__ V red[kFtBlock];
     for (uint32_t c = blockIdx.x; c < nc; c += gridDim.x) {
         V a{0.0f, 0.0f, 0.0f};
@@ -319,11 +320,13 @@ __global__ void __launch_bounds__(kFtBlock) k_ft_spmv(const uint32_t* ftstarts, 
         if (threadIdx.x == 0) y[c] = f4(red[0], 0.0f);
         __syncthreads();
     }
+    pdl_trigger();
 }
 
 __global__ void k_adj_surfel(const uint32_t* cid, const float4* sp, const float4* cp, const float4* y,
                              const float4* albedo, const float4* irr_prev, uint32_t n, int first, float4* ebar,
                              float4* rhobar, float4* t) {
+    pdl_wait();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t c = cid[i];
         V b{0.0f, 0.0f, 0.0f};
@@ -339,6 +342,7 @@ __global__ void k_adj_surfel(const uint32_t* cid, const float4* sp, const float4
             rhobar[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
+    pdl_trigger();
 }
 
 // E = rho * S with S = sum_l e_l a_il: rhobar += Ebar * S.
@@ -483,14 +487,16 @@ int launch_gather_t(cudaStream_t st, const uint32_t* gstarts, const float4* gent
 
 int launch_ft_spmv(cudaStream_t st, const uint32_t* ftstarts, const uint2* ft, const float4* t, uint32_t nc,
                    float4* y) {
-    k_ft_spmv<<<nc < 8192u ? nc : 8192u, kFtBlock, 0, st>>>(ftstarts, ft, t, nc, y);
+    launch_pdl(k_ft_spmv, nc < 8192u ? nc : 8192u, kFtBlock, 0, st, ftstarts, ft, t, nc, y);
     return 1;
 }
 
 int launch_adj_surfel(cudaStream_t st, const uint32_t* cid, const float4* sp, const float4* cp, const float4* y,
                       const float4* albedo, const float4* irr_prev, uint32_t n, int first, float4* ebar,
                       float4* rhobar, float4* t) {
-    k_adj_surfel<<<grid_for(n, 256), 256, 0, st>>>(cid, sp, cp, y, albedo, irr_prev, n, first, ebar, rhobar, t);
+    // Small CTAs: 20,000 surfels leave half the SMs without one of 256.
+    launch_pdl(k_adj_surfel, grid_for(n, 128, 16), 128, 0, st, cid, sp, cp, y, albedo, irr_prev, n, first, ebar, rhobar,
+               t);
     return 1;
 }
 

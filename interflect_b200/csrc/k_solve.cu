@@ -9,14 +9,6 @@
 
 namespace ifx {
 
-// Programmatic dependent launch between the bounce kernels: a kernel starts
-// by waiting until the previous kernel in its stream has completed and its
-// writes are visible (pdl_wait), and once its main loop is done it lets the
-// next kernel be scheduled (pdl_trigger), whose CTAs then wait in their own
-// pdl_wait. Both are no-ops in a launch without the programmatic attribute.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 __device__ __forceinline__ void block_add_u64(unsigned long long v, unsigned long long* out) {
     for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(out, v);
@@ -273,24 +265,6 @@ __global__ void __launch_bounds__(kJacBlock) k_jacobi_sell(const float4* direct,
     }
     pdl_trigger();
     note_residual(dmax, ctl, it);
-}
-
-// A bounce kernel launched with the programmatic-serialization attribute:
-// the stream (or the captured graph's edge) lets it start once the previous
-// kernel has triggered, and pdl_wait orders its work after that kernel.
-template <typename... K, typename... A>
-static void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // One wave of CTAs, as many as are co-resident.

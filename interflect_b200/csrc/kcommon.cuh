@@ -188,6 +188,33 @@ struct WarpQueue {
     __device__ __forceinline__ bool empty() const { return drained && cur >= end; }
 };
 
+// Programmatic dependent launch between the kernels of a bounce, forward or
+// adjoint: a kernel starts
+// by waiting until the previous kernel in its stream has completed and its
+// writes are visible (pdl_wait), and once its main loop is done it lets the
+// next kernel be scheduled (pdl_trigger), whose CTAs then wait in their own
+// pdl_wait. Both are no-ops in a launch without the programmatic attribute.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A bounce kernel launched with the programmatic-serialization attribute:
+// the stream (or the captured graph's edge) lets it start once the previous
+// kernel has triggered, and pdl_wait orders its work after that kernel.
+template <typename... K, typename... A>
+static inline void launch_pdl(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // ------------------------------------------------------ Jacobi bounces ----
 // solve.rs:93-101: whether the solve has stopped before bounce `it`. Every
 // thread of a bounce's first phase decides the same, whether or not it sees
