@@ -82,15 +82,14 @@ __global__ void __launch_bounds__(512) k_spmm(const float4* direct, const float4
 // loads in a row before them; here it is three conflict-free reads and, as
 // the row's links pass through a buffer of the warp (index and weight, 32 at
 // a time), half a 16-byte broadcast. Each (row, rhs) still adds its links in
-// CSR order. 64 right-hand sides of 20,000 rows, 384 clusters and 2.1M links:
-// 157 -> 93 us a bounce, of which the shared-memory pipe is busy two thirds.
+// CSR order. 16 right-hand sides, 12 bounces, Cornell box of 8,000, 20,000 and
+// 60,000 surfels: 0.73 -> 0.61, 1.22 -> 1.01, 2.69 -> 1.95 ms.
 static constexpr size_t kSpmmSharedMax = 200u * 1024u;
-template <uint32_t kRhs>
+static constexpr uint32_t kRhs = 16;
 static size_t spmm_shared_bytes(uint32_t nc, int warps) {
     return (size_t)nc * 3u * kRhs * 4u + (size_t)warps * 32u * 8u;
 }
 
-template <uint32_t kRhs>
 __global__ void __launch_bounds__(1024) k_spmm_shared(const float4* direct, const float4* albedo, float4* irr,
                                                       float4* rad, uint32_t n, uint32_t R, const uint32_t* starts,
                                                       const uint32_t* idx, const float* w, const float4* crad,
@@ -156,18 +155,17 @@ __global__ void __launch_bounds__(1024) k_spmm_shared(const float4* direct, cons
     if (dmax > 0.0f) atomicMax(&res_bits[r], __float_as_uint(dmax));
 }
 
-template <uint32_t kRhs>
 static void launch_spmm_shared(cudaStream_t st, const float4* direct, const float4* albedo, float4* irr, float4* rad,
                                uint32_t n, uint32_t R, const uint32_t* starts, const uint32_t* idx, const float* w,
                                const float4* crad, uint32_t nc, const uint32_t* done, uint32_t* res_bits, int warps) {
-    const size_t sm = spmm_shared_bytes<kRhs>(nc, warps);
+    const size_t sm = spmm_shared_bytes(nc, warps);
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmm_shared<kRhs>, warps * 32, sm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spmm_shared, warps * 32, sm);
     const unsigned chunks = (R + kRhs - 1u) / kRhs;
     const unsigned wave = (unsigned)sm_count() * (unsigned)(per_sm < 1 ? 1 : per_sm);
     const unsigned rows = (unsigned)warps * (32u / kRhs), need = (n + rows - 1u) / rows;
     const unsigned gx = wave / chunks < 1u ? 1u : wave / chunks;
-    k_spmm_shared<kRhs><<<dim3(gx < need ? gx : need, chunks), warps * 32, sm, st>>>(
+    k_spmm_shared<<<dim3(gx < need ? gx : need, chunks), warps * 32, sm, st>>>(
         direct, albedo, irr, rad, n, R, starts, idx, w, crad, nc, done, res_bits);
 }
 
@@ -230,13 +228,14 @@ int launch_batched_bounce(cudaStream_t st, uint32_t n, uint32_t R, const float4*
     const uint32_t chunks = (R + 31) / 32;
     k_agg_batched<<<grid_for((unsigned long long)nc * chunks * 32ull, 256), 256, 0, st>>>(rad, sp, cp, crange,
                                                                                           members, nc, R, crad, done);
-    // Shared memory holds 32 right-hand sides of up to 530 clusters, 16 of up
-    // to 1,060; few right-hand sides leave fewer lanes empty with 16 to a row.
+    // Shared memory holds 16 right-hand sides of up to 1,060 clusters. With
+    // more right-hand sides the warps of k_spmm are many and full, and lanes
+    // whose right-hand side has converged cost it nothing: 256 of them on the
+    // Cornell box's 20,000 surfels 6.1 ms against 9.3 in chunks of 16 (64:
+    // 2.14 and 2.24; 24: 1.36 and 1.41).
     const int warps = 4 * rows_per_block_warps < 32 ? 4 * rows_per_block_warps : 32;
-    if (R > 16u && spmm_shared_bytes<32>(nc, warps) <= kSpmmSharedMax) {
-        launch_spmm_shared<32>(st, direct, albedo, irr, rad, n, R, starts, idx, w, crad, nc, done, res_bits, warps);
-    } else if (spmm_shared_bytes<16>(nc, warps) <= kSpmmSharedMax) {
-        launch_spmm_shared<16>(st, direct, albedo, irr, rad, n, R, starts, idx, w, crad, nc, done, res_bits, warps);
+    if (R <= kRhs && spmm_shared_bytes(nc, warps) <= kSpmmSharedMax) {
+        launch_spmm_shared(st, direct, albedo, irr, rad, n, R, starts, idx, w, crad, nc, done, res_bits, warps);
     } else {
         const int block = 32 * rows_per_block_warps;
         unsigned gx = grid_for((unsigned long long)n * 32ull, block, 4);
@@ -249,8 +248,7 @@ int launch_batched_bounce(cudaStream_t st, uint32_t n, uint32_t R, const float4*
 }
 
 void configure_batch_kernels() {
-    cudaFuncSetAttribute(k_spmm_shared<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpmmSharedMax);
-    cudaFuncSetAttribute(k_spmm_shared<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpmmSharedMax);
+    cudaFuncSetAttribute(k_spmm_shared, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpmmSharedMax);
 }
 
 }  // namespace ifx

@@ -166,27 +166,20 @@ __device__ __forceinline__ void load8(const void* p, uint32_t v[8]) {
 // of a warp lie in 32 places, so each of its loads is 32 cache lines' worth of
 // L1 cycles however little it takes: links come eight at a time in 256-bit
 // loads of whole sectors, from the aligned place at or before the row's first
-// link to the one at or after its last, those of the neighbouring rows masked;
-// and the cluster radiosities, 32 lines to a gather, come from a copy in
-// shared memory where they fit (kShared), some 10 cycles. 800,000 rows of 97
-// links: 3.11 -> 2.33 ms for 10 bounces, 2.7 TB/s of the arrays; 150,000 such
-// rows, which L2 holds, 0.73 -> 0.65 ms for 12. (Tiles of 32 rows copied to
-// shared memory by cp.async first, so that every load is coalesced, took 2.78
-// and 0.82 ms: the shared-memory pipe then moves each link three times.)
-template <bool kShared>
+// link to the one at or after its last, those of the neighbouring rows masked.
+// The stress scene's 1M rows and 109M links: 5.78 -> 4.76 ms for 14 bounces;
+// as many rows and links drawn at random, 3.89 -> 3.39 ms. (With the cluster
+// radiosities in shared memory the random matrix took 2.83 ms but the scene's
+// 9.31: its rows differ in length and see the same clusters, which L1 serves
+// in few lines. Tiles of 32 rows copied to shared memory first: 1.2 times the
+// shared form on the random one.)
 __global__ void __launch_bounds__(kJacBlock) k_jacobi_wide(const float4* direct, const float4* albedo,
                                                             float4* irr_out, float4* rad, uint32_t n,
                                                             const uint32_t* starts, const uint32_t* idx,
-                                                            const float* w, const float4* __restrict__ crad_g,
-                                                            uint32_t nc, SolveCtl* ctl, uint32_t it) {
-    extern __shared__ __align__(16) uint8_t wide_smem[];
+                                                            const float* w, const float4* __restrict__ crad,
+                                                            SolveCtl* ctl, uint32_t it) {
     pdl_wait();
     if (ctl->done) return;
-    float4* cs = reinterpret_cast<float4*>(wide_smem);
-    if constexpr (kShared) {
-        for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x) cs[c] = crad_g[c];
-        __syncthreads();
-    }
     const uint32_t total = starts[n];
     float dmax = 0.0f;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -207,14 +200,14 @@ __global__ void __launch_bounds__(kJacBlock) k_jacobi_wide(const float4* direct,
             if (k >= s && k + 8u <= e) {
                 float4 c[8];
 #pragma unroll
-                for (int t = 0; t < 8; ++t) c[t] = kShared ? cs[a[t]] : crad_g[a[t]];
+                for (int t = 0; t < 8; ++t) c[t] = crad[a[t]];
 #pragma unroll
                 for (int t = 0; t < 8; ++t) irr = irr + mk4(c[t]) * __uint_as_float(b[t]);
             } else {
 #pragma unroll
                 for (uint32_t t = 0; t < 8u; ++t)
                     if (k + t >= s && k + t < e)
-                        irr = irr + mk4(kShared ? cs[a[t]] : crad_g[a[t]]) * __uint_as_float(b[t]);
+                        irr = irr + mk4(crad[a[t]]) * __uint_as_float(b[t]);
             }
         }
         dmax = fmaxf(dmax, row_update(direct, albedo, irr_out, rad, i, irr));
@@ -294,12 +287,8 @@ void launch_solve_bounce(cudaStream_t st, SurfelArrays s, uint32_t n, const floa
             launch_pdl(k_jacobi_sell<false>, grid_for(n, kFewRowsBlock, 16), kFewRowsBlock, 0, st, direct, albedo, s.irr,
                        s.rad, n, *sell, crad, nc, ctl, it);
     } else if (n >= kWideRows && (((uintptr_t)idx | (uintptr_t)w) & 31u) == 0) {
-        if (cbytes <= kSharedRadMax)
-            launch_pdl(k_jacobi_wide<true>, wave_grid(k_jacobi_wide<true>, kJacBlock, cbytes, n), kJacBlock, cbytes, st,
-                       direct, albedo, s.irr, s.rad, n, starts, idx, w, crad, nc, ctl, it);
-        else
-            launch_pdl(k_jacobi_wide<false>, grid_for(n, kJacBlock), kJacBlock, 0, st, direct, albedo, s.irr, s.rad, n,
-                       starts, idx, w, crad, nc, ctl, it);
+        launch_pdl(k_jacobi_wide, grid_for(n, kJacBlock), kJacBlock, 0, st, direct, albedo, s.irr, s.rad, n, starts,
+                   idx, w, crad, ctl, it);
     } else {
         const int vec = (((uintptr_t)idx | (uintptr_t)w) & 15u) == 0 ? 1 : 0;
         launch_pdl(k_jacobi, grid_for(n, kJacBlock), kJacBlock, 0, st, direct, albedo, s.irr, s.rad, n, starts, idx, w,
@@ -392,7 +381,6 @@ int launch_sell_fill(cudaStream_t st, const uint32_t* starts, const uint32_t* id
 // Their own limits, which need no context (ifx_solve_noalloc has none).
 void configure_bounce_kernels() {
     cudaFuncSetAttribute(k_jacobi_sell<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedRadMax);
-    cudaFuncSetAttribute(k_jacobi_wide<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedRadMax);
 }
 
 void configure_solve_kernels(int max_dyn_smem) {

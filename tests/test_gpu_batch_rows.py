@@ -1,6 +1,5 @@
-"""The batched solve's row kernels: right-hand sides 32 or 16 to a row from
-shared memory, or from global memory, by the cluster count (at most 530, at
-most 1,060, above) and the batch size. Every right-hand side must equal its
+"""The batched solve's row kernels: up to 16 right-hand sides from shared
+memory where the clusters fit it (at most 1,060), else from global memory. Every right-hand side must equal its
 own solve to the bit, whichever runs."""
 import numpy as np
 import pytest

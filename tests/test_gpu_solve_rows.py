@@ -1,7 +1,6 @@
 """The device-buffer solve's row kernels against the same f32 sums formed by
 numpy in CSR order: from 49,152 rows on links are read eight at a time from
-aligned places, with the cluster radiosities in shared memory up to 4,096
-clusters. Rows of 0, 1, 31, 32, 33, 64, 65 and other lengths, at every alignment, and
+aligned places. Rows of 0, 1, 31, 32, 33, 64, 65 and other lengths, at every alignment, and
 row counts around the switch and off a warp's multiple. Products and sums
 round the same way, so the results are equal to the bit."""
 import numpy as np
