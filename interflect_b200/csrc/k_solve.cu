@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(kJacBlock) k_jacobi(const float4* direct, cons
     note_residual(dmax, ctl, it);
 }
 
-// Many rows: from here on they fill the GPU's warps. The wide kernel's line is
-// lower where k_jacobi's loads bind and higher where its shorter chain per link
-// does (33,000 rows of 32 links, 9 bounces: 168 us wide, 159 us not; 60,000
-// rows of 97 links: 311 and 323 us).
+// Many rows: from here on they fill the GPU's warps. At the wide kernel's line
+// the two forms are equal within 2% (50,000 and 60,000 rows of 97 links, 8 and 9
+// bounces: 291 and 307 us wide, 286 and 310 us with 16-byte loads and three
+// launches a bounce); below it k_jacobi's shorter chain per link wins.
 static constexpr uint32_t kManyRows = 65536, kWideRows = 49152;
 // Cluster radiosities gathered from shared memory: up to 4,096 clusters. Few
 // rows take as long as the longest one's chain of gathers, each kernel with a
