@@ -26,6 +26,16 @@ static constexpr uint32_t kFlagDone = kPixDone;
 static constexpr uint32_t kFlagEmit = kPixEmit;
 static constexpr uint32_t kMatMask = kPixMatMask;
 
+// Whether a pass before this one left early (a staging wait ran out, which sets
+// the status word that all passes of a frame share). Its pixels' hits were then
+// never written, and what indexes materials or lights by them must leave too:
+// k_setup and k_compose, the other passes use them as coordinates only. Every
+// pass precedes its readers on their stream, and the CTA decides as one; this
+// is also its barrier.
+__device__ __forceinline__ bool earlier_kernel_left(const ShadeParams& P) {
+    return __syncthreads_or(*(volatile const uint32_t*)P.status != 0u) != 0;
+}
+
 // ------------------------------------------------------------ kernels ----
 // Camera rays: trace.rs:27-58 from the eye (main.rs:261), pixels taken in
 // 8 x 4 tiles (pixorder.h). hn1 keeps the march's step count in x until
@@ -77,7 +87,7 @@ __global__ void __launch_bounds__(128) k_setup(ShadeParams P) {
     C cnt;
     __shared__ float t8[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) t8[i] = P.srgb_t[i];
-    __syncthreads();
+    if (earlier_kernel_left(P)) return;
     const uint32_t total = P.w * P.h;
     const V org{P.cam.origin[0], P.cam.origin[1], P.cam.origin[2]};
     const bool tonemapped = P.mode <= 2;
@@ -271,7 +281,7 @@ __global__ void __launch_bounds__(128, 8) k_compose(ShadeParams P) {
     C cnt;
     __shared__ float t8[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) t8[i] = P.srgb_t[i];
-    __syncthreads();
+    if (earlier_kernel_left(P)) return;
     const uint32_t end = P.pix1 ? P.pix1 : P.w * P.h;
     const GatherView g = gview(P.grid);
     for (uint32_t pix = P.pix0 + blockIdx.x * blockDim.x + threadIdx.x; pix < end; pix += gridDim.x * blockDim.x)
