@@ -671,14 +671,18 @@ __device__ __forceinline__ float scene_dist(const SceneView& sv, V p, C& cnt) {
 // kUnion = false walks each lane's own mask instead, for warps whose lanes are
 // in unrelated places (the path tracer's states: 39.2 -> 35.0 ms; the product
 // frame's coherent rays, the other way: 5.50 -> 5.88 ms).
+// in_grid (nullable) receives whether an active lane's p lies in the grid, which
+// never holds without one.
 template <bool kDistOnly, bool kUnion = true, class C>
-__device__ __forceinline__ DistHit dist_warp(const SceneView& sv, V p, bool active, C& cnt) {
+__device__ __forceinline__ DistHit dist_warp(const SceneView& sv, V p, bool active, C& cnt, bool* in_grid = nullptr) {
+    if (in_grid) *in_grid = false;
     if (active) cnt.add(CN_SDF);
     if constexpr (sizeof(C) == 1) {
         if (sv.og.mode != kOgOff) {
             uint32_t cell = 0;
             bool coarse = false;
             bool ok = active && og_cell(sv.og, p.x, p.y, p.z, cell, coarse);
+            if (in_grid) *in_grid = ok;
             OgBest b(coarse ? sv.og.coarse.delta : sv.og.fine.delta);
             if (C::kTree3 || sv.og.mode == kOgMask) {
                 uint32_t m = ok ? __ldg(&sv.og.mask[cell]) : 0u;
@@ -796,7 +800,8 @@ __device__ __forceinline__ bool cone_above(float h, float ph, float t, float k, 
 // is at least 0.12 (so the march advances exactly that, and neither stops nor
 // hits), and the cone term cannot lower res. They are taken without a query;
 // the distance after them is not known. Returns true when the march has
-// ended.
+// ended. Only for marches inside the grid (objgrid.h, og_open_first): farther
+// out coordinates round by more than delta allows for.
 __device__ __forceinline__ bool open_steps(ShadowRay& s, float h, float delta) {
     for (float lower = og_open_first(h, delta); lower >= kOpenStep && cone_cannot_lower(lower, s.t, s.k, s.res);
          lower = og_open_next(lower)) {
@@ -818,7 +823,8 @@ template <class C>
 __device__ __forceinline__ bool shadow_step_w(const SceneView& sv, ShadowRay& s, bool active, float& vis, C& cnt) {
     constexpr bool kSkips = sizeof(C) == 1;
     const bool back = kSkips && s.mode == kPhBack;
-    float h = dist_warp<true>(sv, s.ro + s.rd * (back ? s.tp : s.t), active, cnt).d;
+    bool in_grid;
+    float h = dist_warp<true>(sv, s.ro + s.rd * (back ? s.tp : s.t), active, cnt, &in_grid).d;
     if (!active) return false;
     if (back) {
         // The previous distance, now known, for the step whose own is in ph.
@@ -860,7 +866,7 @@ __device__ __forceinline__ bool shadow_step_w(const SceneView& sv, ShadowRay& s,
     s.ph = h;
     s.t += clampr(h, 0.006f, 0.12f);
     if (!(s.steps < kShadowSteps && s.t < s.tmax) ||
-        (kSkips && sv.og.mode != kOgOff && open_steps(s, h, sv.og.coarse.delta))) {
+        (kSkips && in_grid && open_steps(s, h, sv.og.coarse.delta))) {
         vis = clampr(s.res, 0.0f, 1.0f);
         return true;
     }

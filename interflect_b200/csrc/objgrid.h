@@ -197,7 +197,12 @@ IFX_OG_FN bool og_exact_box(float d1, float d2, float v1, bool dist_only) {
 
 // What a distance h at one point of a cone-shadow march says of the distance
 // one 0.12 step on (rounding of the step, the position and h included), and
-// what that says of the step after.
+// what that says of the step after. The point is one of the grid, or one step
+// from one: h is then no more than the distance from there to the objects, so
+// that the points it speaks of lie within three times the coarse level's
+// coordinates, and delta (the coarse level's) holds their rounding some ten
+// times over. Outside the grid a coordinate can be as large as the caller
+// likes, and nothing follows from h.
 static constexpr float kOpenStep = 0.12f;
 IFX_OG_FN float og_open_first(float h, float delta) { return h - 0.12002f - 4.0f * delta; }
 IFX_OG_FN float og_open_next(float lower) { return lower - 0.12002f; }
