@@ -636,7 +636,12 @@ static int objgrid_build(ifx_ctx* ctx, const std::vector<uint8_t>& blob) {
     // everything. (And at 1e9 squares of lengths are still far from overflow:
     // no distance is NaN.)
     if (!(scale < 1e9) || !(diag < 1e9) || !(side > 0.0) || !(g.fine.delta <= 0.25 * side) || !(g.coarse.delta <= 0.25 * side2)) return IFX_OK;
-    ENSURE(ctx->og_cells, ncells * (masks ? 4 : 16));
+    // The grid never changes a result, so a scene whose grid finds no memory
+    // goes without one.
+    if (ensure(ctx, ctx->og_cells, ncells * (masks ? 4 : 16)) != IFX_OK) {
+        ctx->err.clear();
+        return IFX_OK;
+    }
     g.mode = masks ? kOgMask : kOgList;
     g.id_bits = nobj <= kOgKeyObjects ? 12 : 16;
     uint32_t* mask = masks ? (uint32_t*)ctx->og_cells.p : nullptr;
