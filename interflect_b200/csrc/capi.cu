@@ -682,13 +682,19 @@ extern "C" int ifx_scene_upload(ifx_ctx* ctx, const ifx_scene* scene) {
         if (maxd + 2 > 64) return fail(ctx, IFX_ERR_LIMIT, "BVH deeper than the 64-entry traversal stack");
     }
     std::vector<uint8_t> blob = flatten_scene(s);
+    // From here on the context holds parts of both scenes: if a step below
+    // fails it has none, until an upload succeeds.
+    ctx->has_scene = false;
+    ctx->has_transfer = false;
+    ctx->has_grid = false;
+    ctx->blobref.tree3 = 0;
+    frame_changed(ctx);
     ENSURE(ctx->blob, blob.size());
     CK(cudaMemcpyAsync(ctx->blob.p, blob.data(), blob.size(), cudaMemcpyHostToDevice, ctx->st));
     std::vector<float4> le = light_emissions(s);
     ENSURE(ctx->lemit, le.size() * 16);
     if (!le.empty()) CK(cudaMemcpyAsync(ctx->lemit.p, le.data(), le.size() * 16, cudaMemcpyHostToDevice, ctx->st));
     ctx->nl = (uint32_t)le.size();
-    frame_changed(ctx);
     ctx->scene = s;
     ctx->blobref.ptr = (const uint8_t*)ctx->blob.p;
     ctx->blobref.bytes = (uint32_t)blob.size();
@@ -706,9 +712,6 @@ extern "C" int ifx_scene_upload(ifx_ctx* ctx, const ifx_scene* scene) {
     }
     CK(cudaStreamSynchronize(ctx->st));
     ctx->has_scene = true;
-    ctx->has_transfer = false;
-    ctx->has_grid = false;
-    frame_changed(ctx);
     return IFX_OK;
 }
 
