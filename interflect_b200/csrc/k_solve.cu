@@ -185,9 +185,9 @@ __global__ void __launch_bounds__(kJacBlock) k_jacobi_wide(const float4* direct,
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t s = starts[i], e = starts[i + 1];
         V irr{0.0f, 0.0f, 0.0f};
-        for (uint32_t k = s & ~7u; k < e; k += 8u) {
+        for (uint32_t k = s & ~(kSpan - 1u); k < e; k = span_next(k, e)) {
             uint32_t a[8], b[8];
-            if (k + 8u <= total) {
+            if (span_full(k, total)) {
                 load8(idx + k, a);
                 load8(w + k, b);
             } else {  // the last links of the matrix
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kJacBlock) k_jacobi_wide(const float4* direct,
                     b[t] = k + t < total ? __float_as_uint(__ldg(&w[k + t])) : 0u;
                 }
             }
-            if (k >= s && k + 8u <= e) {
+            if (k >= s && span_full(k, e)) {
                 float4 c[8];
 #pragma unroll
                 for (int t = 0; t < 8; ++t) c[t] = crad[a[t]];

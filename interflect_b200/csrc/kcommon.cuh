@@ -4,6 +4,7 @@
 
 #include "device.cuh"
 #include "kernels.h"
+#include "rowspan.h"
 
 namespace ifx {
 
@@ -246,7 +247,7 @@ __device__ __forceinline__ V jacobi_row(const float4* crad, const uint32_t* __re
     V irr{0.0f, 0.0f, 0.0f};
     if (vec) {
         for (; k < e && (k & 3u); ++k) irr = irr + mk4(crad[__ldg(&idx[k])]) * __ldg(&w[k]);
-        for (; k + 8 <= e; k += 8) {
+        for (; span_full(k, e); k += kSpan) {
             const uint4 i0 = __ldg(reinterpret_cast<const uint4*>(idx + k));
             const uint4 i1 = __ldg(reinterpret_cast<const uint4*>(idx + k + 4));
             const float4 w0 = __ldg(reinterpret_cast<const float4*>(w + k));
