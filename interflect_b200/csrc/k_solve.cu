@@ -378,16 +378,11 @@ int launch_sell_fill(cudaStream_t st, const uint32_t* starts, const uint32_t* id
     return 1;
 }
 
-// Their own limits, which need no context (ifx_solve_noalloc has none).
-void configure_bounce_kernels() {
-    cudaFuncSetAttribute(k_jacobi_sell<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedRadMax);
-}
-
 void configure_solve_kernels(int max_dyn_smem) {
     cudaFuncSetAttribute(k_light_surfels<NoCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
     cudaFuncSetAttribute(k_light_surfels<NoCount3>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
     cudaFuncSetAttribute(k_light_surfels<Counts>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    configure_bounce_kernels();
+    cudaFuncSetAttribute(k_jacobi_sell<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedRadMax);
 }
 
 }  // namespace ifx

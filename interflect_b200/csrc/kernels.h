@@ -392,7 +392,6 @@ int multi_frame_max_blocks(int block);
 void configure_surfel_kernels(int max_dyn_smem);
 void configure_transfer_kernels(int max_dyn_smem);
 void configure_solve_kernels(int max_dyn_smem);
-void configure_bounce_kernels();
 void configure_batch_kernels();
 void configure_shade_kernels(int max_dyn_smem);
 void configure_diff_kernels(int max_dyn_smem);

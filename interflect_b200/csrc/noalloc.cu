@@ -43,7 +43,6 @@ int scratch_for(int device, void** out, char* err, size_t errlen) {
             return IFX_ERR_CUDA;
         }
         g_addr[device] = p;
-        ifx::configure_bounce_kernels();  // per device, like the address
     }
     *out = g_addr[device];
     return IFX_OK;
