@@ -67,7 +67,9 @@ __global__ void __launch_bounds__(256) k_multi_frame(MsParams M) {
     // from the residuals, CTA 0 also notes the scenes' statistics. `it` runs
     // one past the last bounce for that.
     for (uint32_t it = 0; it <= M.max_bounces; ++it) {
-        auto stopped = [&](int s) { return solve_stopped(M.ctl[s], it, 0) || it >= sc[s].max_bounces; };
+        auto stopped = [&](int s) {
+            return solve_stopped<volatile SolveCtl>(M.ctl[s], it, 0) || it >= sc[s].max_bounces;
+        };
         int live = 0;
         for (int s = (int)threadIdx.x; s < M.S; s += (int)blockDim.x) {
             const bool stop = stopped(s);
