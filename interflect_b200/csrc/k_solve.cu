@@ -142,11 +142,19 @@ __global__ void __launch_bounds__(kJacBlock) k_jacobi(const float4* direct, cons
     note_residual(dmax, ctl, it);
 }
 
-// Many rows: from here on they fill the GPU's warps. At the wide kernel's line
-// the two forms are equal within 2% (50,000 and 60,000 rows of 97 links, 8 and 9
-// bounces: 291 and 307 us wide, 286 and 310 us with 16-byte loads and three
-// launches a bounce); below it k_jacobi's shorter chain per link wins.
-static constexpr uint32_t kManyRows = 65536, kWideRows = 49152;
+// Many rows: from here on they fill the GPU's warps.
+static constexpr uint32_t kManyRows = 65536;
+// The wide row walk: from so many rows on, and of so many links each in the
+// mean. Fewer rows are one chain per link, which its masked ends lengthen, and
+// the ends are a larger part of shorter rows. 8 bounces of scenes' transfers
+// with 16-byte loads and wide, in us, by rows and mean links:
+//            20,000     50,000     100,000    250,000      1,000,000
+//    19   132, 158   158, 169   210, 221   422, 434   1,455, 1,530
+//    35   166, 185   185, 194   244, 251   494, 505
+//    57   211, 248   233, 238   303, 305   743, 708
+//   109   310, 361   359, 344   567, 494   1,240, 1,137   3,830, 3,667
+// and a Cornell box's 60,000 rows of 48 links 223, 231, of 119 links 345, 331.
+static constexpr uint32_t kWideRows = 49152, kWideLinks = 64;
 // Cluster radiosities gathered from shared memory: up to 4,096 clusters. Few
 // rows take as long as the longest one's chain of gathers, each kernel with a
 // cold L1: small CTAs spread them over the SMs, and up to 1,024 clusters a copy
@@ -162,7 +170,7 @@ __device__ __forceinline__ void load8(const void* p, uint32_t v[8]) {
         : "l"(p));
 }
 
-// The same where idx and w are 32-byte aligned, as allocations are. The rows
+// A row's sum where idx and w are 32-byte aligned, as allocations are. The rows
 // of a warp lie in 32 places, so each of its loads is 32 cache lines' worth of
 // L1 cycles however little it takes: links come eight at a time in 256-bit
 // loads of whole sectors, from the aligned place at or before the row's first
@@ -173,6 +181,38 @@ __device__ __forceinline__ void load8(const void* p, uint32_t v[8]) {
 // 9.31: its rows differ in length and see the same clusters, which L1 serves
 // in few lines. Tiles of 32 rows copied to shared memory first: 1.2 times the
 // shared form on the random one.)
+__device__ __forceinline__ V wide_row(const float4* __restrict__ crad, const uint32_t* idx, const float* w, uint32_t s,
+                                      uint32_t e, uint32_t total) {
+    V irr{0.0f, 0.0f, 0.0f};
+    for (uint32_t k = s & ~(kSpan - 1u); k < e; k = span_next(k, e)) {
+        uint32_t a[8], b[8];
+        if (span_full(k, total)) {
+            load8(idx + k, a);
+            load8(w + k, b);
+        } else {  // the last links of the matrix
+#pragma unroll
+            for (uint32_t t = 0; t < 8u; ++t) {
+                a[t] = k + t < total ? __ldg(&idx[k + t]) : 0u;
+                b[t] = k + t < total ? __float_as_uint(__ldg(&w[k + t])) : 0u;
+            }
+        }
+        if (k >= s && span_full(k, e)) {
+            float4 c[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) c[t] = crad[a[t]];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) irr = irr + mk4(c[t]) * __uint_as_float(b[t]);
+        } else {
+#pragma unroll
+            for (uint32_t t = 0; t < 8u; ++t)
+                if (k + t >= s && k + t < e) irr = irr + mk4(crad[a[t]]) * __uint_as_float(b[t]);
+        }
+    }
+    return irr;
+}
+
+// The mean row length is known on the device alone, where the caller's arrays
+// are: every thread decides alike by the number of links.
 __global__ void __launch_bounds__(kJacBlock) k_jacobi_wide(const float4* direct, const float4* albedo,
                                                             float4* irr_out, float4* rad, uint32_t n,
                                                             const uint32_t* starts, const uint32_t* idx,
@@ -181,35 +221,11 @@ __global__ void __launch_bounds__(kJacBlock) k_jacobi_wide(const float4* direct,
     pdl_wait();
     if (ctl->done) return;
     const uint32_t total = starts[n];
+    const bool wide = total >= (unsigned long long)n * kWideLinks;
     float dmax = 0.0f;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t s = starts[i], e = starts[i + 1];
-        V irr{0.0f, 0.0f, 0.0f};
-        for (uint32_t k = s & ~(kSpan - 1u); k < e; k = span_next(k, e)) {
-            uint32_t a[8], b[8];
-            if (span_full(k, total)) {
-                load8(idx + k, a);
-                load8(w + k, b);
-            } else {  // the last links of the matrix
-#pragma unroll
-                for (uint32_t t = 0; t < 8u; ++t) {
-                    a[t] = k + t < total ? __ldg(&idx[k + t]) : 0u;
-                    b[t] = k + t < total ? __float_as_uint(__ldg(&w[k + t])) : 0u;
-                }
-            }
-            if (k >= s && span_full(k, e)) {
-                float4 c[8];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) c[t] = crad[a[t]];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) irr = irr + mk4(c[t]) * __uint_as_float(b[t]);
-            } else {
-#pragma unroll
-                for (uint32_t t = 0; t < 8u; ++t)
-                    if (k + t >= s && k + t < e)
-                        irr = irr + mk4(crad[a[t]]) * __uint_as_float(b[t]);
-            }
-        }
+        const V irr = wide ? wide_row(crad, idx, w, s, e, total) : jacobi_row(crad, idx, w, s, e, 1);
         dmax = fmaxf(dmax, row_update(direct, albedo, irr_out, rad, i, irr));
     }
     pdl_trigger();
