@@ -1063,8 +1063,13 @@ static int sell_build(ifx_ctx* ctx, uint64_t longest) {
     ctx->launches += (uint64_t)launch_sell_sizes(ctx->st, len, n, sizes);
     CKL();
     CUB([&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveSum(t, b, sizes, off, (int)ns + 1, ctx->st); });
-    ENSURE(ctx->sell_idx, (size_t)bound * 4);
-    ENSURE(ctx->sell_w, (size_t)bound * 4);
+    // The copy is as large as the transfer and never changes a result: where
+    // there is no memory for it the solve reads the CSR arrays.
+    if (ensure(ctx, ctx->sell_idx, (size_t)bound * 4) != IFX_OK || ensure(ctx, ctx->sell_w, (size_t)bound * 4) != IFX_OK) {
+        free_buf(ctx->sell_idx);
+        ctx->err.clear();
+        return IFX_OK;
+    }
     ctx->launches += (uint64_t)launch_sell_fill(ctx->st, (const uint32_t*)ctx->starts.p, (const uint32_t*)ctx->idx.p,
                                                 (const float*)ctx->w.p, n, perm, len, off,
                                                 (uint32_t*)ctx->sell_idx.p, (float*)ctx->sell_w.p);
