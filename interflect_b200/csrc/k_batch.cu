@@ -228,8 +228,9 @@ int launch_batched_bounce(cudaStream_t st, uint32_t n, uint32_t R, const float4*
     const uint32_t chunks = (R + 31) / 32;
     k_agg_batched<<<grid_for((unsigned long long)nc * chunks * 32ull, 256), 256, 0, st>>>(rad, sp, cp, crange,
                                                                                           members, nc, R, crad, done);
-    // Shared memory holds 16 right-hand sides of up to 1,060 clusters. With
-    // more right-hand sides the warps of k_spmm are many and full, and lanes
+    // Shared memory holds 16 right-hand sides of up to 1,024 clusters (192 bytes
+    // each, beside 256 a warp: 1,056 at the smallest launch shape). With more
+    // right-hand sides the warps of k_spmm are many and full, and lanes
     // whose right-hand side has converged cost it nothing: 256 of them on the
     // Cornell box's 20,000 surfels 6.1 ms against 9.3 in chunks of 16 (64:
     // 2.14 and 2.24; 24: 1.36 and 1.41).
