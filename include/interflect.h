@@ -104,10 +104,15 @@ typedef struct ifx_solve_stats {
 typedef struct ifx_stats {
     uint64_t kernel_launches;  /* kernels this context has launched so far */
     float ms_transfer, ms_light, ms_solve, ms_grid, ms_shade; /* CUDA-event times of the last call of each stage */
-    float ms_visibility, ms_closure; /* CUDA-event times of the last visibility and closure kernels */
+    float ms_visibility, ms_closure; /* CUDA-event times of the last visibility and closure kernels,
+                                      * which run beside each other */
     /* CUDA-event times of the last frame's shading kernels: camera rays,
      * shadow cones of the camera hits, mirror rays, shadow cones of the
-     * mirror hits, and the rest (setup, mirror setup, compose + encode). */
+     * mirror hits, and the rest (setup, mirror setup, compose + encode). A
+     * frame runs kernels beside one another, and each time is then that of the
+     * kernel with its neighbours: in ifx_render_frame with GI the camera hits'
+     * shadow cones beside the mirror passes, in ifx_frame all of these beside
+     * the GI stages. */
     float ms_primary, ms_shadow, ms_reflect, ms_shadow2, ms_shade_other;
     /* CUDA-event times of the last differentiable forward and backward. */
     float ms_diff_forward, ms_diff_backward;

@@ -1180,7 +1180,7 @@ static int transfer_build(ifx_ctx* ctx, int cluster_res, ifx_transfer_info* out,
     CK(cudaEventRecord(ctx->tev[1], ctx->st3));
     const uint32_t* vorder = nullptr;
     if (ncand > 1 && ncand <= 0x7fffffffull) {
-        // 32-bit keys where they hold (nc + 1)^2: every scene of up to 65,534
+        // 32-bit keys where they hold nc (nc + 2): every scene of up to 65,535
         // clusters. (64-bit keys moved 1.5 times the bytes.)
         const unsigned long long kmax = (unsigned long long)nc * (nc + 1ull) + nc;
         const bool narrow = kmax <= 0xffffffffull;

@@ -1,8 +1,8 @@
 // The object grid: for each cell of a uniform grid over the scene, the stored
 // objects that can be nearest to a point of the cell. A distance query then
-// evaluates one or two objects (1.2 listed per cell in the product and Cornell
-// scenes, 1.9 in the 512-object stress scene) instead of traversing the BVH,
-// and answers the reference's traversal exactly or says that it cannot.
+// evaluates one or two objects (over the CPU check's queries in the grid 1.2 are
+// listed in the product and Cornell scenes, 1.5 in the 512-object stress scene)
+// instead of traversing the BVH, and answers the reference's traversal exactly or says that it cannot.
 //
 // The rules, shared by the kernels and by the CPU check against the
 // reference's traversal (tests/cpp/objgrid_check.cpp):
