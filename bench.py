@@ -50,7 +50,7 @@ WORKLOADS = {
                  "transfer, one CSR SpMM solve, 12 bounces max"),
     "c4_multi": ("interflect_b200/scenes/gen_scenes.py:packed_scenes",
                  "64 stress-style scenes (8-128 primitives, 2k-50k surfels, 256^2-1024^2 films, 24 bounces max) "
-                 "solved and shaded in one persistent cooperative launch replayed from a CUDA graph"),
+                 "solved in one persistent cooperative launch and composed in a second, replayed from a CUDA graph"),
     "solve_hbm": ("interflect_b200/scenes/c3_stress.rad",
                   "Jacobi solve alone on a stress-sized transfer: the stress scene's 1M surfels and clusters with "
                   "a synthetic CSR of 109 links per row (109M links), 24 bounces max; the HBM-bound stage"),
@@ -273,8 +273,9 @@ def run_ours(args, world, rank, local) -> dict | None:
     barrier(world)
 
     # Per-stage and per-kernel times (and the roofline's kernel duration) come
-    # from frames made of the stage calls, where no kernel shares the GPU with
-    # another stream.
+    # from frames made of the stage calls. The closure runs beside the
+    # visibility there, and the mirror passes beside the primary shadow rays:
+    # these four times are contended ones.
     staged_ms = 0.0
     kms = {k: [] for k in KERNEL_NAMES}
     stage = {"transfer": [], "light": [], "solve": [], "grid": [], "shade": []}
@@ -467,8 +468,8 @@ def run_batch(args, world, rank, local) -> dict | None:
         "plain_loop": {"value": loop_rate, "unit": "solves/s", "rhs_timed": loop_n,
                        "speedup": value / loop_rate,
                        "contains": "per right-hand side: ifx_surfels_set_emission (E uploaded from host memory, "
-                                   "direct = rad = E, irr = 0) then ifx_solve (one cooperative launch, its stop "
-                                   "rule read back by the host), i.e. the single-RHS API a caller would loop over"},
+                                   "direct = rad = E, irr = 0) then ifx_solve (one graph launch of all bounces, its "
+                                   "stop rule read back by the host), i.e. the single-RHS API a caller would loop over"},
         "roofline": {"kernel": "k_agg_batched + k_spmm + k_bounce_end_batched", "bound": "hbm", "achieved": gbs,
                      "peak": peak, "unit": "GB/s", "frac": gbs / peak, "traffic": None,
                      "bytes_per_step": nbytes, "peak_source": peak_src,
@@ -585,7 +586,7 @@ def run_multi(args, world, rank, local) -> dict | None:
         "scene_preparation_s": prep_s,
         "e2e": {"value": S / (e_max / 1e3), "unit": "scenes/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": d2h,
                 "includes": "graph replay and every scene's sRGB frame downloaded to host"},
-        "gpu_launches": args.steps,
+        "gpu_launches": 2 * args.steps,  # per replay the solve and the composition
         "clocks": clocks,
     }
 
