@@ -1649,7 +1649,7 @@ static int batched_run(ifx_ctx* ctx, uint32_t R, const float* E, uint32_t max_bo
                 (float4*)ctx->birr.p, (float4*)ctx->brad.p, (const float4*)ctx->cp.p, (const uint2*)ctx->crange.p,
                 (const uint32_t*)ctx->members.p, nc, (const uint32_t*)ctx->starts.p, (const uint32_t*)ctx->idx.p,
                 (const float*)ctx->w.p, (float4*)ctx->bcrad.p, (uint32_t*)ctx->bdone.p, (uint32_t*)ctx->biters.p,
-                (uint32_t*)ctx->bres.p, (uint32_t*)ctx->blast.p, it, warps);
+                (uint32_t*)ctx->bres.p, (uint32_t*)ctx->blast.p, it, warps, ctx->links);
         CKL();
         CK(cudaMemcpyAsync(done.data(), ctx->bdone.p, (size_t)R * 4, cudaMemcpyDeviceToHost, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));

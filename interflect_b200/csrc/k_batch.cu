@@ -155,6 +155,28 @@ __global__ void __launch_bounds__(1024) k_spmm_shared(const float4* direct, cons
     if (dmax > 0.0f) atomicMax(&res_bits[r], __float_as_uint(dmax));
 }
 
+// Whether k_spmm_shared is the faster one for a matrix of so many rows and
+// links. A CTA first copies all clusters, and a warp passes through its link
+// buffer once more for each 16 links of a row: that pays from 32 links a row
+// on, or half a million in all. Up to 32 warps a SM (from 530 clusters on one
+// CTA) wait for a row's own loads and stores, which hides less than k_spmm's 64
+// where these come from HBM: there from 60 links a row on. 8 bounces with
+// k_spmm and shared, in us, by rows, clusters, mean links and right-hand sides:
+//   6,000 x 779   117 links  16    472, 363      2,000 x 1,000   15 links  16    164, 193
+//  45,000 x 809   119 links   2  1,664, 1,074   12,000 x 400      4 links  16    240, 300
+// 110,000 x 225    34 links  10  3,222, 2,864  200,000 x 1,000   20 links  16  2,140, 3,422
+// 120,000 x 500     5 links   1    733, 670    200,000 x 400     80 links  16  5,177, 4,638
+// (the left column's first three are scenes' transfers). Over 1,365 matrices the
+// rule costs 1% against the better one of each; k_spmm_shared for all costs 5%,
+// and up to twice the time. It is wrong for up to 2,000 rows of like length and
+// many links (2,000 x 300, 150 links: 257, 289), where scenes' transfers, whose
+// longest rows are several times the mean, gain (2,000 x 862, 179 links: 455, 371).
+static bool spmm_shared_wins(uint32_t n, uint32_t R, uint64_t links) {
+    const uint64_t rows = n;
+    if (links >= 60u * rows) return true;
+    return rows * R <= 1250000u && (links >= 32u * rows || links >= (1u << 19));  // 80 MB an array
+}
+
 static void launch_spmm_shared(cudaStream_t st, const float4* direct, const float4* albedo, float4* irr, float4* rad,
                                uint32_t n, uint32_t R, const uint32_t* starts, const uint32_t* idx, const float* w,
                                const float4* crad, uint32_t nc, const uint32_t* done, uint32_t* res_bits, int warps) {
@@ -224,7 +246,7 @@ int launch_batched_bounce(cudaStream_t st, uint32_t n, uint32_t R, const float4*
                           const float4* direct, float4* irr, float4* rad, const float4* cp, const uint2* crange,
                           const uint32_t* members, uint32_t nc, const uint32_t* starts, const uint32_t* idx,
                           const float* w, float4* crad, uint32_t* done, uint32_t* iterations, uint32_t* res_bits,
-                          uint32_t* last_res, uint32_t it, int rows_per_block_warps) {
+                          uint32_t* last_res, uint32_t it, int rows_per_block_warps, uint64_t links) {
     const uint32_t chunks = (R + 31) / 32;
     k_agg_batched<<<grid_for((unsigned long long)nc * chunks * 32ull, 256), 256, 0, st>>>(rad, sp, cp, crange,
                                                                                           members, nc, R, crad, done);
@@ -235,7 +257,7 @@ int launch_batched_bounce(cudaStream_t st, uint32_t n, uint32_t R, const float4*
     // Cornell box's 20,000 surfels 6.1 ms against 9.3 in chunks of 16 (64:
     // 2.14 and 2.24; 24: 1.36 and 1.41).
     const int warps = 4 * rows_per_block_warps < 32 ? 4 * rows_per_block_warps : 32;
-    if (R <= kRhs && spmm_shared_bytes(nc, warps) <= kSpmmSharedMax) {
+    if (R <= kRhs && spmm_shared_bytes(nc, warps) <= kSpmmSharedMax && spmm_shared_wins(n, R, links)) {
         launch_spmm_shared(st, direct, albedo, irr, rad, n, R, starts, idx, w, crad, nc, done, res_bits, warps);
     } else {
         const int block = 32 * rows_per_block_warps;

@@ -231,7 +231,7 @@ int launch_batched_bounce(cudaStream_t st, uint32_t n, uint32_t R, const float4*
                           const float4* direct, float4* irr, float4* rad, const float4* cp, const uint2* crange,
                           const uint32_t* members, uint32_t nc, const uint32_t* starts, const uint32_t* idx,
                           const float* w, float4* crad, uint32_t* done, uint32_t* iterations, uint32_t* res_bits,
-                          uint32_t* last_res, uint32_t it, int rows_per_block_warps);
+                          uint32_t* last_res, uint32_t it, int rows_per_block_warps, uint64_t links);
 
 // ---- grid + shade (surfel.rs:71-114, main.rs:229-367, film.rs:51-61) ----
 void launch_grid_keys(cudaStream_t st, const float4* p, uint32_t n, GridParams g, unsigned long long* keys);
