@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(1024) k_spmm_shared(const float4* direct, cons
 //  45,000 x 809   119 links   2  1,664, 1,074   12,000 x 400      4 links  16    240, 300
 // 110,000 x 225    34 links  10  3,222, 2,864  200,000 x 1,000   20 links  16  2,140, 3,422
 // 120,000 x 500     5 links   1    733, 670    200,000 x 400     80 links  16  5,177, 4,638
-// (the left column's first three are scenes' transfers). Over 1,365 matrices the
+// (the left column's first three are scenes' transfers). Over 1,323 matrices the
 // rule costs 1% against the better one of each; k_spmm_shared for all costs 5%,
 // and up to twice the time. It is wrong for up to 2,000 rows of like length and
 // many links (2,000 x 300, 150 links: 257, 289), where scenes' transfers, whose
