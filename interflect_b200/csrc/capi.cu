@@ -63,6 +63,8 @@ struct ifx_ctx {
     uint32_t stage_limit = kDefaultStageLimit;
     bool objgrid_on = true;  // build the object grid at the next upload (ifx_set_leaf_grid)
     DBuf og_cells;           // its per-cell masks or lists
+    int max_smem = 0;        // dynamic shared memory that the kernels are allowed
+    bool no_grid_ready = false;  // those of scenes without a grid too
     SceneConsts sc{};
     DBuf status;  // uint32 device status word
     DBuf srgb_t;  // 256 f32 thresholds
@@ -438,7 +440,8 @@ extern "C" int ifx_ctx_create(int device, ifx_ctx** out) {
         // The opt-in maximum less room for the kernels' static shared memory.
         int optin = kMaxDynSmem;
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-        configure_kernels(std::min(optin, kMaxDynSmem) - 4096);
+        ctx->max_smem = std::min(optin, kMaxDynSmem) - 4096;
+        configure_kernels(ctx->max_smem, false);
         if ((e = cudaGetLastError()) != cudaSuccess) return bail(e);
     }
     if ((e = cudaStreamSynchronize(ctx->st)) != cudaSuccess) return bail(e);
@@ -698,16 +701,22 @@ extern "C" int ifx_scene_upload(ifx_ctx* ctx, const ifx_scene* scene) {
     ctx->scene = s;
     ctx->blobref.ptr = (const uint8_t*)ctx->blob.p;
     ctx->blobref.bytes = (uint32_t)blob.size();
-    ctx->blobref.stage_bytes = reinterpret_cast<const BlobHeader*>(blob.data())->off_lights;
-    choose_staging(ctx);
     ctx->blobref.stack_depth = maxd + 2;
     ctx->blobref.wait_polls = ctx->wait_polls;
     ctx->sc = scene_consts(s);
     {
         int r = objgrid_build(ctx, blob);
         if (r) return r;
-        // The three-node kernels read the grid as masks.
+        // The packed objects, last of the geometry, are read with a grid only.
         const BlobHeader* bh = reinterpret_cast<const BlobHeader*>(blob.data());
+        ctx->blobref.stage_bytes = ctx->blobref.og.mode == kOgOff ? bh->off_fast : bh->off_lights;
+        choose_staging(ctx);
+        if (ctx->blobref.og.mode == kOgOff && !ctx->no_grid_ready) {
+            configure_kernels(ctx->max_smem, true);
+            ctx->no_grid_ready = true;
+        }
+        ctx->blobref.linear = bh->use_bvh ? 0 : 1;
+        // The three-node kernels read the grid as masks.
         ctx->blobref.tree3 = bh->use_bvh && bh->n_nodes == 3 && ctx->blobref.og.mode != kOgList ? 1 : 0;
     }
     CK(cudaStreamSynchronize(ctx->st));

@@ -171,16 +171,24 @@ enum CounterId : int {
 // be a root with two leaves, so the distance queries compile only that
 // traversal; a kernel then carries a fraction of the code, which matters to
 // instruction-fetch-bound ray marches. NoCount3 is NoCount for such scenes.
+// kGrid: the scene has an object grid (objgrid.h). Kernels for scenes without
+// one (NoGrid, NoGrid3) and the counting kernels hold the plain traversal.
 struct NoCount {
-    static constexpr bool kTree3 = false;
+    static constexpr bool kTree3 = false, kGrid = true;
     __device__ __forceinline__ void add(int, uint32_t = 1) {}
 };
 struct NoCount3 : NoCount {
     static constexpr bool kTree3 = true;
 };
+struct NoGrid : NoCount {
+    static constexpr bool kGrid = false;
+};
+struct NoGrid3 : NoGrid {
+    static constexpr bool kTree3 = true;
+};
 
 struct Counts {
-    static constexpr bool kTree3 = false;
+    static constexpr bool kTree3 = false, kGrid = false;
     uint32_t v[kNumCounters];
     __device__ __forceinline__ Counts() {
 #pragma unroll
@@ -337,34 +345,51 @@ __device__ __forceinline__ float prim_dist(const DPrim& pr, V p, C& cnt) {
 // but for rounding (a few ulps of its operands, far below the margin here).
 // So in the uncounted kernels, once the distance is at or beyond `best` (plus
 // that margin for the smooth form) it cannot win the comparison, and the
-// subtractions left are not evaluated; the returned value is then itself >=
-// best. The counting kernels evaluate everything, as the reference does.
+// subtractions left are not evaluated (without a grid: all or none); the
+// returned value is then itself >= best. The counting kernels evaluate
+// everything, as the reference does.
 template <class C>
 __device__ __forceinline__ float obj_dist(const SceneView& sv, const DObject& o, V p, C& cnt, float best = kMaxF) {
-    float d = 0.0f;
-    const float limit = best + (o.smooth > 0.0f ? 1e-5f * (1.0f + fabsf(best) + o.smooth) : 0.0f);
-    // The base is the loop's first turn, so that prim_dist has one site.
+    if constexpr (C::kGrid) {
+        const float limit = best + (o.smooth > 0.0f ? 1e-5f * (1.0f + fabsf(best) + o.smooth) : 0.0f);
+        float d = 0.0f;
+        // The base is the loop's first turn, so that prim_dist has one site.
 #pragma unroll 1
-    for (int s = 0; s <= o.nsub; ++s) {
-        const float sd = prim_dist(sv.prim(o.prim + s), p, cnt);
-        if (s > 0) cnt.add(o.smooth > 0.0f ? CN_SMOOTH : CN_HARD);
-        if (s == 0) {
-            d = sd;
-        } else if (o.smooth > 0.0f) {
-            float k = o.smooth;
-            // Where d + sd >= k the weight hk is 0 and the blend is d.
-            if (sizeof(C) > 1 || !(d + sd >= 1.00001f * k && sd < 1e30f)) {
-                float hk = clampr(0.5f - 0.5f * (d + sd) / k, 0.0f, 1.0f);
-                d = d * (1.0f - hk) + (-sd) * hk + k * hk * (1.0f - hk);
+        for (int s = 0; s <= o.nsub; ++s) {
+            const float sd = prim_dist(sv.prim(o.prim + s), p, cnt);
+            if (s == 0) {
+                d = sd;
+            } else if (o.smooth > 0.0f) {
+                float k = o.smooth;
+                // Where d + sd >= k the weight hk is 0 and the blend is d.
+                if (!(d + sd >= 1.00001f * k && sd < 1e30f)) {
+                    float hk = clampr(0.5f - 0.5f * (d + sd) / k, 0.0f, 1.0f);
+                    d = d * (1.0f - hk) + (-sd) * hk + k * hk * (1.0f - hk);
+                }
+            } else {
+                d = fmaxf(d, -sd);
             }
-        } else {
-            d = fmaxf(d, -sd);
-        }
-        if constexpr (sizeof(C) == 1) {
             if (s < o.nsub && d >= limit) return d;
         }
+        return d;
+    } else {
+        float d = prim_dist(sv.prim(o.prim), p, cnt);
+        if constexpr (sizeof(C) == 1) {
+            if (o.nsub > 0 && d >= best + (o.smooth > 0.0f ? 1e-5f * (1.0f + fabsf(best) + o.smooth) : 0.0f)) return d;
+        }
+        for (int s = 1; s <= o.nsub; ++s) {
+            const float sd = prim_dist(sv.prim(o.prim + s), p, cnt);
+            cnt.add(o.smooth > 0.0f ? CN_SMOOTH : CN_HARD);
+            if (o.smooth > 0.0f) {
+                float k = o.smooth;
+                float hk = clampr(0.5f - 0.5f * (d + sd) / k, 0.0f, 1.0f);
+                d = d * (1.0f - hk) + (-sd) * hk + k * hk * (1.0f - hk);
+            } else {
+                d = fmaxf(d, -sd);
+            }
+        }
+        return d;
     }
-    return d;
 }
 
 // bvh.rs:46-50 before its square root: the box distance is
@@ -382,7 +407,269 @@ struct DistHit {
     uint32_t mat;
 };
 
-// ------------------------------------------------- the reference query ----
+// ------------------------------------ the traversal of scenes without a grid ----
+// Scenes that have no object grid (cones, no BVH, degenerate primitives) ask the
+// reference's traversal for every step, as the counting kernels do. Each kind
+// of range has its own loop here: with the grid's fallback below, whose one
+// evaluation site serves its kernels' instruction cache, and with lanes that wait
+// to be refilled (kRefill), these scenes' frames took 1.1 to 1.6 times as long
+// (128 objects and a cone, 300 x 200: 66.1 ms, 54.3 now; without the BVH 101 and
+// 64 ms).
+
+// scene.rs:191-208 with bvh.rs:100-150 (query) or bvh.rs:155-163 (linear).
+template <class C>
+__device__ __forceinline__ DistHit dist_mat_tree(const SceneView& sv, V p, C& cnt) {
+    DistHit best{kMaxF, 0u};
+    for (int i = 0; i < sv.n_planes; ++i) {
+        const DObject o = sv.obj(i);
+        float d = obj_dist(sv, o, p, cnt, best.d);
+        if (d < best.d) best = DistHit{d, o.mat};
+    }
+    if constexpr (C::kTree3) {
+        // bvh.rs:100-150 on a root and two leaves: the same tests, prunes and
+        // visit order as the stack traversal below.
+        if (sq_ge(aabb_dist2(p, sv.node(0), cnt), best.d)) return best;
+        const int r = sv.node(0).link;
+        const float dl = aabb_dist2(p, sv.node(1), cnt), dr = aabb_dist2(p, sv.node(r), cnt);
+        const bool lfirst = sq_lt(dl, dr);
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            const bool left = (pass == 0) == lfirst;
+            if (sq_ge(left ? dl : dr, best.d)) continue;
+            const DNode& nd = sv.node(left ? 1 : r);
+            for (int k = nd.link; k < nd.link + nd.count; ++k) {
+                const DObject o = sv.obj(k);
+                const float d = obj_dist(sv, o, p, cnt, best.d);
+                if (d < best.d) {
+                    best.d = d;
+                    best.mat = o.mat;
+                }
+            }
+        }
+        return best;
+    }
+    if (sv.use_bvh) {
+        if (sv.n_nodes == 0) return best;
+        // bvh.rs:100-150. A node's box distance is a pure function of p and
+        // the node, so the value computed when it was pushed (bvh.rs:135-136)
+        // is the one the reference recomputes when it pops it (:116); it is
+        // kept on the stack and counted as the reference's test.
+        // The stack holds squared box distances (see sq_ge / sq_lt).
+        uint32_t* const stack = sv.stk;
+        float* const stackd = sv.stkd;
+        const int stride = sv.stk_stride;
+        int sp = 0;
+        stack[0] = 0;
+        stackd[0] = aabb_dist2(p, sv.node(0), cnt);
+        sp = 1;
+        bool first = true;
+        while (sp > 0) {
+            --sp;
+            const int ni = (int)stack[sp * stride];
+            const DNode nd = sv.node(ni);
+            if (!first) cnt.add(CN_NODE);
+            first = false;
+            if (sq_ge(stackd[sp * stride], best.d)) continue;
+            if (nd.count > 0) {
+                for (int k = nd.link; k < nd.link + nd.count; ++k) {
+                    const DObject o = sv.obj(k);
+                    float d = obj_dist(sv, o, p, cnt, best.d);
+                    if (d < best.d) {
+                        best.d = d;
+                        best.mat = o.mat;
+                    }
+                }
+            } else {
+                const int l = ni + 1, r = nd.link;
+                float dl = aabb_dist2(p, sv.node(l), cnt);
+                float dr = aabb_dist2(p, sv.node(r), cnt);
+                // Near-first DFS holds at most depth + 1 entries; the host
+                // sizes the stack to depth + 2 (and rejects trees deeper
+                // than the reference's 64-entry stack). The guard keeps an
+                // unexpected overflow inside the stack: traversal stops.
+                if (sp + 2 > sv.stk_depth) break;
+                if (sq_lt(dl, dr)) {
+                    stack[sp * stride] = (uint32_t)r;
+                    stackd[sp * stride] = dr;
+                    stack[(sp + 1) * stride] = (uint32_t)l;
+                    stackd[(sp + 1) * stride] = dl;
+                } else {
+                    stack[sp * stride] = (uint32_t)l;
+                    stackd[sp * stride] = dl;
+                    stack[(sp + 1) * stride] = (uint32_t)r;
+                    stackd[(sp + 1) * stride] = dr;
+                }
+                sp += 2;
+            }
+        }
+    } else {
+        for (int k = 0; k < sv.n_objects; ++k) {
+            const DObject o = sv.obj(sv.lin(k));
+            float d = obj_dist(sv, o, p, cnt, best.d);
+            if (d < best.d) {
+                best.d = d;
+                best.mat = o.mat;
+            }
+        }
+    }
+    return best;
+}
+
+// Evaluates leaf `leaf`'s objects into `best` (bvh.rs:118-126).
+template <class C>
+__device__ __forceinline__ void leaf_eval(const SceneView& sv, int leaf, V p, DistHit& best, C& cnt) {
+    const DNode nd = sv.node(leaf);
+    for (int k = nd.link; k < nd.link + nd.count; ++k) {
+        const DObject o = sv.obj(k);
+        const float d = obj_dist(sv, o, p, cnt, best.d);
+        if (d < best.d) {
+            best.d = d;
+            best.mat = o.mat;
+        }
+    }
+}
+
+// dist_mat_tree_warp's traversal for a three-node tree (a root and two leaves):
+// the same box tests, pruning decisions, visit order and counts, with the two
+// pending leaves held in registers instead of the shared-memory stack. The
+// root is popped first (not counted, as in dist_mat_tree), then the nearer leaf,
+// then the other; leaves are evaluated in warp rounds of one leaf each.
+template <class C>
+__device__ __forceinline__ DistHit dist_mat_tree_warp3(const SceneView& sv, V p, bool active, DistHit best, C& cnt) {
+    int next = -1, last = -1;  // leaves still to pop, in order
+    float dnext = 0.0f, dlast = 0.0f;
+    if (active) {
+        const float d0 = aabb_dist2(p, sv.node(0), cnt);
+        if (!sq_ge(d0, best.d)) {
+            const int l = 1, r = sv.node(0).link;
+            const float dl = aabb_dist2(p, sv.node(l), cnt);
+            const float dr = aabb_dist2(p, sv.node(r), cnt);
+            if (sq_lt(dl, dr)) {
+                next = l, dnext = dl, last = r, dlast = dr;
+            } else {
+                next = r, dnext = dr, last = l, dlast = dl;
+            }
+        }
+    }
+    int pending = -1;
+    while (true) {
+        while (pending < 0 && next >= 0) {
+            cnt.add(CN_NODE);
+            if (!sq_ge(dnext, best.d)) pending = next;
+            next = last, dnext = dlast, last = -1;
+        }
+        const unsigned waiting = __ballot_sync(0xffffffffu, pending >= 0);
+        if (!waiting) break;
+        const int leaf = __shfl_sync(0xffffffffu, pending, __ffs(waiting) - 1);
+        if (pending == leaf) {
+            leaf_eval(sv, leaf, p, best, cnt);
+            pending = -1;
+        }
+    }
+    return best;
+}
+
+// dist_mat_tree for a whole warp (all 32 lanes call it; lanes with !active only
+// take part in the votes). Each active lane runs its own near-first BVH
+// traversal with the reference's pruning, but leaves are evaluated in
+// warp-synchronous rounds: a lane advances through interior nodes until it
+// reaches a leaf that passes the AABB test; then, once every lane has either
+// found one or finished, either the lanes sharing the first waiting lane's
+// leaf evaluate it together (the primitive code runs converged) or, in trees
+// of more than four leaves when fewer than 7/8 of the waiting lanes share
+// that leaf, every waiting lane evaluates its own leaf in the same round
+// (lanes at different leaves then diverge only by primitive kind, instead of
+// waiting a round per leaf). A lane's sequence of node
+// tests, object evaluations and best-distance updates is exactly the one
+// dist_mat_tree() makes.
+template <class C>
+__device__ __forceinline__ DistHit dist_mat_tree_warp(const SceneView& sv, V p, bool active, C& cnt) {
+    DistHit best{kMaxF, 0u};
+    if (active) {
+        for (int i = 0; i < sv.n_planes; ++i) {
+            const DObject o = sv.obj(i);
+            float d = obj_dist(sv, o, p, cnt, best.d);
+            if (d < best.d) best = DistHit{d, o.mat};
+        }
+    }
+    if constexpr (C::kTree3) return dist_mat_tree_warp3(sv, p, active, best, cnt);
+    if (!sv.use_bvh) {
+        if (active) {
+            for (int k = 0; k < sv.n_objects; ++k) {
+                const DObject o = sv.obj(sv.lin(k));
+                float d = obj_dist(sv, o, p, cnt, best.d);
+                if (d < best.d) {
+                    best.d = d;
+                    best.mat = o.mat;
+                }
+            }
+        }
+        return best;
+    }
+    if (sv.n_nodes == 0) return best;
+    if (sv.n_nodes == 3) return dist_mat_tree_warp3(sv, p, active, best, cnt);
+    uint32_t* const stack = sv.stk;
+    float* const stackd = sv.stkd;
+    const int stride = sv.stk_stride;
+    int sp = 0;
+    bool first = true;
+    if (active) {
+        stack[0] = 0;
+        stackd[0] = aabb_dist2(p, sv.node(0), cnt);
+        sp = 1;
+    }
+    int pending = -1;
+    while (true) {
+        while (pending < 0 && sp > 0) {
+            --sp;
+            const int ni = (int)stack[sp * stride];
+            const DNode nd = sv.node(ni);
+            // The box distance stored at push time (see dist_mat_tree).
+            if (!first) cnt.add(CN_NODE);
+            first = false;
+            if (sq_ge(stackd[sp * stride], best.d)) continue;
+            if (nd.count > 0) {
+                pending = ni;
+                break;
+            }
+            const int l = ni + 1, r = nd.link;
+            float dl = aabb_dist2(p, sv.node(l), cnt);
+            float dr = aabb_dist2(p, sv.node(r), cnt);
+            if (sp + 2 > sv.stk_depth) {
+                sp = 0;
+                break;
+            }
+            if (sq_lt(dl, dr)) {
+                stack[sp * stride] = (uint32_t)r;
+                stackd[sp * stride] = dr;
+                stack[(sp + 1) * stride] = (uint32_t)l;
+                stackd[(sp + 1) * stride] = dl;
+            } else {
+                stack[sp * stride] = (uint32_t)l;
+                stackd[sp * stride] = dl;
+                stack[(sp + 1) * stride] = (uint32_t)r;
+                stackd[(sp + 1) * stride] = dr;
+            }
+            sp += 2;
+        }
+        const unsigned waiting = __ballot_sync(0xffffffffu, pending >= 0);
+        if (!waiting) break;
+        const int leaf = __shfl_sync(0xffffffffu, pending, __ffs(waiting) - 1);
+        // Trees of at most four leaves: one leaf per round, converged. Larger
+        // trees: the first waiting lane's leaf is evaluated alone when at
+        // least 7/8 of the waiting lanes share it; otherwise every waiting
+        // lane evaluates its own leaf in this round.
+        const bool shared = sv.n_nodes <= 7 || 8 * __popc(__ballot_sync(0xffffffffu, pending == leaf)) >=
+                                                   7 * __popc(waiting);
+        if (pending >= 0 && (pending == leaf || !shared)) {
+            leaf_eval(sv, pending, p, best, cnt);
+            pending = -1;
+        }
+    }
+    return best;
+}
+
+// ------------------------------------------------- the grid's fallback ----
 // scene.rs:191-208 with bvh.rs:100-150 (query) or bvh.rs:155-163 (linear) as a
 // sequence of object ranges: the planes, then the leaves the pruned near-first
 // traversal reaches (or all objects in parse order). Every range is evaluated
@@ -631,7 +918,9 @@ __device__ __forceinline__ bool og_walk_list(const SceneView& sv, OgBest& b, uin
 template <class C>
 __device__ __forceinline__ DistHit dist_mat(const SceneView& sv, V p, C& cnt) {
     cnt.add(CN_SDF);
-    if constexpr (sizeof(C) == 1) {
+    if constexpr (!C::kGrid) {
+        return dist_mat_tree(sv, p, cnt);
+    } else {
         uint32_t cell;
         bool coarse;
         if (sv.og.mode != kOgOff && og_cell(sv.og, p.x, p.y, p.z, cell, coarse)) {
@@ -644,8 +933,8 @@ __device__ __forceinline__ DistHit dist_mat(const SceneView& sv, V p, C& cnt) {
             }
             if (ok && b.d1 < kMaxF && b.exact(sv, p, false)) return DistHit{b.d1, sv.obj(b.o1).mat};
         }
+        return dist_mat_ref(sv, p, cnt);
     }
-    return dist_mat_ref(sv, p, cnt);
 }
 
 template <class C>
@@ -677,7 +966,9 @@ template <bool kDistOnly, bool kUnion = true, class C>
 __device__ __forceinline__ DistHit dist_warp(const SceneView& sv, V p, bool active, C& cnt, bool* in_grid = nullptr) {
     if (in_grid) *in_grid = false;
     if (active) cnt.add(CN_SDF);
-    if constexpr (sizeof(C) == 1) {
+    if constexpr (!C::kGrid) {
+        return dist_mat_tree_warp(sv, p, active, cnt);
+    } else {
         if (sv.og.mode != kOgOff) {
             uint32_t cell = 0;
             bool coarse = false;
@@ -702,8 +993,8 @@ __device__ __forceinline__ DistHit dist_warp(const SceneView& sv, V p, bool acti
             }
             return h;
         }
+        return dist_mat_ref_warp(sv, p, active, cnt);
     }
-    return dist_mat_ref_warp(sv, p, active, cnt);
 }
 
 // ------------------------------------------------------------ trace.rs ----
@@ -821,7 +1112,7 @@ __device__ __forceinline__ bool open_steps(ShadowRay& s, float h, float delta) {
 // trace.rs:84-124. Returns true when the march has ended, with `vis` set.
 template <class C>
 __device__ __forceinline__ bool shadow_step_w(const SceneView& sv, ShadowRay& s, bool active, float& vis, C& cnt) {
-    constexpr bool kSkips = sizeof(C) == 1;
+    constexpr bool kSkips = C::kGrid;
     const bool back = kSkips && s.mode == kPhBack;
     bool in_grid;
     float h = dist_warp<true>(sv, s.ro + s.rd * (back ? s.tp : s.t), active, cnt, &in_grid).d;

@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(128) k_path(ShadeParams P, uint32_t spp, const
     const unsigned long long total = (unsigned long long)P.w * P.h;
     const float tmax = P.tmax;
     constexpr uint32_t kMaxDepth = 12u;  // main.rs:255
-    WarpQueue q(total);
+    WarpQueue<C> q(total);
 
     int phase = kPhIdle, tap = 0, li = 0;
     uint32_t pix = 0, sample = 0, depth = 0, hmat = 0;
@@ -214,19 +214,18 @@ int launch_path(cudaStream_t st, const ShadeParams& p, uint32_t spp, const float
                 unsigned long long* cursor) {
     const size_t sm = blob_smem(p.blob, 128);
     const unsigned long long px = (unsigned long long)p.w * p.h;
-    if (p.counts)
-        k_path<Counts><<<persistent_grid(k_path<Counts>, 128, sm, px), 128, sm, st>>>(p, spp, sincos, cursor);
-    else if (p.blob.tree3)
-        k_path<NoCount3><<<persistent_grid(k_path<NoCount3>, 128, sm, px), 128, sm, st>>>(p, spp, sincos, cursor);
-    else
-        k_path<NoCount><<<persistent_grid(k_path<NoCount>, 128, sm, px), 128, sm, st>>>(p, spp, sincos, cursor);
+    with_policy(p.blob, p.counts != nullptr, [&](auto policy) {
+        using C = typename decltype(policy)::type;
+        k_path<C><<<persistent_grid(k_path<C>, 128, sm, px, p.blob), 128, sm, st>>>(p, spp, sincos, cursor);
+    });
     return 1;
 }
 
-void configure_path_kernels(int max_dyn_smem) {
-    cudaFuncSetAttribute(k_path<NoCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_path<NoCount3>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_path<Counts>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+void configure_path_kernels(int max_dyn_smem, bool no_grid) {
+    for_each_policy(no_grid, [&](auto policy) {
+        cudaFuncSetAttribute(k_path<typename decltype(policy)::type>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             max_dyn_smem);
+    });
 }
 
 }  // namespace ifx

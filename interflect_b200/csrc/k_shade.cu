@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(128) k_primary(ShadeParams P) {
     IFX_SCENE_PROLOGUE(P.blob, P.status, sv);
     C cnt;
     const unsigned long long total = (unsigned long long)P.w * P.h;
-    WarpQueue q(total);
+    WarpQueue<C> q(total);
     const V org{P.cam.origin[0], P.cam.origin[1], P.cam.origin[2]};
     uint32_t item = ~0u;
     TraceRay ray{};
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(128) k_shadow(ShadeParams P, const float4* hp,
     IFX_SCENE_PROLOGUE(P.blob, P.status, sv);
     C cnt;
     const unsigned long long total = *qlen;
-    WarpQueue q(total);
+    WarpQueue<C> q(total);
     uint32_t item = ~0u;
     ShadowRay ray{};
     unsigned long long ev = 0;
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(128) k_reflect(ShadeParams P) {
     IFX_SCENE_PROLOGUE(P.blob, P.status, sv);
     C cnt;
     const unsigned long long total = P.qlen[1];
-    WarpQueue q(total);
+    WarpQueue<C> q(total);
     uint32_t item = ~0u, pix = 0;
     TraceRay ray{};
     unsigned long long ev = 0;
@@ -310,7 +310,7 @@ static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, i
     auto rec = [&](int i) { rec_on(i, st); };
     if (part & kShadeFront) {
         rec(0);
-        k_primary<C><<<persistent_grid(k_primary<C>, 128, sm, px), 128, sm, st>>>(with(0));
+        k_primary<C><<<persistent_grid(k_primary<C>, 128, sm, px, p.blob), 128, sm, st>>>(with(0));
         rec(1);
         rec(8);
         k_setup<C><<<grid_for(px, 128, 16), 128, sm, st>>>(with(4));
@@ -322,19 +322,19 @@ static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, i
             cudaStreamWaitEvent(st1, side->fork, 0);
         }
         rec_on(2, st1);
-        k_shadow<C><<<persistent_grid(k_shadow<C>, 128, sm, slots), 128, sm, st1>>>(
+        k_shadow<C><<<persistent_grid(k_shadow<C>, 128, sm, slots, p.blob), 128, sm, st1>>>(
             with(1), p.hp1, p.hn1, p.q1, &p.qlen[0], p.vis1, &p.cursors[2]);
         rec_on(3, st1);
         if (fork) cudaEventRecord(side->join, st1);
         rec(4);
-        if (p.has_gi) k_reflect<C><<<persistent_grid(k_reflect<C>, 128, sm, px), 128, sm, st>>>(with(2));
+        if (p.has_gi) k_reflect<C><<<persistent_grid(k_reflect<C>, 128, sm, px, p.blob), 128, sm, st>>>(with(2));
         rec(5);
         rec(10);
         if (p.has_gi) k_setup2<C><<<grid_for(px, 128, 16), 128, sm, st>>>(with(4));
         rec(11);
         rec(6);
         if (p.has_gi)
-            k_shadow<C><<<persistent_grid(k_shadow<C>, 128, sm, slots), 128, sm, st>>>(
+            k_shadow<C><<<persistent_grid(k_shadow<C>, 128, sm, slots, p.blob), 128, sm, st>>>(
                 with(3), p.hp2, p.hn2, p.q2, &p.qlen[2], p.vis2, &p.cursors[3]);
         rec(7);
         if (fork) cudaStreamWaitEvent(st, side->join, 0);
@@ -342,15 +342,15 @@ static void launch_all(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, i
     if (part & kShadeCompose) {
         rec(12);
         const unsigned long long cpx = p.pix1 ? (unsigned long long)(p.pix1 - p.pix0) : px;
-        k_compose<C><<<grid_for(cpx, 128, kComposeCtas), 128, 0, st>>>(with(4));
+        using K = std::conditional_t<sizeof(C) == 1, NoCount, C>;  // it asks for no distance
+        k_compose<K><<<grid_for(cpx, 128, kComposeCtas), 128, 0, st>>>(with(4));
         rec(13);
     }
 }
 
 int launch_shade(cudaStream_t st, const ShadeParams& p, cudaEvent_t* ev, int part, const SideStream* side) {
-    if (p.counts) launch_all<Counts>(st, p, ev, part, side);
-    else if (p.blob.tree3) launch_all<NoCount3>(st, p, ev, part, side);
-    else launch_all<NoCount>(st, p, ev, part, side);
+    with_policy(p.blob, p.counts != nullptr,
+                [&](auto policy) { launch_all<typename decltype(policy)::type>(st, p, ev, part, side); });
     return ((part & kShadeFront) ? (p.has_gi ? 6 : 3) : 0) + ((part & kShadeCompose) ? 1 : 0);
 }
 
@@ -412,19 +412,12 @@ int launch_light_slots(cudaStream_t st, const ShadeParams& p, const SurfelArrays
                        float* vis, float* terms, unsigned long long* cursor) {
     const size_t sm = blob_smem(p.blob, 128);
     const unsigned long long slots = (unsigned long long)n * (unsigned long long)(p.nl > 0 ? p.nl : 1);
-    if (p.counts) {
-        k_light_setup<Counts><<<grid_for(n, 128, 16), 128, sm, st>>>(p, s.p, s.n, n, ff);
-        k_shadow<Counts><<<persistent_grid(k_shadow<Counts>, 128, sm, slots), 128, sm, st>>>(
-            p, s.p, s.n, p.q1, &p.qlen[0], vis, cursor);
-    } else if (p.blob.tree3) {
-        k_light_setup<NoCount3><<<grid_for(n, 128, 16), 128, sm, st>>>(p, s.p, s.n, n, ff);
-        k_shadow<NoCount3><<<persistent_grid(k_shadow<NoCount3>, 128, sm, slots), 128, sm, st>>>(
-            p, s.p, s.n, p.q1, &p.qlen[0], vis, cursor);
-    } else {
-        k_light_setup<NoCount><<<grid_for(n, 128, 16), 128, sm, st>>>(p, s.p, s.n, n, ff);
-        k_shadow<NoCount><<<persistent_grid(k_shadow<NoCount>, 128, sm, slots), 128, sm, st>>>(
-            p, s.p, s.n, p.q1, &p.qlen[0], vis, cursor);
-    }
+    with_policy(p.blob, p.counts != nullptr, [&](auto policy) {
+        using C = typename decltype(policy)::type;
+        k_light_setup<C><<<grid_for(n, 128, 16), 128, sm, st>>>(p, s.p, s.n, n, ff);
+        k_shadow<C><<<persistent_grid(k_shadow<C>, 128, sm, slots, p.blob), 128, sm, st>>>(p, s.p, s.n, p.q1, &p.qlen[0], vis,
+                                                                                  cursor);
+    });
     k_light_compose<<<grid_for(n, 128, 16), 128, sm, st>>>(p, s, n, ff, vis, terms);
     return 3;
 }
@@ -432,10 +425,7 @@ int launch_light_slots(cudaStream_t st, const ShadeParams& p, const SurfelArrays
 int launch_compose(cudaStream_t st, const ShadeParams& p) {
     ShadeParams q = p;
     q.counts = nullptr;
-    if (p.blob.tree3)
-        k_compose<NoCount3><<<grid_for((unsigned long long)p.w * p.h, 128, kComposeCtas), 128, 0, st>>>(q);
-    else
-        k_compose<NoCount><<<grid_for((unsigned long long)p.w * p.h, 128, kComposeCtas), 128, 0, st>>>(q);
+    k_compose<NoCount><<<grid_for((unsigned long long)p.w * p.h, 128, kComposeCtas), 128, 0, st>>>(q);
     return 1;
 }
 
@@ -446,15 +436,11 @@ static void configure_one(int max_dyn_smem) {
     cudaFuncSetAttribute(k_shadow<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
     cudaFuncSetAttribute(k_reflect<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
     cudaFuncSetAttribute(k_setup2<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+    cudaFuncSetAttribute(k_light_setup<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
 }
 
-void configure_shade_kernels(int max_dyn_smem) {
-    configure_one<NoCount>(max_dyn_smem);
-    configure_one<NoCount3>(max_dyn_smem);
-    configure_one<Counts>(max_dyn_smem);
-    cudaFuncSetAttribute(k_light_setup<NoCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_light_setup<NoCount3>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_light_setup<Counts>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+void configure_shade_kernels(int max_dyn_smem, bool no_grid) {
+    for_each_policy(no_grid, [&](auto policy) { configure_one<typename decltype(policy)::type>(max_dyn_smem); });
     cudaFuncSetAttribute(k_light_compose, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
 }
 

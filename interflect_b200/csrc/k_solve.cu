@@ -242,12 +242,10 @@ __global__ void k_solve_end(SolveCtl* ctl, uint32_t it) {
 void launch_light_surfels(cudaStream_t st, BlobRef blob, SurfelArrays s, uint32_t n, unsigned long long* evals,
                           uint32_t* status, unsigned long long* counts, float* terms) {
     const unsigned g = grid_for(n, 128, 16);
-    if (counts)
-        k_light_surfels<Counts><<<g, 128, blob_smem(blob, 128), st>>>(blob, s, n, evals, status, counts, terms);
-    else if (blob.tree3)
-        k_light_surfels<NoCount3><<<g, 128, blob_smem(blob, 128), st>>>(blob, s, n, evals, status, nullptr, terms);
-    else
-        k_light_surfels<NoCount><<<g, 128, blob_smem(blob, 128), st>>>(blob, s, n, evals, status, nullptr, terms);
+    with_policy(blob, counts != nullptr, [&](auto policy) {
+        using C = typename decltype(policy)::type;
+        k_light_surfels<C><<<g, 128, blob_smem(blob, 128), st>>>(blob, s, n, evals, status, counts, terms);
+    });
 }
 
 // kShared: many rows gather the cluster radiosities from shared memory, where
@@ -394,10 +392,11 @@ int launch_sell_fill(cudaStream_t st, const uint32_t* starts, const uint32_t* id
     return 1;
 }
 
-void configure_solve_kernels(int max_dyn_smem) {
-    cudaFuncSetAttribute(k_light_surfels<NoCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_light_surfels<NoCount3>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_light_surfels<Counts>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+void configure_solve_kernels(int max_dyn_smem, bool no_grid) {
+    for_each_policy(no_grid, [&](auto policy) {
+        cudaFuncSetAttribute(k_light_surfels<typename decltype(policy)::type>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+    });
     cudaFuncSetAttribute(k_jacobi_sell<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedRadMax);
 }
 

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(128) k_visibility(BlobRef blob, SceneConsts sc
                                                      unsigned long long* counts, unsigned long long* cursor) {
     IFX_SCENE_PROLOGUE(blob, status, sv);
     C cnt;
-    WarpQueue q(ncand);
+    WarpQueue<C> q(ncand);
     const float off = sc.diag * 5e-4f, tmin = sc.diag * 1e-3f;
     uint32_t item = ~0u;
     ShadowRay ray{};
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(128) k_closure(BlobRef blob, SceneConsts sc, c
     IFX_SCENE_PROLOGUE(blob, status, sv);
     C cnt;
     const unsigned long long total = (unsigned long long)n * 16ull;
-    WarpQueue q(total);
+    WarpQueue<C> q(total);
     const float tmax = sc.diag * 2.0f;
     uint32_t item = ~0u;
     TraceRay ray{};
@@ -327,17 +327,11 @@ void launch_visibility(cudaStream_t st, BlobRef blob, SceneConsts sc, const floa
                        uint32_t* status, unsigned long long* counts, unsigned long long* cursor) {
     if (ncand == 0) return;
     const size_t sm = blob_smem(blob, 128);
-    if (counts)
-        k_visibility<Counts><<<persistent_grid(k_visibility<Counts>, 128, sm, ncand), 128, sm, st>>>(
+    with_policy(blob, counts != nullptr, [&](auto policy) {
+        using C = typename decltype(policy)::type;
+        k_visibility<C><<<persistent_grid(k_visibility<C>, 128, sm, ncand, blob), 128, sm, st>>>(
             blob, sc, sp, sn, cp, cn, cand_c, cand_row, order, ncand, cand_vis, cand_steps, status, counts, cursor);
-    else if (blob.tree3)
-        k_visibility<NoCount3><<<persistent_grid(k_visibility<NoCount3>, 128, sm, ncand), 128, sm, st>>>(
-            blob, sc, sp, sn, cp, cn, cand_c, cand_row, order, ncand, cand_vis, cand_steps, status, nullptr,
-            cursor);
-    else
-        k_visibility<NoCount><<<persistent_grid(k_visibility<NoCount>, 128, sm, ncand), 128, sm, st>>>(
-            blob, sc, sp, sn, cp, cn, cand_c, cand_row, order, ncand, cand_vis, cand_steps, status, nullptr,
-            cursor);
+    });
 }
 
 // Sort keys of the visibility order: target cluster, then the source
@@ -373,15 +367,11 @@ void launch_closure(cudaStream_t st, BlobRef blob, SceneConsts sc, const float4*
                     unsigned long long* cursor) {
     const size_t sm = blob_smem(blob, 128);
     const unsigned long long items = (unsigned long long)n * 16ull;
-    if (counts)
-        k_closure<Counts><<<persistent_grid(k_closure<Counts>, 128, sm, items), 128, sm, st>>>(
-            blob, sc, sp, sn, n, order, clo, status, counts, cursor);
-    else if (blob.tree3)
-        k_closure<NoCount3><<<persistent_grid(k_closure<NoCount3>, 128, sm, items), 128, sm, st>>>(
-            blob, sc, sp, sn, n, order, clo, status, nullptr, cursor);
-    else
-        k_closure<NoCount><<<persistent_grid(k_closure<NoCount>, 128, sm, items), 128, sm, st>>>(
-            blob, sc, sp, sn, n, order, clo, status, nullptr, cursor);
+    with_policy(blob, counts != nullptr, [&](auto policy) {
+        using C = typename decltype(policy)::type;
+        k_closure<C><<<persistent_grid(k_closure<C>, 128, sm, items, blob), 128, sm, st>>>(blob, sc, sp, sn, n, order, clo,
+                                                                                    status, counts, cursor);
+    });
 }
 
 // Sort keys of the closure order: the row's cluster (nc when it has none),
@@ -445,13 +435,12 @@ void launch_check_transfer(cudaStream_t st, uint32_t n, uint32_t nc, unsigned lo
 }
 #endif
 
-void configure_transfer_kernels(int max_dyn_smem) {
-    cudaFuncSetAttribute(k_visibility<NoCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_visibility<NoCount3>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_visibility<Counts>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_closure<NoCount>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_closure<NoCount3>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
-    cudaFuncSetAttribute(k_closure<Counts>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+void configure_transfer_kernels(int max_dyn_smem, bool no_grid) {
+    for_each_policy(no_grid, [&](auto policy) {
+        using C = typename decltype(policy)::type;
+        cudaFuncSetAttribute(k_visibility<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+        cudaFuncSetAttribute(k_closure<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem);
+    });
 }
 
 }  // namespace ifx

@@ -101,6 +101,33 @@ static inline int sm_count() {
     return cached[dev];
 }
 
+// Calls f with the counter policy that a tracing kernel takes for the scene:
+// the counting kernels, or by its tree and by whether it has an object grid.
+template <class C>
+struct Policy {
+    using type = C;
+};
+template <class F>
+static inline void with_policy(const BlobRef& b, bool counts, F&& f) {
+    if (counts) f(Policy<Counts>{});
+    else if (b.og.mode == kOgOff && b.tree3) f(Policy<NoGrid3>{});
+    else if (b.og.mode == kOgOff) f(Policy<NoGrid>{});
+    else if (b.tree3) f(Policy<NoCount3>{});
+    else f(Policy<NoCount>{});
+}
+// The policies of scenes without a grid, or the others.
+template <class F>
+static inline void for_each_policy(bool no_grid, F&& f) {
+    if (no_grid) {
+        f(Policy<NoGrid3>{});
+        f(Policy<NoGrid>{});
+    } else {
+        f(Policy<Counts>{});
+        f(Policy<NoCount3>{});
+        f(Policy<NoCount>{});
+    }
+}
+
 static inline unsigned grid_for(unsigned long long items, int block, int per_sm_ctas = 8) {
     unsigned long long need = (items + (unsigned long long)block - 1) / (unsigned long long)block;
     unsigned long long cap = (unsigned long long)sm_count() * (unsigned long long)per_sm_ctas;
@@ -112,17 +139,19 @@ static inline unsigned grid_for(unsigned long long items, int block, int per_sm_
 // are spread thinly (WarpQueue then leaves lanes of every warp empty) until
 // there are kSpreadCtas per SM: a warp issues at most every fourth cycle or so
 // along a ray's dependent chain, so a scheduler needs about five warps to
-// stay busy, and a warp of fewer rays takes fewer divergent turns per step.
+// stay busy, and a warp of fewer rays takes fewer divergent turns per step. Not
+// so without a BVH, where all rays of a warp evaluate the same objects and more
+// warps do the same work again (40 objects, 97 x 61: 2.33 -> 2.63 ms spread).
 static constexpr unsigned kSpreadCtas = 5;
 template <class K>
-static inline unsigned persistent_grid(K kernel, int block, size_t smem, unsigned long long items) {
+static inline unsigned persistent_grid(K kernel, int block, size_t smem, unsigned long long items, const BlobRef& blob) {
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
     if (per_sm < 1) per_sm = 1;
     unsigned long long cap = (unsigned long long)sm_count() * (unsigned long long)per_sm;
     unsigned long long need = (items + (unsigned long long)block - 1) / (unsigned long long)block;
     const unsigned long long thin = (items * 32ull + (unsigned long long)block - 1) / (unsigned long long)block;
-    const unsigned long long spread = (unsigned long long)sm_count() * kSpreadCtas;
+    const unsigned long long spread = blob.linear ? 0ull : (unsigned long long)sm_count() * kSpreadCtas;
     need = need > spread ? need : (thin < spread ? thin : spread);
     if (need < 1) need = 1;
     return (unsigned)(need < cap ? need : cap);
@@ -139,8 +168,10 @@ static inline unsigned persistent_grid(K kernel, int block, size_t smem, unsigne
 // roots), and all lanes pay for it however few start. At 1, 4, 8, 12, 16: the
 // 512-object scene's visibility 17.8, 16.5, 16.6, 17.1, 17.7 ms, the product
 // scene's shadow rays 1.01, 0.94, 0.91, 0.89, 0.90 ms, its camera rays 0.72,
-// 0.72, 0.74, 0.83, 0.87 ms.
+// 0.72, 0.74, 0.83, 0.87 ms. Without a grid a step is dearer and an idle lane
+// costs more than a start: those kernels refill at one.
 static constexpr uint32_t kRefill = 8;
+template <class C>
 struct WarpQueue {
     uint32_t cur, end;  // warp-uniform private range [cur, end)
     uint32_t kChunk;    // items taken per atomic: about 1/8 of a fair share per warp, 32..256, or
@@ -165,7 +196,7 @@ struct WarpQueue {
         idle = idle && (uint32_t)lane < lanes;
         unsigned need = __ballot_sync(kFull, idle);
         uint32_t item = ~0u;
-        if ((uint32_t)__popc(need) < kRefill * lanes / 32u || !need) return item;
+        if ((uint32_t)__popc(need) < (C::kGrid ? kRefill : 1u) * lanes / 32u || !need) return item;
         if (cur >= end && !drained) {
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(cursor, (unsigned long long)kChunk);

@@ -12,8 +12,9 @@ namespace ifx {
 struct GatherView;
 
 // Program blob as handed to every tracing kernel. When `staged` is set the
-// kernel copies its geometry prefix (header, objects, primitives, BVH nodes,
-// packed objects: the first stage_bytes bytes, all the ray marches read) into dynamic shared
+// kernel copies its geometry prefix (header, objects, primitives, BVH nodes and,
+// where there is an object grid, packed objects: the first stage_bytes bytes, all
+// the ray marches read) into dynamic shared
 // memory; lights, materials and the linear order are always read from global
 // memory. Unstaged (large) scenes are read from global memory through L1.
 struct BlobRef {
@@ -23,6 +24,7 @@ struct BlobRef {
     int staged;
     int stack_depth;  // BVH traversal stack entries per thread (tree depth + 2)
     uint32_t wait_polls;  // poll budget of the staging wait (kDefaultWaitPolls unless the host lowers it)
+    int linear;           // every query evaluates all objects in parse order: no BVH
     int tree3;            // BVH in use and made of a root and two leaves: the NoCount3 kernels apply
     ObjGrid og;           // candidate objects per cell (objgrid.h); mode kOgOff where it does not apply
 };
@@ -390,12 +392,12 @@ int multi_frame_max_blocks(int block);
 
 // Raises the dynamic shared-memory limit of every scene-staging kernel.
 void configure_surfel_kernels(int max_dyn_smem);
-void configure_transfer_kernels(int max_dyn_smem);
-void configure_solve_kernels(int max_dyn_smem);
+void configure_transfer_kernels(int max_dyn_smem, bool no_grid);
+void configure_solve_kernels(int max_dyn_smem, bool no_grid);
 void configure_batch_kernels();
-void configure_shade_kernels(int max_dyn_smem);
+void configure_shade_kernels(int max_dyn_smem, bool no_grid);
 void configure_diff_kernels(int max_dyn_smem);
-void configure_path_kernels(int max_dyn_smem);
+void configure_path_kernels(int max_dyn_smem, bool no_grid);
 // Level l of the scene's object grid (objgrid.h): lo is its corner, cell its
 // cells' side; g.mode picks which of mask and list is written.
 void launch_og_build(cudaStream_t st, const BlobRef& blob, const ObjGrid& g, const OgLevel& l, const float lo[3],
@@ -404,14 +406,18 @@ void launch_og_build(cudaStream_t st, const BlobRef& blob, const ObjGrid& g, con
 // frame; sincos holds (sinf, cosf) of the 2^24 sampler angles.
 int launch_path(cudaStream_t st, const ShadeParams& p, uint32_t spp, const float2* sincos,
                 unsigned long long* cursor);
-inline void configure_kernels(int max_dyn_smem) {
-    configure_surfel_kernels(max_dyn_smem);
-    configure_transfer_kernels(max_dyn_smem);
-    configure_solve_kernels(max_dyn_smem);
-    configure_batch_kernels();
-    configure_shade_kernels(max_dyn_smem);
-    configure_diff_kernels(max_dyn_smem);
-    configure_path_kernels(max_dyn_smem);
+// A context sets the limits of its kernels when it is made (each first call for a
+// kernel loads it: 0.1 ms), those of scenes without a grid when one is uploaded.
+inline void configure_kernels(int max_dyn_smem, bool no_grid) {
+    if (!no_grid) {
+        configure_surfel_kernels(max_dyn_smem);
+        configure_batch_kernels();
+        configure_diff_kernels(max_dyn_smem);
+    }
+    configure_transfer_kernels(max_dyn_smem, no_grid);
+    configure_solve_kernels(max_dyn_smem, no_grid);
+    configure_shade_kernels(max_dyn_smem, no_grid);
+    configure_path_kernels(max_dyn_smem, no_grid);
 }
 
 }  // namespace ifx
