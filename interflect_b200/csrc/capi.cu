@@ -810,8 +810,10 @@ extern "C" int ifx_surfels_download(ifx_ctx* ctx, float* p, float* nrm, float* a
                                                      {&ctx->sdir, direct}, {&ctx->sirr, irr}, {&ctx->srad, rad}};
     // The arrays are packed to the caller's layout on the device: the host
     // unpacked 16-byte records by loops, 2.0 ms of 55,000 surfels' download.
-    // It still does where the device has no memory left for the packed arrays.
-    if (ensure(ctx, ctx->dlpack, n * 19 * 4) != IFX_OK) {
+    // It still does where the device has no memory left for the packed arrays,
+    // and for few surfels, where seven more launches cost more (on the host and
+    // on the device 60 surfels 106 and 138 us, 500 130 and 147, 2,000 202 and 175).
+    if (n <= 1024 || ensure(ctx, ctx->dlpack, n * 19 * 4) != IFX_OK) {
         ctx->err.clear();
         for (const auto& f : fields)
             if (int r = f.second ? unpack_on_host(ctx, *f.first, f.second, false) : IFX_OK) return r;
