@@ -1085,7 +1085,8 @@ static int sell_build(ifx_ctx* ctx, uint64_t longest) {
                                                 (const float*)ctx->w.p, n, perm, len, off,
                                                 (uint32_t*)ctx->sell_idx.p, (float*)ctx->sell_w.p);
     CKL();
-    ctx->sellm = SellMatrix{perm, len, off, (const uint32_t*)ctx->sell_idx.p, (const float*)ctx->sell_w.p};
+    ctx->sellm = SellMatrix{perm, len, off, (const uint32_t*)ctx->sell_idx.p, (const float*)ctx->sell_w.p,
+                            ctx->links};
     ctx->sell_ready = true;
     return IFX_OK;
 }

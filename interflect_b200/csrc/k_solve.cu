@@ -159,7 +159,9 @@ static constexpr uint32_t kWideRows = 49152, kWideLinks = 64;
 // rows take as long as the longest one's chain of gathers, each kernel with a
 // cold L1: small CTAs spread them over the SMs, and up to 1,024 clusters a copy
 // per CTA pays (20,000 rows, 793 clusters: 12 bounces 0.325 -> 0.258 ms; 50,000
-// rows, 2,504 clusters, 40 KiB a copy: 0.44 -> 0.47 ms).
+// rows, 2,504 clusters, 40 KiB a copy: 0.44 -> 0.47 ms). It pays where a CTA
+// gathers as many links as it copies clusters (8,000 rows of 5 links, 1,000
+// clusters, 12 bounces: 89 us copied, 69 not).
 static constexpr size_t kSharedRadMax = 64u * 1024u, kSharedRadSmall = 16u * 1024u;
 static constexpr unsigned kFewRowsBlock = 128;
 
@@ -291,12 +293,12 @@ void launch_solve_bounce(cudaStream_t st, SurfelArrays s, uint32_t n, const floa
     const float4 *direct = s.direct, *albedo = s.albedo, *crad = cluster_rad;
     const size_t cbytes = (size_t)nc * 16u;
     if (sell && sell->perm) {
-        if (n >= kManyRows && cbytes <= kSharedRadMax)
-            launch_pdl(k_jacobi_sell<true>, wave_grid(k_jacobi_sell<true>, kJacBlock, cbytes, n), kJacBlock, cbytes, st,
-                       direct, albedo, s.irr, s.rad, n, *sell, crad, nc, ctl, it);
-        else if (cbytes <= kSharedRadSmall)
-            launch_pdl(k_jacobi_sell<true>, grid_for(n, kFewRowsBlock), kFewRowsBlock, cbytes, st, direct, albedo, s.irr,
-                       s.rad, n, *sell, crad, nc, ctl, it);
+        const bool many = n >= kManyRows && cbytes <= kSharedRadMax;
+        const unsigned block = many ? (unsigned)kJacBlock : kFewRowsBlock;
+        const unsigned grid = many ? wave_grid(k_jacobi_sell<true>, kJacBlock, cbytes, n) : grid_for(n, kFewRowsBlock);
+        if ((many || cbytes <= kSharedRadSmall) && sell->links >= (uint64_t)grid * nc)
+            launch_pdl(k_jacobi_sell<true>, grid, block, cbytes, st, direct, albedo, s.irr, s.rad, n, *sell, crad, nc, ctl,
+                       it);
         else
             launch_pdl(k_jacobi_sell<false>, grid_for(n, kFewRowsBlock, 16), kFewRowsBlock, 0, st, direct, albedo, s.irr,
                        s.rad, n, *sell, crad, nc, ctl, it);

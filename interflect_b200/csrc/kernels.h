@@ -209,6 +209,7 @@ struct SellMatrix {
     const uint32_t* slice_off;  // per slice: first entry (multiple of 128)
     const uint32_t* idx;
     const float* w;
+    uint64_t links;             // of all rows, for the choice of kernel
 };
 void launch_solve_bounce(cudaStream_t st, SurfelArrays s, uint32_t n, const float4* cp, const uint2* crange,
                          const uint32_t* members, uint32_t nc, const uint32_t* starts, const uint32_t* idx,

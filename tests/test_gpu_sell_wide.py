@@ -28,11 +28,21 @@ def placed(scene, res, count, n, rng):
 @pytest.mark.parametrize("n,nc", [(65535, 1024), (65536, 1024), (65535, 1025), (65536, 1025), (65573, 4096), (65573, 4097),
                                   (230001, 3000), (400003, 700)])
 def test_rows_equal_the_ordered_sums(n, nc):
+    check(n, nc, np.random.default_rng(n).choice([0, 1, 3, 4, 5, 8, 9, 12, 31, 32, 33, 65], n))
+
+
+@pytest.mark.parametrize("n,nc,links", [(8000, 1000, 63000), (8000, 1000, 62999), (70001, 2500, 350005)])
+def test_rows_of_few_links(n, nc, links):
+    """A CTA of 128 rows copies the radiosities where it has as many links as there are clusters."""
+    length = np.random.default_rng(n).multinomial(links, np.full(n, 1 / n))
+    check(n, nc, length)
+
+
+def check(n, nc, length):
     rng = np.random.default_rng(n + nc)
     scene = ifx.parse(scene_src("cornell"))
     p, nrm = placed(scene, 9, nc, n, rng)
     albedo, e, area = rng.random((n, 3), np.float32), rng.random((n, 3), np.float32), 0.5 + rng.random(n, np.float32)
-    length = rng.choice([0, 1, 3, 4, 5, 8, 9, 12, 31, 32, 33, 65], n)
     starts = np.zeros(n + 1, np.uint32)
     starts[1:] = np.cumsum(length)
     idx = rng.integers(0, nc, starts[-1])
